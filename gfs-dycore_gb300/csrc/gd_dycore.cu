@@ -246,76 +246,79 @@ class Dycore : public DycoreBase {
     }
     launch_r2c<R>(sd, plan, grid, GP, ldP, GH, ldH, stream);
   }
-  std::map<int, GemmPlan> synth0_cache, anal0_cache;  // order-0-only SIMT work lists
-  // Side stream of the split modes: order 0 runs on the SIMT path beside the
-  // tensor-core GEMM of orders m >= 1 (disjoint output rows; the small SIMT
-  // CTAs fit in the SM resources the persistent GEMM leaves free).  Forked
-  // and joined with events on the context's stream, so a graph captured on
-  // that stream captures both branches.
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  void fork() {
-    GD_CUDA(cudaEventRecord(ev_fork, stream));
-    GD_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
-  }
-  void join() {
-    GD_CUDA(cudaEventRecord(ev_join, side));
-    GD_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
-  }
-  void do_synth(bool useH, const GemmPlan& plan, const R* B, long ldB, int ncr, R* F, long ldF) {
+  // One Legendre transform of an array: its columns through a table.  The
+  // split modes run order 0 on the IEEE path ahead of the tensor-core GEMMs of
+  // orders m >= 1, both tables' order 0 in one launch.
+  struct Leg {
+    bool useH;
+    const GemmPlan* plan;  // all-orders SIMT work list (not used by the split modes)
+    const R* in;
+    long ldin;
+    int ncr;
+    R* out;
+    long ldout;
+    Order0<R> order0() const { return Order0<R>{in, ldin, out, ldout, ncr / 2, useH ? 1 : 0, nullptr}; }
+  };
+  void do_synth(const Leg& a, const Leg* b = nullptr) {
     if (tcp) {
-      auto it = synth0_cache.find(ncr);
-      if (it == synth0_cache.end()) it = synth0_cache.emplace(ncr, make_synth_plan(T, nh, ncr, stream, 0, 0)).first;
-      if constexpr (std::is_same<R, float>::value) {
-        fork();
-        tc_synth(*tcp, moff, useH, B, ldB, nlm_rows, ncr, F, ldF, stream);
-        launch_synth<R>(sd, useH, it->second, B, ldB, ncr, F, ldF, side);
-        join();
-      } else {
-        // FP64 state: the GEMM of orders m >= 1 reads an FP32 copy of the
-        // spectral columns and writes FP32 Fourier rows, widened after it;
-        // order 0 runs on the FP64 SIMT path straight into F
-        // (the eddy FFT reads the FP32 rows where the GEMM left them)
-        launch_convert2d<double, float>(B, ldB, stSpec, ldB, nlm_rows, ncr, stream);
-        fork();
-        tc_synth(*tcp, moff, useH, stSpec, ldB, nlm_rows, ncr, stFour(F), ldF, stream);
-        launch_synth<R>(sd, useH, it->second, B, ldB, ncr, F, ldF, side);
-        join();
-        if (!eddy_)
-          launch_convert2d<float, double>(stFour(F) + (long)nlat * ldF, ldF, F + (long)nlat * ldF, ldF,
-                                          (long)T * nlat, ncr, stream);
-      }
+      const Order0<R> g[2] = {a.order0(), b ? b->order0() : a.order0()};
+      launch_synth0<R>(sd, g, b ? 2 : 1, stream);
+    }
+    synth_orders(a);
+    if (b) synth_orders(*b);
+  }
+  void do_anal(const Leg& a, const Leg* b = nullptr) {
+    if (tcp) {
+      const Order0<R> g[2] = {a.order0(), b ? b->order0() : a.order0()};
+      launch_anal0<R>(sd, g, b ? 2 : 1, stream);
+    }
+    anal_orders(a);
+    if (b) anal_orders(*b);
+  }
+  void synth_orders(const Leg& a) {
+    if (!tcp) {
+      launch_synth<R>(sd, a.useH, *a.plan, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
       return;
     }
-    launch_synth<R>(sd, useH, plan, B, ldB, ncr, F, ldF, stream);
+    if constexpr (std::is_same<R, float>::value) {
+      tc_synth(*tcp, moff, a.useH, a.in, a.ldin, nlm_rows, a.ncr, a.out, a.ldout, stream);
+    } else {
+      // FP64 state: the GEMM of orders m >= 1 reads an FP32 copy of the
+      // spectral columns and writes FP32 Fourier rows, widened after it
+      // (the eddy FFT reads the FP32 rows where the GEMM left them)
+      launch_convert2d<double, float>(a.in, a.ldin, stSpec, a.ldin, nlm_rows, a.ncr, stream);
+      tc_synth(*tcp, moff, a.useH, stSpec, a.ldin, nlm_rows, a.ncr, stFour(a.out), a.ldout, stream);
+      if (!eddy_)
+        launch_convert2d<float, double>(stFour(a.out) + (long)nlat * a.ldout, a.ldout, a.out + (long)nlat * a.ldout,
+                                        a.ldout, (long)T * nlat, a.ncr, stream);
+    }
   }
-  void do_anal(bool useH, const GemmPlan& plan, const R* G, long ldG, int ncr, R* A, long ldA) {
-    if (tcp) {
-      auto it = anal0_cache.find(ncr);
-      if (it == anal0_cache.end()) it = anal0_cache.emplace(ncr, make_anal_plan(T, ncr, stream, 0, 0)).first;
-      if constexpr (std::is_same<R, float>::value) {
-        fork();
-        tc_anal(*tcp, moff, useH, G, ldG, ncr, A, ldA, stream);
-        launch_anal<R>(sd, useH, it->second, G, ldG, ncr, A, ldA, side);
-        join();
-      } else {
-        // FP64 state: FP32 copy of every Fourier row (order 0 included, so the
-        // GEMM reads no stale staging), FP32 result rows of orders m >= 1
-        // (spectral rows T+1.. in the m-major order) widened after it
-        // (the eddy FFT already wrote the FP32 rows, with zeros for order 0)
-        if (!eddy_) launch_convert2d<double, float>(G, ldG, stFour(G), ldG, (long)(T + 1) * nlat, ncr, stream);
-        fork();
-        tc_anal(*tcp, moff, useH, stFour(G), ldG, ncr, stSpec, ldA, stream);
-        launch_anal<R>(sd, useH, it->second, G, ldG, ncr, A, ldA, side);
-        join();
-        // the analysis GEMM's K segments are added here in FP64
-        launch_sumconvert(stSpec + (long)(T + 1) * ldA, ldA, (long)nlm * ldA, tc_anal_segments(*tcp),
-                          A + (long)(T + 1) * ldA, ldA, (long)nlm - (T + 1), ncr, stream);
-      }
+  void anal_orders(const Leg& a) {
+    if (!tcp) {
+      launch_anal<R>(sd, a.useH, *a.plan, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
       return;
     }
-    launch_anal<R>(sd, useH, plan, G, ldG, ncr, A, ldA, stream);
+    if constexpr (std::is_same<R, float>::value) {
+      tc_anal(*tcp, moff, a.useH, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
+    } else {
+      // FP64 state: FP32 copy of every Fourier row (order 0 included, so the
+      // GEMM reads no stale staging), FP32 result rows of orders m >= 1
+      // (spectral rows T+1.. in the m-major order) widened after it
+      // (the eddy FFT already wrote the FP32 rows, with zeros for order 0)
+      if (!eddy_)
+        launch_convert2d<double, float>(a.in, a.ldin, stFour(a.in), a.ldin, (long)(T + 1) * nlat, a.ncr, stream);
+      tc_anal(*tcp, moff, a.useH, stFour(a.in), a.ldin, a.ncr, stSpec, a.ldout, stream);
+      // the analysis GEMM's K segments are added here in FP64
+      launch_sumconvert(stSpec + (long)(T + 1) * a.ldout, a.ldout, (long)nlm * a.ldout, tc_anal_segments(*tcp),
+                        a.out + (long)(T + 1) * a.ldout, a.ldout, (long)nlm - (T + 1), a.ncr, stream);
+    }
   }
+  // the step's transforms: synthesis of the state, analyses of the tendencies
+  // and of the column physics' increments
+  Leg leg_synP() { return Leg{false, &synP, S, ldS, 2 * sc.ncol, FPb, ldFP}; }
+  Leg leg_synH() { return Leg{true, &synH, S + 2 * (2 * L), ldS, 2 * (sc.ncol - 2 * L), FHb, ldFH}; }
+  Leg leg_anaP(const GemmPlan& plan, int ncol) { return Leg{false, &plan, FPb, ldGP, 2 * ncol, AP, ldAP}; }
+  Leg leg_anaH() { return Leg{true, &anaH, FHb, ldGH, 2 * ah.ncol, AH, ldAH}; }
   void check() override {
     tc_status();
     if (closure) mlp_check(closure, stream);
@@ -364,9 +367,6 @@ class Dycore : public DycoreBase {
     init_buffers();
     init_plans();
     if (split_mode()) {
-      GD_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-      GD_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-      GD_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
       tcp.reset(new TcPlan());
       // widest N tile at init (GD_TC_TILE_CAP: a tuning and measurement knob)
       tcp->tile_cap = std::max(16, env_int("GD_TC_TILE_CAP", tcp->tile_cap) / 16 * 16);
@@ -411,8 +411,6 @@ class Dycore : public DycoreBase {
     free_plan(anaPhys);
     for (auto& kv : synth_cache) free_plan(kv.second);
     for (auto& kv : anal_cache) free_plan(kv.second);
-    for (auto& kv : synth0_cache) free_plan(kv.second);
-    for (auto& kv : anal0_cache) free_plan(kv.second);
     free_fft_plan(c2rFull);
     free_fft_plan(c2rInv);
     free_fft_plan(r2cDyn);
@@ -421,11 +419,7 @@ class Dycore : public DycoreBase {
     free_fft_plan(r2cSimple);
     free_fft_plan(r2cClos);
     if (stream) cudaStreamSynchronize(stream);
-    if (side) cudaStreamSynchronize(side);
     for (void* p : allocs) cudaFree(p);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
     if (stream && own_stream) cudaStreamDestroy(stream);
   }
 
@@ -801,8 +795,8 @@ class Dycore : public DycoreBase {
 
   // ------------------------------------------------------------ passes --
   void synthesis(const FftPlan& plan) {
-    do_synth(false, synP, S, ldS, 2 * sc.ncol, FPb, ldFP);
-    do_synth(true, synH, S + 2 * (2 * L), ldS, 2 * (sc.ncol - 2 * L), FHb, ldFH);
+    const Leg h = leg_synH();
+    do_synth(leg_synP(), &h);
     mark(PH_LSYN);
     c2r(plan, FPb, ldFP, FHb, ldFH, gS);
     mark(PH_FSYN);
@@ -854,8 +848,8 @@ class Dycore : public DycoreBase {
     mark(PH_COL);
     r2c(r2cDyn, gA, FPb, ldGP, FHb, ldGH);
     mark(PH_FANA);
-    do_anal(false, anaP, FPb, ldGP, 2 * ap.ncol, AP, ldAP);
-    do_anal(true, anaH, FHb, ldGH, 2 * ah.ncol, AH, ldAH);
+    const Leg legh = leg_anaH();
+    do_anal(leg_anaP(anaP, ap.ncol), &legh);
     mark(PH_LANA);
   }
   void inverse_pass(bool want_extra) {
@@ -972,8 +966,8 @@ class Dycore : public DycoreBase {
     mark(PH_PHYS);
     r2c(r2cSimple, gA, FPb, ldGP, FHb, ldGH);
     mark(PH_FANA);
-    do_anal(false, anaSimple, FPb, ldGP, 2 * (4 * L + 1), AP, ldAP);
-    do_anal(true, anaH, FHb, ldGH, 2 * ah.ncol, AH, ldAH);
+    const Leg legh = leg_anaH();
+    do_anal(leg_anaP(anaSimple, 4 * L + 1), &legh);
     mark(PH_LANA);
   }
   void phys_pass() {
@@ -994,7 +988,7 @@ class Dycore : public DycoreBase {
     if (c.heldsuarez || c.massfix) {
       r2c(r2cPhys, gA, FPb, ldGP, FHb, ldGH);
       mark(PH_FANA);
-      do_anal(false, anaPhys, FPb, ldGP, 2 * (3 * L + 1), AP, ldAP);
+      do_anal(leg_anaP(anaPhys, 3 * L + 1));
       mark(PH_LANA);
       launch_phys_update<R>(S, ldS, sc, L, nt, nlm, AP, ldAP, c.massfix, c.heldsuarez, (R)c.dt, lapv,
                             (R)Phys::rerth, stream);
@@ -1052,10 +1046,9 @@ class Dycore : public DycoreBase {
           if (na > 2 && tc_slots(*tcp, n) < na && tc_slots(*tcp, tcp->nana) < na) continue;
           tc_set_nsyn(*tcp, n);
           const float ms = timed([&] {
-            do_synth(false, synP, S, ldS, 2 * sc.ncol, FPb, ldFP);
-            do_synth(true, synH, S + 2 * (2 * L), ldS, 2 * (sc.ncol - 2 * L), FHb, ldFH);
-            do_anal(false, anaP, FPb, ldGP, 2 * ap.ncol, AP, ldAP);
-            do_anal(true, anaH, FHb, ldGH, 2 * ah.ncol, AH, ldAH);
+            const Leg sh = leg_synH(), ah_ = leg_anaH();
+            do_synth(leg_synP(), &sh);
+            do_anal(leg_anaP(anaP, ap.ncol), &ah_);
           });
           if (verbose)
             fprintf(stderr, "autotune: synthesis tile %d, A slots %d/%d (synthesis/analysis): %.3f ms\n", n,
@@ -1090,8 +1083,8 @@ class Dycore : public DycoreBase {
     mark(PH_PHYS);
     r2c(r2cClos, gA, FPb, ldGP, FHb, ldGH);
     mark(PH_FANA);
-    do_anal(false, anaSimple, FPb, ldGP, 2 * (4 * L + 1), AP, ldAP);
-    do_anal(true, anaH, FHb, ldGH, 2 * ah.ncol, AH, ldAH);
+    const Leg legh = leg_anaH();
+    do_anal(leg_anaP(anaSimple, 4 * L + 1), &legh);
     mark(PH_LANA);
     launch_simple_update<R>(S, ldS, sc, L, nlm, AP, ldAP, AH, ldAH, 0, 0, (R)c.dt, (R)(1.0 / Phys::rerth), lapv,
                             (R)Phys::rerth, stream);
@@ -1454,8 +1447,8 @@ class Dycore : public DycoreBase {
     if (simple()) {  // phy_run_simple.f90:145-160 on the grid of the last getdyntend
       launch_simple_physics<R>(simple_args(), stream);
       r2c(r2cSimple, gA, FPb, ldGP, FHb, ldGH);
-      do_anal(false, anaSimple, FPb, ldGP, 2 * (4 * L + 1), AP, ldAP);
-      do_anal(true, anaH, FHb, ldGH, 2 * ah.ncol, AH, ldAH);
+      const Leg legh = leg_anaH();
+      do_anal(leg_anaP(anaSimple, 4 * L + 1), &legh);
       const R ai = (R)(1.0 / Phys::rerth);
       // vorticity and divergence to AP columns [2L+1, 4L+1)
       launch_combine<R>(AP, ldAP, 2 * L + 1, AH, ldAH, 0, AP, ldAP, 2 * L + 1, 2 * L, nlm, ai, stream);
@@ -1486,7 +1479,7 @@ class Dycore : public DycoreBase {
     }
     launch_hs_forcing<R>(hs_args(), stream);
     r2c(r2cPhys, gA, FPb, ldGP, FHb, ldGH);
-    do_anal(false, anaPhys, FPb, ldGP, 2 * (3 * L + 1), AP, ldAP);
+    do_anal(leg_anaP(anaPhys, 3 * L + 1));
     double* tmp = dalloc<double>(2L * nlm * L);
     spec_out(AP, ldAP, 0, L, dtv, tmp);
     spec_out(AP, ldAP, L, L, dvrt, tmp);
@@ -1511,8 +1504,9 @@ class Dycore : public DycoreBase {
   // synthesis of ncs complex columns X[nlm][ldS] with descriptors -> host grids
   template <typename H>
   void api_synth(const R* X, int ncs, bool needH, const std::vector<SynthDesc>& ds, int nrows, H* out) {
-    do_synth(false, synth_plan(2 * ncs), X, ldS, 2 * ncs, FPb, ldS);
-    if (needH) do_synth(true, synth_plan(2 * ncs), X, ldS, 2 * ncs, FHb, ldS);
+    const GemmPlan* plan = tcp ? nullptr : &synth_plan(2 * ncs);
+    const Leg h{true, plan, X, ldS, 2 * ncs, FHb, ldS};
+    do_synth(Leg{false, plan, X, ldS, 2 * ncs, FPb, ldS}, needH ? &h : nullptr);
     FftPlan p = mk_c2r(ds.data(), (int)ds.size());
     c2r(p, FPb, ldS, FHb, ldS, gS);
     grid_out(gS, nrows, out);
@@ -1631,8 +1625,8 @@ class Dycore : public DycoreBase {
   void api_anal(const std::vector<AnalDesc>& ds, int ncP, int ncH) {
     FftPlan p = mk_r2c(ds.data(), (int)ds.size());
     r2c(p, gA, FPb, ldS, FHb, ldS);
-    do_anal(false, anal_plan(2 * ncP), FPb, ldS, 2 * ncP, AP, ldAP);
-    if (ncH > 0) do_anal(true, anal_plan(2 * ncH), FHb, ldS, 2 * ncH, AH, ldAH);
+    const Leg h{true, tcp || ncH <= 0 ? nullptr : &anal_plan(2 * ncH), FHb, ldS, 2 * ncH, AH, ldAH};
+    do_anal(Leg{false, tcp ? nullptr : &anal_plan(2 * ncP), FPb, ldS, 2 * ncP, AP, ldAP}, ncH > 0 ? &h : nullptr);
     free_fft_plan(p);
   }
   int achunk() const { return std::max(1, std::min(ap.ncol / 2, ar.total / 2)); }

@@ -47,9 +47,8 @@ struct GemmPlan {
   int4* items = nullptr;  // device work list
   int nitems = 0;
 };
-// work lists over orders m in [m_lo, m_hi] (default: all orders)
-GemmPlan make_synth_plan(int T, int nh, int ncols_real, cudaStream_t s, int m_lo = 0, int m_hi = -1);
-GemmPlan make_anal_plan(int T, int ncols_real, cudaStream_t s, int m_lo = 0, int m_hi = -1);
+GemmPlan make_synth_plan(int T, int nh, int ncols_real, cudaStream_t s);
+GemmPlan make_anal_plan(int T, int ncols_real, cudaStream_t s);
 void free_plan(GemmPlan& p);
 template <typename R>
 void launch_synth(const ShtDev<R>& d, bool useH, const GemmPlan& plan, const R* B, long ldB, int ncols_real,
@@ -57,6 +56,22 @@ void launch_synth(const ShtDev<R>& d, bool useH, const GemmPlan& plan, const R* 
 template <typename R>
 void launch_anal(const ShtDev<R>& d, bool useH, const GemmPlan& plan, const R* G, long ldG, int ncols_real,
                  R* A, long ldA, cudaStream_t s);
+// order 0 alone (the split modes' zonal means), up to two tables' jobs per
+// launch: out[j][c] from in[q][c] (synthesis), out[q][c] from in[j][c]
+// (analysis) over ncc complex columns, row pitches in reals
+template <typename R>
+struct Order0 {
+  const R* in;
+  long ldin;
+  R* out;
+  long ldout;
+  int ncc, parityH;  // parityH: the dP/dphi table
+  const R* tab;      // filled in by the launcher
+};
+template <typename R>
+void launch_synth0(const ShtDev<R>& d, const Order0<R>* jobs, int njobs, cudaStream_t s);
+template <typename R>
+void launch_anal0(const ShtDev<R>& d, const Order0<R>* jobs, int njobs, cudaStream_t s);
 
 // Longitude stage.
 struct SynthDesc {  // a run of output grid rows

@@ -8,6 +8,7 @@
 // shtns_spat_to_sh (shtns.f90:195,199,225,229) and the vector forms
 // (shtns.f90:261,270,303,308,341,348).  Convention: orthonormal harmonics
 // without Condon-Shortley phase (shtns.f90:110), latitudes north to south.
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 #include <vector>
@@ -211,11 +212,10 @@ void launch_sumconvert(const float* src, long lds, long seg_stride, int nseg, do
 // by 16 for conflict-free shared reads and coalesced stores).
 constexpr int GT_R = 32, GT_C = 64, GT_K = 16;
 
-GemmPlan make_synth_plan(int T, int nh, int ncols_real, cudaStream_t s, int m_lo, int m_hi) {
+GemmPlan make_synth_plan(int T, int nh, int ncols_real, cudaStream_t s) {
   std::vector<int4> it;
   int tj = ceil_div(nh, GT_R), tc = ceil_div(ncols_real, GT_C);
-  if (m_hi < 0) m_hi = T;
-  for (int m = m_lo; m <= m_hi; ++m)  // longest K first for load balance
+  for (int m = 0; m <= T; ++m)  // longest K first for load balance
     for (int a = 0; a < tj; ++a)
       for (int b = 0; b < tc; ++b) it.push_back(make_int4(m, a, b, 0));
   GemmPlan p;
@@ -226,11 +226,10 @@ GemmPlan make_synth_plan(int T, int nh, int ncols_real, cudaStream_t s, int m_lo
   return p;
 }
 
-GemmPlan make_anal_plan(int T, int ncols_real, cudaStream_t s, int m_lo, int m_hi) {
+GemmPlan make_anal_plan(int T, int ncols_real, cudaStream_t s) {
   std::vector<int4> it;
   int tc = ceil_div(ncols_real, GT_C);
-  if (m_hi < 0) m_hi = T;
-  for (int m = m_lo; m <= m_hi; ++m)
+  for (int m = 0; m <= T; ++m)
     for (int a = 0; a < ceil_div(T - m + 1, GT_R); ++a)
       for (int b = 0; b < tc; ++b) it.push_back(make_int4(m, a, b, 0));
   GemmPlan p;
@@ -394,6 +393,183 @@ template void launch_anal<double>(const ShtDev<double>&, bool, const GemmPlan&, 
                                   long, cudaStream_t);
 template void launch_anal<float>(const ShtDev<float>&, bool, const GemmPlan&, const float*, long, int, float*,
                                  long, cudaStream_t);
+
+// Order 0 of the split modes (the zonal means, on the IEEE path): real
+// coefficients, so only the real parts are summed -- half the multiply-adds of
+// the general kernels above; the imaginary parts (zero for a real field) are
+// written as 0 times their operands, which keeps a NaN or infinity there
+// visible.  A CTA takes 8 latitude pairs (or degrees) x 32 columns, one row per
+// warp and one column per lane, the contraction staged in chunks with the
+// next chunk's loads in flight over the current one's sums.  One launch takes
+// both tables' jobs (blockIdx.z).  The sums run over the contraction index in order, as in k_synth and
+// k_anal (same bits).
+//
+// Bound by the FP64 pipe for R = double (two multiply-adds per clock and SM),
+// by the launch and the load latency for R = float.  The general kernels'
+// 32 x 64 tiles left most SMs idle here (78 CTAs at T254, 39 at T126) and,
+// on a second stream beside the persistent GEMM, slowed both down: the
+// Legendre phases of an FP64-state (eddy) step took 14.3 ms at T254L64 and
+// 6.0 ms at T126L64 with 4.6 and 1.0 ms of GEMM, now 6.5 and 1.7 ms; of a
+// TF32x3 step at T254L64 3.4 ms, now 2.9 ms.
+constexpr int Z0_K = 64, Z0_C = 32;
+template <typename R>
+__global__ void __launch_bounds__(256) k_synth0(int K, int nh, int nlat, Order0<R> jobP, Order0<R> jobH) {
+  const Order0<R> g = blockIdx.z ? jobH : jobP;
+  const R* __restrict__ tab = g.tab;
+  const R* __restrict__ B = g.in;
+  R* __restrict__ F = g.out;
+  const long ldB = g.ldin, ldF = g.ldout;
+  const int ncc = g.ncc, parityH = g.parityH;
+  typedef typename C2<R>::T V;
+  constexpr int TJ = 8, NB = Z0_K * Z0_C / 256, NA = TJ * Z0_K / 256;
+  __shared__ R sA[TJ][Z0_K];
+  __shared__ R sB[Z0_K][Z0_C];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int j0 = blockIdx.x * TJ, c = blockIdx.y * Z0_C + lane;
+  if (blockIdx.y * Z0_C >= ncc) return;  // the grid covers the wider job
+  R e = R(0), o = R(0), z = R(0);
+  R va[NA];
+  V vb[NB];
+  auto load = [&](int q0) {
+#pragma unroll
+    for (int u = 0; u < NA; ++u) {
+      const int x = threadIdx.x + 256 * u, j = j0 + x / Z0_K, q = q0 + x % Z0_K;
+      va[u] = (j < nh && q < K) ? tab[(long)j * K + q] : R(0);
+    }
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      const int q = q0 + w + 8 * u;
+      vb[u] = mk2<R>(R(0), R(0));
+      if (q < K && c < ncc) vb[u] = *reinterpret_cast<const V*>(B + (long)q * ldB + 2 * c);
+    }
+  };
+  load(0);
+  for (int q0 = 0; q0 < K; q0 += Z0_K) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NA; ++u) {
+      const int x = threadIdx.x + 256 * u;
+      sA[x / Z0_K][x % Z0_K] = va[u];
+    }
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      sB[w + 8 * u][lane] = vb[u].x;
+      z += R(0) * vb[u].y;
+    }
+    __syncthreads();
+    if (q0 + Z0_K < K) load(q0 + Z0_K);
+    const int n = min(Z0_K, (K - q0 + 1) & ~1);  // an odd count's last partner is a staged zero
+#pragma unroll 8
+    for (int q = 0; q < n; q += 2) {
+      e += sA[w][q] * sB[q][lane];
+      o += sA[w][q + 1] * sB[q + 1][lane];
+    }
+  }
+  // the warps' shares of the imaginary operands meet in sB
+  __syncthreads();
+  sB[w][lane] = z;
+  __syncthreads();
+  z = R(0);
+#pragma unroll
+  for (int u = 0; u < 8; ++u) z += sB[u][lane];
+  if (c >= ncc) return;
+  const int j = j0 + w;
+  if (j >= nh) return;
+  *reinterpret_cast<V*>(F + (long)j * ldF + 2 * c) = mk2<R>(e + o, z);
+  *reinterpret_cast<V*>(F + (long)(nlat - 1 - j) * ldF + 2 * c) = mk2<R>(parityH ? o - e : e - o, z);
+}
+template <typename R>
+__global__ void __launch_bounds__(256) k_anal0(int K, int nh, int nlat, Order0<R> jobP, Order0<R> jobH) {
+  const Order0<R> g0 = blockIdx.z ? jobH : jobP;
+  const R* __restrict__ tab = g0.tab;
+  const R* __restrict__ G = g0.in;
+  R* __restrict__ A = g0.out;
+  const long ldG = g0.ldin, ldA = g0.ldout;
+  const int ncc = g0.ncc, parityH = g0.parityH;
+  typedef typename C2<R>::T V;
+  constexpr int TQ = 8, KJ = Z0_K / 2, NB = KJ * Z0_C / 256, NA = TQ * KJ / 256;
+  __shared__ R sT[KJ][TQ];
+  __shared__ R sE[KJ][Z0_C], sO[KJ][Z0_C];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int q0 = blockIdx.x * TQ, c = blockIdx.y * Z0_C + lane;
+  if (blockIdx.y * Z0_C >= ncc) return;  // the grid covers the wider job
+  R acc = R(0), z = R(0);
+  R va[NA];
+  V vn[NB], vs[NB];
+  auto load = [&](int jb) {
+#pragma unroll
+    for (int u = 0; u < NA; ++u) {
+      const int x = threadIdx.x + 256 * u, j = jb + x / TQ, q = q0 + x % TQ;
+      va[u] = (j < nh && q < K) ? tab[(long)j * K + q] : R(0);
+    }
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      const int j = jb + w + 8 * u;
+      vn[u] = vs[u] = mk2<R>(R(0), R(0));
+      if (j < nh && c < ncc) {
+        vn[u] = *reinterpret_cast<const V*>(G + (long)j * ldG + 2 * c);
+        vs[u] = *reinterpret_cast<const V*>(G + (long)(nlat - 1 - j) * ldG + 2 * c);
+      }
+    }
+  };
+  load(0);
+  for (int jb = 0; jb < nh; jb += KJ) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NA; ++u) {
+      const int x = threadIdx.x + 256 * u;
+      sT[x / TQ][x % TQ] = va[u];
+    }
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+      const R p = vn[u].x + vs[u].x, m = vn[u].x - vs[u].x;
+      // degrees with even n - m pair with north + south for P, north - south for dP/dphi
+      sE[w + 8 * u][lane] = parityH ? m : p;
+      sO[w + 8 * u][lane] = parityH ? p : m;
+      z += R(0) * (vn[u].y + vs[u].y);
+    }
+    __syncthreads();
+    if (jb + KJ < nh) load(jb + KJ);
+    const int n = min(KJ, nh - jb);
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) acc += sT[j][w] * ((w & 1) ? sO[j][lane] : sE[j][lane]);
+  }
+  __syncthreads();
+  sE[w][lane] = z;
+  __syncthreads();
+  z = R(0);
+#pragma unroll
+  for (int u = 0; u < 8; ++u) z += sE[u][lane];
+  if (c >= ncc) return;
+  const int q = q0 + w;
+  if (q < K) *reinterpret_cast<V*>(A + (long)q * ldA + 2 * c) = mk2<R>(acc, z);
+}
+template <typename R, typename Kern>
+static void launch_order0(Kern kern, const ShtDev<R>& d, int rows, const Order0<R>* jobs, int njobs, cudaStream_t s) {
+  Order0<R> g[2] = {};
+  int ncc = 0;
+  for (int i = 0; i < njobs; ++i) {
+    g[i] = jobs[i];
+    g[i].tab = jobs[i].parityH ? d.H : d.P;
+    ncc = std::max(ncc, g[i].ncc);
+  }
+  if (ncc <= 0) return;
+  kern<<<dim3(ceil_div(rows, 8), ceil_div(ncc, Z0_C), njobs), 256, 0, s>>>(d.T + 1, d.nh, d.nlat, g[0], g[1]);
+  count_launch();
+  GD_LAUNCH_CHECK();
+}
+template <typename R>
+void launch_synth0(const ShtDev<R>& d, const Order0<R>* jobs, int njobs, cudaStream_t s) {
+  launch_order0<R>(k_synth0<R>, d, d.nh, jobs, njobs, s);
+}
+template <typename R>
+void launch_anal0(const ShtDev<R>& d, const Order0<R>* jobs, int njobs, cudaStream_t s) {
+  launch_order0<R>(k_anal0<R>, d, d.T + 1, jobs, njobs, s);
+}
+template void launch_synth0<double>(const ShtDev<double>&, const Order0<double>*, int, cudaStream_t);
+template void launch_synth0<float>(const ShtDev<float>&, const Order0<float>*, int, cudaStream_t);
+template void launch_anal0<double>(const ShtDev<double>&, const Order0<double>*, int, cudaStream_t);
+template void launch_anal0<float>(const ShtDev<float>&, const Order0<float>*, int, cudaStream_t);
 
 // -------------------------------------------------------------- FFTs ------
 // Real transforms of length nlon = 2M through one complex Stockham FFT of
