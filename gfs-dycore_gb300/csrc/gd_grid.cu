@@ -426,8 +426,31 @@ template void launch_dyn_columns<float>(const ColumnArgs<float>&, bool, cudaStre
 
 // Held-Suarez forcing on the grid (phy_run_hs.f90:42-77); prs and psg are
 // recomputed from ln(ps) as in calc_pressdata.
+//
+// The layer pressure prs = ((p1^(k+1) - p0^(k+1)) / ((k+1)(p1 - p0)))^(1/k) of
+// the layer p0..p1 is pm times a function of z = (p1 - p0) / (p1 + p0) alone,
+// pm = (p1 + p0) / 2: even in z, so ln(prs/pm) and prs/pm are power series in
+// w = z^2 (binomial series, coefficients from the launcher).  One logarithm
+// and a few multiply-adds replace two powers, a logarithm and an exponential
+// per level, and the difference of powers no longer cancels in thin layers.
+// w <= 1/64: 9 terms (the remainder is below 1e-18); w <= 0.16: 20 terms
+// (below 1e-17); thicker layers (the top two or three of a set that starts at
+// p = 0) take the powers.  prs itself matters only below sigma = sigbot.
+//
+// Bound by the FP64 pipe in the FP64 state and, on small grids, by the threads
+// in flight: a thread takes a.lt levels, so a T42L20 grid is 320 CTAs instead
+// of 32.  Physics phase of a step (this kernel, the mass fixer and the
+// update), before -> after: T254L64 FP64 state 7.77 -> 3.82 ms, T126L64 FP64
+// 1.97 -> 0.97 ms, T42L20 FP64 0.330 -> 0.088 ms, T574L64 FP32 0.563 -> 0.467 ms.
+template <typename R, int N>
+__device__ __forceinline__ R hs_series(const R* c, R w) {
+  R v = c[N - 1];
+#pragma unroll
+  for (int k = N - 2; k >= 0; --k) v = v * w + c[k];
+  return v;
+}
 template <typename R>
-__global__ void __launch_bounds__(256) k_hs(HsArgs<R> a) {
+__global__ void __launch_bounds__(128) k_hs(const __grid_constant__ HsArgs<R> a) {
   const long ng = (long)a.nlon * a.nlat;
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= ng) return;
@@ -436,13 +459,13 @@ __global__ void __launch_bounds__(256) k_hs(HsArgs<R> a) {
   const R ps = exp(a.gS[(long)a.s.lnps * ng + p]);
   const R sl = a.sinlat[j], cl = a.coslat[j];
   const R s2 = sl * sl, c2 = cl * cl, c4 = c2 * c2;
-  const R p0 = R(1.e5), logp0 = log(p0);
-  // levels in groups of four: the group's grid loads are issued before its
-  // arithmetic, and pk^kappa of an interface is carried from the level below
-  // (the bottom interface of a level is the top one of the level under it)
+  const R rp0 = R(1.e-5), ips = R(1) / ps, psbot = a.sigbot * ps, isig = R(1) / (R(1) - a.sigbot);
+  const R t0 = R(315) - R(60) * s2, t1 = R(10) * c2, kb = (a.kradb - a.krada) * c4;
+  const R sp = a.sppt ? a.sppt[p] : R(0);
+  const int b1 = min(L, ((int)blockIdx.y + 1) * a.lt);
+  // levels in groups of four: the group's grid loads are issued before its arithmetic
   constexpr int G = 4;
-  R pw1 = pow(a.ak[L] + a.bk[L] * ps, a.kappa);
-  for (int b0 = 0; b0 < L; b0 += G) {
+  for (int b0 = blockIdx.y * a.lt; b0 < b1; b0 += G) {
     R tvv[G], vrv[G], dvv[G];
 #pragma unroll
     for (int u = 0; u < G; ++u) {
@@ -454,35 +477,67 @@ __global__ void __launch_bounds__(256) k_hs(HsArgs<R> a) {
 #pragma unroll
     for (int u = 0; u < G; ++u) {
       const int b = b0 + u;
-      if (b >= L) break;
+      if (b >= b1) break;
       const int t = L - 1 - b;
       const R pkt = a.ak[t] + a.bk[t] * ps, pkt1 = a.ak[t + 1] + a.bk[t + 1] * ps;
-      const R pw0 = pow(pkt, a.kappa);
-      // Phillips layer pressure prs = X^(1/kappa) and ln(prs/p0) from one
-      // logarithm of X: three logarithms and two powers fewer per level than
-      // pow(X, 1/kappa), pow(prs/p0, expo) and log(prs/p0) (the level loop's
-      // FP64 cost; the results agree to ~1e-14 relative)
-      const R lx = log((pw1 * pkt1 - pw0 * pkt) / ((a.kappa + R(1)) * (pkt1 - pkt))) / a.kappa;
-      const R prs = exp(lx);
-      const R lp = lx - logp0;
-      pw1 = pw0;
-      R bl = prs / ps;
-      R teq = exp(a.expo * lp) * (R(315) - R(60) * s2 - R(10) * lp * c2);
-      bl = (bl - a.sigbot) / (R(1) - a.sigbot);
+      const R dp = pkt1 - pkt, sum = pkt1 + pkt, pm = R(0.5) * sum;
+      const R z = dp / sum, w = z * z;
+      const bool low = !(pkt1 < psbot);  // prs < pkt1: above this level the drag profile is zero
+      R lp, bl = R(0);                // ln(prs / p0), (prs / ps - sigbot) / (1 - sigbot)
+      if (w <= R(0.16)) {
+        lp = log(pm * rp0) + (w <= R(0.015625) ? hs_series<R, 9>(a.lns, w) : hs_series<R, HsArgs<R>::NS>(a.lns, w));
+        if (low)
+          bl = pm * ips * (w <= R(0.015625) ? hs_series<R, 9>(a.prss, w) : hs_series<R, HsArgs<R>::NS>(a.prss, w));
+      } else {
+        const R x = (pow(pkt1, a.kappa) * pkt1 - pow(pkt, a.kappa) * pkt) / ((a.kappa + R(1)) * dp);
+        const R lx = log(x) / a.kappa;
+        lp = lx + log(rp0);
+        if (low) bl = exp(lx) * ips;
+      }
+      bl = low ? (bl - a.sigbot) * isig : R(0);
       if (bl < R(0)) bl = R(0);
+      R teq = exp(a.expo * lp) * (t0 - lp * t1);
       if (teq < R(200)) teq = R(200);
       const R tv = tvv[u], vr = vrv[u], dv = dvv[u];
-      const R f = a.sppt ? R(1) + a.vfact[b] * a.sppt[p] : R(1);
-      a.gA[(long)b * ng + p] = f * ((a.krada + (a.kradb - a.krada) * bl * c4) * (teq - tv));
+      const R f = a.sppt ? R(1) + a.vfact[b] * sp : R(1);
+      a.gA[(long)b * ng + p] = f * ((a.krada + kb * bl) * (teq - tv));
       a.gA[(long)(L + b) * ng + p] = f * (-(bl * a.kdrag) * vr);
       a.gA[(long)(2 * L + b) * ng + p] = f * (-(bl * a.kdrag) * dv);
     }
   }
 }
 template <typename R>
-void launch_hs_forcing(const HsArgs<R>& a, cudaStream_t s) {
-  long ng = (long)a.nlon * a.nlat;
-  k_hs<R><<<ceil_div(ng, 256), 256, 0, s>>>(a);
+void launch_hs_forcing(const HsArgs<R>& in, cudaStream_t s) {
+  HsArgs<R> a = in;
+  const long ng = (long)a.nlon * a.nlat;
+  constexpr int NS = HsArgs<R>::NS;
+  // g(w) = ((1+z)^(k+1) - (1-z)^(k+1)) / (2 (k+1) z) = sum_i C(k+1, 2i+1) / (k+1) w^i,
+  // h = ln(g) / k and exp(h), each series from the one before by its derivative
+  const double kap = (double)a.kappa;
+  double c[NS], h[NS], e[NS];
+  double bin = 1.0;  // C(k+1, 2i+1) / (k+1)
+  for (int i = 0; i < NS; ++i) {
+    if (i > 0) bin *= (kap + 2.0 - 2 * i) * (kap + 1.0 - 2 * i) / ((2.0 * i) * (2.0 * i + 1.0));
+    c[i] = bin;
+  }
+  h[0] = 0.0;
+  for (int i = 1; i < NS; ++i) {
+    double v = i * c[i];
+    for (int q = 1; q < i; ++q) v -= q * h[q] * kap * c[i - q];
+    h[i] = v / (i * kap);
+  }
+  e[0] = 1.0;
+  for (int i = 1; i < NS; ++i) {
+    double v = 0.0;
+    for (int q = 1; q <= i; ++q) v += q * h[q] * e[i - q];
+    e[i] = v / i;
+  }
+  for (int i = 0; i < NS; ++i) a.lns[i] = (R)h[i], a.prss[i] = (R)e[i];
+  // eight levels per thread share the column's exp and profiles; four while
+  // that leaves fewer than eight CTAs per SM
+  const int nx = ceil_div(ng, 128);
+  a.lt = (long)nx * ceil_div(a.L, 8) >= 8 * 152 ? 8 : 4;
+  k_hs<R><<<dim3(nx, ceil_div(a.L, a.lt)), 128, 0, s>>>(a);
   count_launch();
   GD_LAUNCH_CHECK();
 }

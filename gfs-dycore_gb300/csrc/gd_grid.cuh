@@ -56,6 +56,12 @@ struct HsArgs {
   const R* vfact;  // [L] bottom to top
   R kappa;
   R sigbot, kdrag, krada, kradb, expo;
+  // filled in by the launcher: levels per thread, and the power series in
+  // ((p1 - p0) / (p1 + p0))^2 of ln(prs / pm) and prs / pm, prs the Phillips
+  // pressure of the layer p0..p1 and pm its mean pressure
+  static constexpr int NS = 20;
+  int lt;
+  R lns[NS], prss[NS];
 };
 template <typename R>
 void launch_hs_forcing(const HsArgs<R>& a, cudaStream_t s);
