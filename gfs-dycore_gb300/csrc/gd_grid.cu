@@ -15,28 +15,60 @@
 
 namespace gd {
 
-template <typename R>
-__device__ __forceinline__ R epstiny_of();
-template <>
-__device__ __forceinline__ double epstiny_of<double>() {
-  return DBL_MIN;
-}
-template <>
-__device__ __forceinline__ float epstiny_of<float>() {
-  return FLT_MIN;
-}
-
 constexpr int LMAX = 128;
 
-// Division and logarithm of the column kernel: IEEE for the FP64 path (the
-// reference restated exactly), the hardware approximations for the FP32
-// state (relative error ~1e-7, below the FP32 state's own rounding).
-__device__ __forceinline__ double cdiv(double a, double b) { return a / b; }
+// Division, reciprocal and logarithm of the column kernel: the hardware
+// approximations for the FP32 state (relative error ~1e-7, below the FP32
+// state's own rounding).  In the FP64 state the FP64 pipe (two lanes per clock
+// and SM) bounds the kernel, so its reciprocal is one step of Halley's
+// third-order iteration r (1 + e + e^2), e = 1 - x r, on the hardware's
+// approximation (relative error 2^-20 at worst; e^3 is below 2^-59): three
+// multiply-adds, last-bit differences from the IEEE quotient.  Operands here
+// are pressures, layer thicknesses and tracer differences, normal numbers.
+__device__ __forceinline__ double crcp(double a) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+  const double e = fma(-a, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ double cdiv(double a, double b) {
+  const double r = crcp(b), q = a * r;
+  return fma(fma(-b, q, a), r, q);
+}
 __device__ __forceinline__ float cdiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double clog(double a) { return log(a); }
-__device__ __forceinline__ double crcp(double a) { return 1.0 / a; }
 __device__ __forceinline__ float crcp(float a) { return __fdividef(1.f, a); }
 __device__ __forceinline__ float clog(float a) { return __logf(a); }
+
+// ln(p1 / p0) and alfa = 1 - p0 / (p1 - p0) ln(p1 / p0) of a layer (dp = p1 -
+// p0) in the FP64 state: 2 atanh(z) = 2 z (1 + s), z = dp / (p1 + p0), s = w
+// (1/3 + w/5 + ...), w = z^2, and alfa = z - (1 - z) s.  For thin layers this
+// is both cheaper than a quotient and a logarithm and free of alfa's
+// cancellation.  w <= 1/64: 8 terms, w <= 0.16: 19 terms (remainders below
+// 3e-18); thicker layers take the logarithm.
+__device__ __forceinline__ void layer_log(double p0, double p1, double dp, double& rl, double& al) {
+  const double z = dp * crcp(p1 + p0), w = z * z;
+  double s;
+  if (w <= 0.015625) {
+    s = 1.0 / 17;
+#pragma unroll
+    for (int k = 15; k >= 3; k -= 2) s = fma(s, w, 1.0 / k);
+  } else if (w <= 0.16) {
+    s = 1.0 / 39;
+#pragma unroll
+    for (int k = 37; k >= 3; k -= 2) s = fma(s, w, 1.0 / k);
+  } else {
+    rl = log(p1 / p0);
+    al = 1.0 - (p0 / dp) * rl;
+    return;
+  }
+  s *= w;
+  rl = fma(z + z, s, z + z);
+  al = fma(z - 1.0, s, z);
+}
+__device__ __forceinline__ void layer_log(float p0, float p1, float dp, float& rl, float& al) {
+  rl = clog(cdiv(p1, p0));
+  al = 1.f - (p0 * crcp(dp)) * rl;
+}
 
 // Thuburn (1993) limited half-level value at interior interface k
 // (dyn_run.f90:574-590): qa = level above the interface, qb = level below,
@@ -46,24 +78,37 @@ __device__ __forceinline__ float clog(float a) { return __logf(a); }
 // 2 phi / (1 + phi) = 2 r / (d0 + r) when r and d0 have one sign and 0
 // otherwise: one division instead of two, and finite where r / d0 would
 // overflow (d0 is clamped to the smallest normal, not to zero).
-template <typename R>
-__device__ __forceinline__ R thuburn_half(R qa, R qb, R dm, R d0, R dp, R eta) {
-  const R h = R(0.5) * (qb + qa);
-  const bool up = eta > R(0);
-  const R qu = up ? qa : qb;
-  const R r = up ? dm : dp;
-  const bool same = (r > R(0)) == (d0 > R(0)) && r != R(0);
-  const R lim = same ? cdiv(R(2) * r, d0 + r) : R(0);
+__device__ __forceinline__ float thuburn_half(float qa, float qb, float dm, float d0, float dp, float eta) {
+  const float h = 0.5f * (qb + qa);
+  const bool up = eta > 0.f;
+  const float qu = up ? qa : qb;
+  const float r = up ? dm : dp;
+  const bool same = (r > 0.f) == (d0 > 0.f) && r != 0.f;
+  const float lim = same ? cdiv(2.f * r, d0 + r) : 0.f;
   return qu + lim * (h - qu);
+}
+// FP64: h - qu is half of +-(qb - qa), so the limited value is qu +- (qb - qa)
+// r / (d0 + r); the signs are read from the bit patterns (comparisons run on
+// the FP64 pipe).  eta = 0 takes the other upwind value than eta > 0 would in
+// the form above: its flux is 0 either way.
+__device__ __forceinline__ double thuburn_half(double qa, double qb, double dm, double d0, double dp, double eta) {
+  const bool up = __double2hiint(eta) >= 0;
+  const double qu = up ? qa : qb, r = up ? dm : dp, d = qb - qa;
+  const bool same = (__double2hiint(r) ^ __double2hiint(d0)) >= 0;
+  const double lim = same ? r * crcp(d0 + r) : 0.0;
+  return fma(lim, up ? d : -d, qu);
 }
 
 // dd[k] = q(level below k) - q(level above k) at interior interface k,
 // clamped away from zero (dyn_run.f90:519-524)
-template <typename R>
-__device__ __forceinline__ R dd_mid(R qbelow, R qabove) {
-  const R eps = epstiny_of<R>();
-  const R d = qbelow - qabove;
-  return (fabs(d) < eps) ? copysign(eps, d) : d;
+__device__ __forceinline__ float dd_mid(float qbelow, float qabove) {
+  const float d = qbelow - qabove;
+  return (fabsf(d) < FLT_MIN) ? copysignf(FLT_MIN, d) : d;
+}
+__device__ __forceinline__ double dd_mid(double qbelow, double qabove) {
+  const double d = qbelow - qabove;
+  const int hi = __double2hiint(d);  // |d| < DBL_MIN: the exponent field is zero
+  return (hi & 0x7ff00000) == 0 ? __hiloint2double((hi & (int)0x80000000) | 0x00100000, 0) : d;
 }
 // one-sided boundary differences (dyn_run.f90:507-518): dd[0] from the top
 // level qt and the one below it, dd[L] from the bottom level qb and the one
@@ -113,13 +158,16 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
   const int j = (int)(p / a.nlon);
   R* part = reinterpret_cast<R*>(smcol);  // [5][NW][32] block sums, then [2][32] column totals
   R* etas = part + (5 * NW + 2) * 32;      // [L+1][32] etadot
-  // FP64: ln(p(t+1)/p(t)) and 1/p(t) of every layer from phase 1 for phase 3
-  // (each thread reads back only what it wrote: no barrier).  Its log and
-  // reciprocals are the costly FP64 operations of the level loop; the FP32
-  // kernel recomputes them (hardware approximations).
+  // FP64: ln(p(t+1)/p(t)) and alfa of every layer and bk(t)/p(t) of its top
+  // interface, from phase 1 for phase 3 (each thread reads back only what it
+  // wrote: no barrier); the FP32 kernel recomputes them (hardware
+  // approximations).
   constexpr bool kKeep = sizeof(R) == 8;
   R* rls = etas + (L + 1) * 32;  // [L][32] (FP64 only)
-  R* ipks = rls + L * 32;        // [L][32] (FP64 only)
+  R* als = rls + L * 32;         // [L][32] (FP64 only)
+  R* bps = als + L * 32;         // [L][32] (FP64 only)
+  // an inverse pass without omega/p needs only the divergence sums
+  const bool brief = inverse_only && !a.dlnpdtg;
   auto PART = [&](int q, int ww) -> R& { return part[(q * NW + ww) * 32 + lane]; };
   auto ETA = [&](int t) -> R& { return etas[t * 32 + lane]; };
   const R* gS = a.gS;
@@ -131,16 +179,15 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
   const R ps = exp(S(a.s.lnps));
   const R dlx = S(a.s.dlnpsdx), dly = S(a.s.dlnpsdy);
   auto PK = [&](int t) -> R { return __ldg(ak + t) + __ldg(bk + t) * ps; };
-  auto RLN = [&](int t, R pkt, R pkt1) -> R { return (t == 0) ? a.rlnp_top : clog(cdiv(pkt1, pkt)); };
   const int b0 = w * LB;
   const int nb = max(0, min(LB, L - b0));
 
   // phase 1
   R xdb[LB], xcb[LB];
   R s2 = R(0), su = R(0), sv = R(0);
-  // pressure and its reciprocal at the bottom interface of the current level,
-  // carried upward (the top interface of level i is the bottom one of i + 1)
-  R pkb = PK(L - b0), ipkb = crcp(pkb);
+  // pressure and bk / p at the bottom interface of the current level, carried
+  // upward (the top interface of level i is the bottom one of i + 1)
+  R pkb = PK(L - b0), bpb = __ldg(bk + L - b0) * crcp(pkb);
   // the block's inputs, all loads issued before the arithmetic (levels past
   // the block's end load its last level again and are not used)
   R lu[LB], lv[LB], ldv[LB], ltv[LB], ltx[LB], lty[LB];
@@ -150,9 +197,12 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
     lu[i] = S(a.s.u + b);
     lv[i] = S(a.s.v + b);
     ldv[i] = S(a.s.div + b);
-    ltv[i] = S(a.s.tv + b);
-    ltx[i] = S(a.s.dtvdx + b);
-    lty[i] = S(a.s.dtvdy + b);
+    ltv[i] = ltx[i] = lty[i] = R(0);
+    if (!inverse_only) {  // the inverse transform leaves no temperature gradients
+      ltv[i] = S(a.s.tv + b);
+      ltx[i] = S(a.s.dtvdx + b);
+      lty[i] = S(a.s.dtvdy + b);
+    }
   }
 #pragma unroll
   for (int i = 0; i < LB; ++i) {
@@ -161,22 +211,26 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
     if (i < nb) {
       const int b = b0 + i, t = L - 1 - b;
       const R pkt = PK(t), pkt1 = pkb, dp = pkt1 - pkt;
-      const R ipkt = t > 0 ? crcp(pkt) : R(0), ipk1 = ipkb;
       pkb = pkt;
-      ipkb = ipkt;
       const R cg = lu[i] * dlx + lv[i] * dly;
       xdb[i] = ldv[i] * dp;
       xcb[i] = cg * __ldg(dbk + t);
-      if (t > 0) {  // terms of the sums over the layers below a layer
-        const R rl = clog(cdiv(pkt1, pkt));
-        s2 += (__ldg(bk + t + 1) * ipk1 - __ldg(bk + t) * ipkt) * ltv[i];
-        su += rl * ltx[i];
-        sv += rl * lty[i];
-        if (kKeep) rls[t * 32 + lane] = rl;
-      } else if (kKeep) {
-        rls[lane] = a.rlnp_top;
+      if (!brief) {
+        const R bpt = t > 0 ? __ldg(bk + t) * crcp(pkt) : R(0);  // unused at the model top (pk = 0)
+        R rl = a.rlnp_top, al = a.log2sp;
+        if (t > 0) {  // terms of the sums over the layers below a layer
+          layer_log(pkt, pkt1, dp, rl, al);
+          s2 += (bpb - bpt) * ltv[i];
+          su += rl * ltx[i];
+          sv += rl * lty[i];
+        }
+        if (kKeep) {
+          rls[t * 32 + lane] = rl;
+          als[t * 32 + lane] = al;
+          bps[t * 32 + lane] = bpt;
+        }
+        bpb = bpt;
       }
-      if (kKeep) ipks[t * 32 + lane] = ipkt;
       if (a.prs && valid)
         a.prs[(long)b * ng + p] =
             pow((pow(pkt1, a.kappa) * pkt1 - pow(pkt, a.kappa) * pkt) / ((a.kappa + R(1)) * dp), R(1) / a.kappa);
@@ -237,7 +291,7 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
       if (!inverse_only) a.gA[(long)a.a.dlnps * ng + p] = dlnpsdt;
     }
   }
-  if (inverse_only && !a.dlnpdtg) return;  // uniform over the CTA
+  if (brief) return;  // uniform over the CTA
   __syncthreads();
 
   // phase 3
@@ -248,7 +302,7 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
   const R fcor = a.omega2 * a.sinlat[j];
   const R dphx = a.dphisdx[p], dphy = a.dphisdy[p];
   R uu[LB], vv[LB], idpa[LB];
-  R pkb3 = PK(L - b0), ipkb3 = crcp(pkb3);
+  R pkb3 = PK(L - b0), bpb3 = __ldg(bk + L - b0) * crcp(pkb3);
   R um = R(0), vm = R(0), tm = R(0);
   R uc = R(0), vc = R(0), tc = R(0);
   if (nb > 0) {
@@ -275,52 +329,54 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
       tp = S(a.s.tv + b + 1);
     }
     const R pkt = PK(t), pkt1 = pkb3, dp = pkt1 - pkt, idp = crcp(dp);
-    // 1/pk(t) is unused at the model top (pk = 0)
-    const R ipkt = kKeep ? ipks[t * 32 + lane] : (t > 0 ? crcp(pkt) : R(0)), ipk1 = ipkb3;
     pkb3 = pkt;
-    ipkb3 = ipkt;
     idpa[i] = idp;
-    const R rl = kKeep ? rls[t * 32 + lane] : RLN(t, pkt, pkt1);
-    const R al = (t == 0) ? a.log2sp : R(1) - (pkt * idp) * rl;
+    const R bkt = __ldg(bk + t), bkt1 = __ldg(bk + t + 1);
+    const R bp1 = bpb3;  // bk(t+1) / p(t+1)
+    R rl, al, bpt;
+    if (kKeep) {
+      rl = rls[t * 32 + lane];
+      al = als[t * 32 + lane];
+      bpt = bps[t * 32 + lane];
+    } else {
+      bpt = t > 0 ? bkt * crcp(pkt) : R(0);
+      rl = a.rlnp_top;
+      al = a.log2sp;
+      if (t > 0) {
+        rl = clog(cdiv((float)pkt1, (float)pkt));
+        al = R(1) - (pkt * idp) * rl;
+      }
+    }
+    bpb3 = bpt;
     const R cg = uc * dlx + vc * dly;
     const R dv = S(a.s.div + b);
     const R dbkt = __ldg(dbk + t);
+    const R pcg = ps * cg;
     R wb, wc;
     if (t == 0) {
-      wb = al * (dv * dp + ps * (cg * dbkt) * dbkt);
-      wc = ps * cg * dbkt;
+      wb = al * (dv * dp + pcg * dbkt * dbkt);
+      wc = pcg * dbkt;
     } else {
-      wb = rl * (xdb[i] + ps * xcb[i]) + al * (dv * dp + ps * cg * dbkt);
-      wc = ps * cg * (dbkt + __ldg(a.ck + t) * rl * idp);
+      wb = rl * (xdb[i] + ps * xcb[i]) + al * (dv * dp + pcg * dbkt);
+      wc = pcg * (dbkt + __ldg(a.ck + t) * (rl * idp));
     }
     const R dlnpdt = (wc - wb) * idp;  // omega / p
     if (a.dlnpdtg && valid) a.dlnpdtg[(long)b * ng + p] = dlnpdt;
     if (!inverse_only) {
       const R dtx = S(a.s.dtvdx + b), dty = S(a.s.dtvdy + b);
-      const R bkt = __ldg(bk + t), bkt1 = __ldg(bk + t + 1);
-      const R cofb2 = -rd * S2, px3u = -rd * SU, px3v = -rd * SV;
-      const R cofb1 = (t == 0) ? -idp * (al * dbkt) : -idp * (bkt * rl + al * dbkt);
-      const R cofa = -idp * (bkt1 * pkt * ipk1 - bkt + rl * (bkt - pkt * dbkt * idp));
-      const R prsgx =
-          cofb1 * rd * tc * ps * dlx - dphx + cofb2 * ps * dlx + px3u - rd * al * dtx - cofa * rd * tc * ps * dlx;
-      const R prsgy =
-          cofb1 * rd * tc * ps * dly - dphy + cofb2 * ps * dly + px3v - rd * al * dty - cofa * rd * tc * ps * dly;
+      // the pressure gradient's factor of R_d Tv ps grad ln ps, cofb1 - cofa of
+      // dyn_run.f90:405-415: with alfa = 1 - pk/dpk rlnp all but -bk(t+1)/pk(t+1)
+      // cancels; the top layer's alfa and rlnp are constants of their own
+      const R pc = t == 0 ? idp * (bkt1 * pkt * crcp(pkt1) - bkt + rl * (bkt - pkt * dbkt * idp) - al * dbkt) : -bp1;
+      const R com = (rd * ps) * (pc * tc - S2);
+      const R prsgx = (com * dlx - dphx) - rd * (SU + al * dtx);
+      const R prsgy = (com * dly - dphy) - rd * (SV + al * dty);
       const R e1 = ETA(t + 1), e0 = ETA(t);
       const R h = R(0.5) * idp;
-      R vu = R(0), vvv = R(0), vt = R(0);
-      if (b > 0) {
-        vu += e1 * (um - uc);
-        vvv += e1 * (vm - vc);
-        vt += e1 * (tm - tc);
-      }
-      if (b + 1 < L) {
-        vu += e0 * (uc - up);
-        vvv += e0 * (vc - vp);
-        vt += e0 * (tc - tp);
-      }
-      vu *= h;
-      vvv *= h;
-      vt *= h;
+      const R h1 = b > 0 ? h * e1 : R(0), h0 = b + 1 < L ? h * e0 : R(0);
+      const R vu = h1 * (um - uc) + h0 * (uc - up);
+      const R vvv = h1 * (vm - vc) + h0 * (vc - vp);
+      const R vt = h1 * (tm - tc) + h0 * (tc - tp);
       R vq = a.kappa * dlnpdt * tc;
       if (a.nt > 0) vq = cdiv(vq, R(1) + a.cvap_cp * S(a.s.trc + b));
       const R vr = S(a.s.vrt + b);
@@ -329,7 +385,7 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
       A(a.a.fv + b, vc * (vr + fcor) - (vu - prsgx));
       A(a.a.ke + b, R(0.5) * (uc * uc + vc * vc));
       if (t > 0) {
-        S2 += (bkt1 * ipk1 - bkt * ipkt) * tc;
+        S2 += (bp1 - bpt) * tc;
         SU += rl * dtx;
         SV += rl * dty;
       }
@@ -389,8 +445,8 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
         dA = dN;
       }
       const R idp = idpa[i];
-      const R vadq = idp * ((hb * e1 - ht * e0) + (q0 * (e0 - e1)));
-      A(a.a.qtend + iq * L + b, -uu[i] * gqx[i] - vv[i] * gqy[i] - vadq);
+      const R vadq = (hb * e1 - ht * e0) + (q0 * (e0 - e1));
+      A(a.a.qtend + iq * L + b, -uu[i] * gqx[i] - vv[i] * gqy[i] - idp * vadq);
       hb = ht;
       e1 = e0;
       q0 = q1;
@@ -404,7 +460,7 @@ template <typename R, int LB, int NWM>
 static void launch_cols_lb(const ColumnArgs<R>& a, bool inverse_only, cudaStream_t s) {
   const long ng = (long)a.nlon * a.nlat;
   const int nw = ceil_div(a.L, LB);
-  const size_t sm = (size_t)(5 * nw + 2 + a.L + 1 + (sizeof(R) == 8 ? 2 * a.L : 0)) * 32 * sizeof(R);
+  const size_t sm = (size_t)(5 * nw + 2 + a.L + 1 + (sizeof(R) == 8 ? 3 * a.L : 0)) * 32 * sizeof(R);
   if (sm > 48 * 1024)
     GD_CUDA(cudaFuncSetAttribute(k_dyn_columns<R, LB, NWM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   k_dyn_columns<R, LB, NWM><<<(unsigned)ceil_div(ng, 32), dim3(32, nw), sm, s>>>(a, inverse_only ? 1 : 0);
