@@ -129,7 +129,8 @@ class Dycore : public DycoreBase {
   // vertical coordinate, damping, semi-implicit matrices
   R *ak = nullptr, *bk = nullptr, *dbk = nullptr, *ck = nullptr;
   R *lapv = nullptr, *disspec = nullptr, *diff_prof = nullptr, *dmp_prof = nullptr;
-  R *amhyb = nullptr, *bmhyb = nullptr, *svhyb = nullptr, *tor = nullptr, *dhyb = nullptr;
+  R *gw = nullptr, *tor = nullptr, *dhyb = nullptr;  // gw, svs_: StageArgs' operators
+  double svs_ = 0.0;
   // state and work buffers
   R *S = nullptr, *S0 = nullptr, *TD[3] = {nullptr, nullptr, nullptr}, *AP = nullptr, *AH = nullptr;
   R *FPb = nullptr, *FHb = nullptr, *gS = nullptr, *gA = nullptr;
@@ -599,17 +600,19 @@ class Dycore : public DycoreBase {
     // the r_kind values (semimp_data.f90:130,216-234)
     for (auto* v : {&am, &bm, &sv, &to})
       for (auto& x : *v) x = (double)(R)x;
-    // the stage kernel reads the L x L operators transposed (coalesced over
-    // the output level): upload A^T, B^T, and invert Y^T = (inv Y)^T below
-    std::vector<double> amT((long)L * L), bmT((long)L * L);
-    for (int i = 0; i < L; ++i)
-      for (int j = 0; j < L; ++j) {
-        amT[(long)j * L + i] = am[(long)i * L + j];
-        bmT[(long)j * L + i] = bm[(long)i * L + j];
-      }
-    amhyb = upload(toR(amT));
-    bmhyb = upload(toR(bmT));
-    svhyb = upload(toR(sv));
+    // the operators as the stage kernel applies them (smem_scan): A(k, j) is
+    // the same for every k > j, B(k, j) a factor of k times dpk(j) for j > k
+    std::vector<double> gv((size_t)5 * L, 0.0);
+    for (int k = 0; k < L; ++k) {
+      const int t = L - 1 - k;  // top to bottom
+      gv[k] = am[(long)k * L + k];
+      gv[L + k] = k + 1 < L ? am[(long)(k + 1) * L + k] : 0.0;
+      gv[2 * L + k] = bm[(long)k * L + k];
+      gv[3 * L + k] = t > 0 ? (KAPPA * TREF / dpkref[t]) * log(pkref[t + 1] / pkref[t]) : 0.0;
+      gv[4 * L + k] = dpkref[t];
+    }
+    gw = upload(toR(gv));
+    svs_ = 1.0 / PREF;
     tor = upload(toR(to));
     std::vector<double> ym((long)L * L);
     for (int i = 0; i < L; ++i) {
@@ -879,9 +882,8 @@ class Dycore : public DycoreBase {
     a.TD1 = TD[1];
     a.TD2 = TD[2];
     a.ldTD = ldTD;
-    a.amhyb = amhyb;
-    a.bmhyb = bmhyb;
-    a.svhyb = svhyb;
+    a.gw = gw;
+    a.svs = (R)svs_;
     a.tor = tor;
     a.dhyb = dhyb;
     a.disspec = disspec;

@@ -74,8 +74,7 @@ __device__ __forceinline__ void smem_matvec_even(const R* __restrict__ AT, const
 // of two coefficients when four would leave threads of the group idle.
 // Odd L: one level per thread.  Rows past cnt are computed from unused
 // shared memory and not stored.  Every output sums over j in order, so both
-// forms give the same bits.  Threads t = 0 .. nt-1 of a group share the work
-// (two independent products run side by side on the two halves of a CTA).
+// forms give the same bits.  Threads t = 0 .. nt-1 of a group share the work.
 // st(i, k, y) takes output (i, k): stores it, or folds the step that uses it
 // into the product's epilogue
 template <typename V>
@@ -126,33 +125,54 @@ __device__ __forceinline__ void smem_matvec(const R* __restrict__ AT, const V* X
   }
 }
 
-// Y3[i] = sum_k w[k] X[i][k] for i < cnt: eight threads per coefficient, each
-// summing every eighth level, then a shuffle tree over the eight.  The group
-// (nt threads, a multiple of 32) runs whole warps, all of them to the end.
-template <typename R, typename V, typename St>
-__device__ __forceinline__ void smem_dot(const R* __restrict__ w, const V* X, St st, int L, int cnt, int t, int nt) {
-  const int g = t & 7, per = nt >> 3;
-  for (int base = 0; base < cnt; base += per) {
-    const int i = base + (t >> 3);
-    R sx = R(0), sy = R(0);
-    if (i < cnt)
-      for (int k = g; k < L; k += 8) {
-        const R wk = __ldg(w + k);
-        sx += wk * X[i * L + k].x;
-        sy += wk * X[i * L + k].y;
-      }
+// The gravity-wave operators are semiseparable: A(k, j) = c_j below the
+// diagonal (the hydrostatic sum over the layers under k) and B(k, j) = g_k d_j
+// above it (the divergence of the layers over k), so their products with a
+// column are a running sum and a multiply-add per level instead of L
+// multiply-adds.  Sixteen threads per coefficient, each a block of adjacent
+// levels: block sums, a shuffle scan over the sixteen, then the block again
+// with its offset.  Three of the stage's four L x L products went this way:
+// k_stage of a step (three launches) T254L64 FP64 state 8.36 -> 3.38 ms (FP64
+// pipe), T126L64 2.41 -> 0.99 ms, T574L64 FP32 3.45 -> 3.06 ms (memory).
+// f(i, k, x, run) gets level k's value and the sum of w x
+// over the levels below it (UP) or above it; the sum over all levels is
+// returned to all sixteen.  All threads of the CTA call it.
+template <typename R, typename V, bool UP, typename F>
+__device__ __forceinline__ V smem_scan(const R* __restrict__ w, const V* X, int L, int cnt, F f) {
+  static_assert(QC == 16, "one pass of 256 threads covers the CTA's coefficients");
+  const int i = threadIdx.x >> 4, g = threadIdx.x & 15, per = (L + 15) >> 4;
+  const int k0 = g * per, k1 = i < cnt ? min(L, k0 + per) : k0;
+  V s = vz<V>();
+  for (int k = k0; k < k1; ++k) {
+    const V x = X[i * L + k];
+    s.x += w[k] * x.x;
+    s.y += w[k] * x.y;
+  }
+  V inc = s;  // inclusive scan over the blocks, from the bottom or from the top
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      sx += __shfl_xor_sync(0xffffffffu, sx, o);
-      sy += __shfl_xor_sync(0xffffffffu, sy, o);
-    }
-    if (g == 0 && i < cnt) {
-      V y;
-      y.x = sx;
-      y.y = sy;
-      st(i, 0, y);
+  for (int o = 1; o < 16; o <<= 1) {
+    V y;
+    y.x = UP ? __shfl_up_sync(0xffffffffu, inc.x, o, 16) : __shfl_down_sync(0xffffffffu, inc.x, o, 16);
+    y.y = UP ? __shfl_up_sync(0xffffffffu, inc.y, o, 16) : __shfl_down_sync(0xffffffffu, inc.y, o, 16);
+    if (UP ? g >= o : g + o < 16) {
+      inc.x += y.x;
+      inc.y += y.y;
     }
   }
+  V run, tot;
+  run.x = UP ? __shfl_up_sync(0xffffffffu, inc.x, 1, 16) : __shfl_down_sync(0xffffffffu, inc.x, 1, 16);
+  run.y = UP ? __shfl_up_sync(0xffffffffu, inc.y, 1, 16) : __shfl_down_sync(0xffffffffu, inc.y, 1, 16);
+  if (g == (UP ? 0 : 15)) run = vz<V>();
+  tot.x = __shfl_sync(0xffffffffu, inc.x, UP ? 15 : 0, 16);
+  tot.y = __shfl_sync(0xffffffffu, inc.y, UP ? 15 : 0, 16);
+  for (int q = 0; q < k1 - k0; ++q) {
+    const int k = UP ? k0 + q : k1 - 1 - q;
+    const V x = X[i * L + k];
+    f(i, k, x, run);
+    run.x += w[k] * x.x;
+    run.y += w[k] * x.y;
+  }
+  return tot;
 }
 
 template <typename R>
@@ -213,13 +233,22 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? GD_STAGE_MINB : 2) k_sta
   }
   for (int i = threadIdx.x; i < cnt; i += blockDim.x) LN[i] = ld2(a.S, IDX(i), a.ldS, a.sc.lnps);
   __syncthreads();
-  const int th = (int)blockDim.x >> 1;  // half of the CTA, whole warps
+  // coefficients of the gravity-wave operators (see smem_scan)
+  const R *aD = a.gw, *aC = aD + L, *bD = aC + L, *bG = bD + L, *dP = bG + L;
+  const int ci = threadIdx.x >> 4;  // the coefficient this thread scans
+  const bool lead = (threadIdx.x & 15) == 0 && ci < cnt;
   if (!a.explicit_) {  // linear terms on the current state (run.f90:329-335)
-    if ((int)threadIdx.x < th) {
-      smem_matvec<R, V>(a.amhyb, TV, MvStore<V>{Y, L}, L, cnt, threadIdx.x, th);
-    } else {
-      smem_matvec<R, V>(a.bmhyb, DV, MvStore<V>{Y2, L}, L, cnt, threadIdx.x - th, th);
-      smem_dot<R, V>(a.svhyb, DV, MvStore<V>{Y3, 1}, L, cnt, threadIdx.x - th, th);  // Y3[i]
+    smem_scan<R, V, true>(aC, TV, L, cnt, [&](int i, int k, V x, V run) {
+      Y[i * L + k].x = aD[k] * x.x + run.x;
+      Y[i * L + k].y = aD[k] * x.y + run.y;
+    });
+    const V tot = smem_scan<R, V, false>(dP, DV, L, cnt, [&](int i, int k, V x, V run) {
+      Y2[i * L + k].x = bD[k] * x.x + bG[k] * run.x;
+      Y2[i * L + k].y = bD[k] * x.y + bG[k] * run.y;
+    });
+    if (lead) {
+      Y3[ci].x = a.svs * tot.x;
+      Y3[ci].y = a.svs * tot.y;
     }
   }
   __syncthreads();
@@ -355,38 +384,24 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? GD_STAGE_MINB : 2) k_sta
   __syncthreads();
   if (!a.explicit_ && a.cimp != R(0)) {  // implicit solve for divergence
     const R c = a.cimp;
-    // right-hand side r = D - c lap dt (A T + tor ln ps), formed in the
-    // epilogue of the A T product
-    smem_matvec<R, V>(
-        a.amhyb, TV,
-        [&](int i, int k, V y) {
-          V r;
-          r.x = DV[i * L + k].x - c * lap * dt * (y.x + a.tor[k] * LN[i].x);
-          r.y = DV[i * L + k].y - c * lap * dt * (y.y + a.tor[k] * LN[i].y);
-          Y2[i * L + k] = r;
-        },
-        L, cnt, threadIdx.x, blockDim.x);
+    // right-hand side r = D - c lap dt (A T + tor ln ps)
+    smem_scan<R, V, true>(aC, TV, L, cnt, [&](int i, int k, V x, V run) {
+      Y2[i * L + k].x = DV[i * L + k].x - c * lap * dt * (aD[k] * x.x + run.x + a.tor[k] * LN[i].x);
+      Y2[i * L + k].y = DV[i * L + k].y - c * lap * dt * (aD[k] * x.y + run.y + a.tor[k] * LN[i].y);
+    });
     __syncthreads();
     const R* D = a.dhyb + ((long)s * (a.T + 1) + n) * L * L;
     smem_matvec<R, V>(D, Y2, MvStore<V>{DV, L}, L, cnt, threadIdx.x, blockDim.x);
     __syncthreads();
-    // back-substitution into T and ln ps in the epilogues of B D and sv . D
-    if ((int)threadIdx.x < th)
-      smem_matvec<R, V>(
-          a.bmhyb, DV,
-          [&](int i, int k, V y) {
-            TV[i * L + k].x -= c * dt * y.x;
-            TV[i * L + k].y -= c * dt * y.y;
-          },
-          L, cnt, threadIdx.x, th);
-    else
-      smem_dot<R, V>(
-          a.svhyb, DV,
-          [&](int i, int, V y) {
-            LN[i].x -= c * dt * y.x;
-            LN[i].y -= c * dt * y.y;
-          },
-          L, cnt, threadIdx.x - th, th);
+    // back-substitution into T and ln ps
+    const V tot = smem_scan<R, V, false>(dP, DV, L, cnt, [&](int i, int k, V x, V run) {
+      TV[i * L + k].x -= c * dt * (bD[k] * x.x + bG[k] * run.x);
+      TV[i * L + k].y -= c * dt * (bD[k] * x.y + bG[k] * run.y);
+    });
+    if (lead) {
+      LN[ci].x -= c * dt * (a.svs * tot.x);
+      LN[ci].y -= c * dt * (a.svs * tot.y);
+    }
     __syncthreads();
   }
   for (int e = threadIdx.x; e < L * cnt; e += blockDim.x) {

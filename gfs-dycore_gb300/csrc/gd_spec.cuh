@@ -39,9 +39,11 @@ struct StageArgs {
   R* TD1;
   R* TD2;
   long ldTD;
-  const R* amhyb;  // [L][L] transposed: amhyb[j][k] = A(k, j), k = output level
-  const R* bmhyb;  // transposed likewise
-  const R* svhyb;  // [L]
+  // gravity-wave operators of the state's columns, levels bottom to top, [5][L]:
+  // A(k, k) | A(k, j), j < k | B(k, k) | B(k, j) / d_j, j > k | d_j; sv . D is
+  // svs times the sum of d_j D_j
+  const R* gw;
+  R svs;
   const R* tor;    // [L]
   const R* dhyb;   // [3][T+1][L][L], each matrix transposed
   const R* disspec;
