@@ -10,18 +10,20 @@
 // trained net is exactly the BF16 net it is evaluated as.
 //
 // The products with the batch (the grid's columns) as rows, X W^T and dZ W,
-// run on the tensor cores (k_tc_mlp in gd_tc.cu) when every layer is at most
-// 256 wide: the weights are exact in TF32 and each activation or gradient is
-// split into TF32 hi + lo, so two MMAs per K step give the FP32 products of
-// the BF16 net.  That covers inference (gd_mlp_forward and the closure in
-// the step), the training forward pass (which also stores each hidden
-// layer's Z and A) and the backward product dZ_l W_l with the GELU
-// derivative fused.  The weight gradient dZ^T A, a reduction over the batch,
-// runs on the tensor cores too (k_tc_wgrad): both operands transposed with
-// the batch contiguous and split hi + lo (k_tsplit), the batch in K slices
-// whose partial tiles k_wsum adds in order.  Nets wider than 256 (and
-// GD_MLP_TRAIN_TC=0) train on a tiled SIMT GEMM: 64 x 64 output tiles, K in
-// steps of 16 through shared memory, 4 x 4 outputs per thread, operands
+// run on the tensor cores when every layer is at most 256 wide: one launch
+// (k_tc_chain in gd_tc.cu) takes 128 rows through all layers with the
+// activations on chip, as BF16 hi + mid + lo slices against the BF16 weights,
+// so three MMAs per K step give the FP32 products of the BF16 net.  That
+// covers inference (gd_mlp_forward and the closure in the step), the training
+// forward pass (which also stores each hidden layer's Z and A) and the chain
+// of backward products dZ_l W_l with the GELU derivative fused.  The weights
+// it reads are packed (padded, and transposed for the backward chain) once
+// per update.  The weight gradients dZ^T A, reductions over the batch, run on
+// the tensor cores too (k_tc_wgrad, all layers in one launch): the operands
+// transposed with the batch contiguous and split hi + lo (k_tsplit), the batch
+// in slices whose partial tiles k_wsum adds in order.  Nets wider than 256
+// (and GD_MLP_TRAIN_TC=0) train on a tiled SIMT GEMM: 64 x 64 output tiles, K
+// in steps of 16 through shared memory, 4 x 4 outputs per thread, operands
 // addressed through (row, column) strides, split K for the weight gradient.
 #include <cuda_bf16.h>
 
@@ -38,6 +40,29 @@
 #include "gd_common.cuh"
 #include "gd_mlp.cuh"
 #include "gd_tc.cuh"
+
+namespace gd {
+// a packed weight row: cnt entries of the BF16 copy from off on, stride apart
+struct PackRow {
+  long off;
+  int stride, cnt;
+};
+// transposing split: src [n][w] (null: the batch's inputs) to rows of dh, dl;
+// boff >= 0: also the column sums, into the bias partials from boff on
+struct TsplitJob {
+  const float* src;
+  int w, boff;
+  uint32_t *dh, *dl;
+};
+// where a layer's gradient entries are: in the packed gradient (offw, offb),
+// the partial tiles and the bias partials
+struct WgradLayer {
+  long offw, offb, poff;
+  int fo, fi, Np, boff;
+};
+constexpr int kSlab = 32768;  // columns of the batch transposed at a time
+constexpr int kTrows = 128;   // columns of the batch per k_tsplit CTA
+}  // namespace gd
 
 struct gd_mlp {
   int device = 0;
@@ -58,40 +83,34 @@ struct gd_mlp {
   // activations: Z_l (pre-activation) and A_l (GELU) of each hidden layer,
   // the output and its gradient, two gradient buffers for the backward pass
   int bcap = 0;
-  float *zb = nullptr, *ab = nullptr, *yb = nullptr, *gy = nullptr, *g0 = nullptr, *g1 = nullptr;
+  float *zb = nullptr, *ab = nullptr, *yb = nullptr, *gy = nullptr, *g0 = nullptr, *g1 = nullptr;  // g0, g1: SIMT
   float* partial = nullptr;  // loss partial sums
   float* kpart = nullptr;    // split-K partial weight gradients
   float* lossd = nullptr;
-  // tensor-core inference (gd_tc.cu, k_tc_mlp): weights exact in TF32, padded
-  // to [Np][Kp] per layer; the input and hidden activations split hi + lo
-  bool tc = false;
-  std::vector<int> kp, npd;
-  std::vector<long> tcoff;
-  float* wtc = nullptr;
-  uint32_t *xh = nullptr, *xl = nullptr;
-  uint32_t* hh[2] = {nullptr, nullptr};
-  uint32_t* hl[2] = {nullptr, nullptr};
-  std::vector<gd::TcMlpLayer> layers;
-  // tensor-core training: the forward pass that keeps Z and A (tlayers) and
-  // the backward products dZ_l W_l (blayers, l >= 1) against the weights
-  // transposed to [npt][kpt] (wtct); the output gradient and the hidden
-  // gradients split hi + lo (gyh/gyl, dzh/dzl ping-pong)
-  bool tcb = false;
-  std::vector<int> kpt, npt;
-  std::vector<long> tctoff;
-  float* wtct = nullptr;
-  uint32_t *gyh = nullptr, *gyl = nullptr;
-  uint32_t* dzh[2] = {nullptr, nullptr};
-  uint32_t* dzl[2] = {nullptr, nullptr};
-  std::vector<gd::TcMlpLayer> tlayers, blayers;
-  // the weight gradients dZ_l^T A_{l-1}: dZ and the layer inputs transposed
-  // (batch contiguous) and split, the slices' partial tiles
-  std::vector<gd::TcWgrad> wgl;
+  // tensor-core chains (gd_tc.cu): the weights packed as rows of kpf BF16
+  // (wpf, every layer's W_l) and of kpb (wpb, the transposed W_l of l >= 1),
+  // each layer's block padded to 64 rows; pack = where each packed row comes
+  // from.  Layer tables (device): inference, training forward, backward.
+  bool tc = false, tcb = false;
+  int kpf = 0, kpb = 0;
+  long rowsf = 0, rowsb = 0;
+  std::vector<int> wrowf, wrowb;
+  __nv_bfloat16 *wpf = nullptr, *wpb = nullptr;
+  gd::PackRow* pack = nullptr;
+  CUtensorMap mapf, mapb;
+  gd::TcChainLayer *inf_layers = nullptr, *trn_layers = nullptr, *bwd_layers = nullptr;
+  float* dzb = nullptr;  // dZ of the hidden layers, [nl][bcap][nh]
+  // weight gradients: dZ^T and the layers' inputs transposed, stacked and
+  // split over a slab of the batch (kSlab columns at most), the slices'
+  // partial tiles, the bias gradients' partial sums
+  gd::TcWgrad wg;
   uint32_t *zth = nullptr, *ztl = nullptr, *ath = nullptr, *atl = nullptr;
-  float* wpart = nullptr;
-  int tcap = 0;        // batch capacity of the training buffers
-  int tbcap = 0;       // bcap the training layers were built over
-  int wsplit_max = 0;  // slices the partial buffer holds
+  gd::WgradLayer* wlay = nullptr;  // device, one per layer
+  gd::TsplitJob* jobs = nullptr;   // device, two per layer
+  float *wpart = nullptr, *bpart = nullptr;
+  int nbias = 0, opcols = 0;  // columns of the transposed operands (slab capacity)
+  int tcap = 0;               // batch capacity of the training buffers
+  int nsm = 0;
   int* terr = nullptr;
   cudaStream_t stream = nullptr;  // the stream the net's work runs on
   cudaStream_t own = nullptr;     // the net's own stream (destroyed with it)
@@ -313,64 +332,85 @@ __global__ void k_to_bf16(const float* p, __nv_bfloat16* w16, long n) {
     w16[i] = __float2bfloat16_rn(p[i]);
 }
 
-// a layer's BF16 weights as FP32 (exact in TF32), padded to [Np][Kp] with zeros
-__global__ void k_w_tc(const __nv_bfloat16* __restrict__ w, int fo, int fi, int Np, int Kp, float* __restrict__ o) {
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)Np * Kp; e += (long)gridDim.x * blockDim.x) {
-    const int n = (int)(e / Kp), k = (int)(e % Kp);
-    o[e] = (n < fo && k < fi) ? __bfloat162float(w[(long)n * fi + k]) : 0.f;
-  }
+// packed weight rows: row r < rowsf of the forward pack, then the backward
+// pack's, zero past the row's entries; one CTA per row
+__global__ void k_pack(const __nv_bfloat16* __restrict__ w, const PackRow* __restrict__ rows, long rowsf, int kpf,
+                       int kpb, __nv_bfloat16* __restrict__ wpf, __nv_bfloat16* __restrict__ wpb) {
+  const long r = blockIdx.x;
+  const PackRow pr = rows[r];
+  const int kp = r < rowsf ? kpf : kpb;
+  __nv_bfloat16* o = r < rowsf ? wpf + r * kpf : wpb + (r - rowsf) * kpb;
+  for (int k = threadIdx.x; k < kp; k += blockDim.x)
+    o[k] = k < pr.cnt ? w[pr.off + (long)k * pr.stride] : __float2bfloat16_rn(0.f);
 }
-// the same weights transposed, [Np][Kp] with Np >= fi and Kp >= fo: the B
-// operand of the backward product dZ W
-__global__ void k_w_tc_t(const __nv_bfloat16* __restrict__ w, int fo, int fi, int Np, int Kp, float* __restrict__ o) {
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)Np * Kp; e += (long)gridDim.x * blockDim.x) {
-    const int n = (int)(e / Kp), k = (int)(e % Kp);
-    o[e] = (n < fi && k < fo) ? __bfloat162float(w[(long)k * fi + n]) : 0.f;
-  }
-}
-// rows r < nbc of src [n][w] (rows r >= n read as zero) transposed and
-// split to TF32 hi + lo: dh / dl [c][r], row pitch kp -- the operands of a
-// weight gradient, with the batch contiguous
-__global__ void k_tsplit(const float* __restrict__ src, int n, int w, int nbc, int kp, uint32_t* __restrict__ dh,
-                         uint32_t* __restrict__ dl) {
+// Operands of the weight gradients, every layer in one launch (blockIdx.z the
+// job): rows r0 + [0, nbc) of src [n][w] (rows past n read as zero) transposed
+// and split to TF32 hi + lo, dh / dl [c][r], row pitch kp, the batch
+// contiguous.  A CTA takes kTrows rows x 32 columns; for a dZ job it also adds
+// up its rows for the bias gradient (fixed order: eight strided sums, then
+// those in order), one partial per CTA.
+__global__ void __launch_bounds__(256) k_tsplit(const TsplitJob* __restrict__ jobs, const float* __restrict__ x,
+                                                long r0, int n, int nbc, int kp, float* __restrict__ bpart, int nbias) {
   __shared__ float t[32][33];
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    t[i][threadIdx.x] = (r < n && c < w) ? src[(long)r * w + c] : 0.f;
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < w && r < nbc) {
-      const float v = t[threadIdx.x][i];
-      const uint32_t h = (__float_as_uint(v) + 0x1000u) & 0xFFFFE000u;  // nearest TF32, ties away
-      dh[(long)c * kp + r] = h;
-      dl[(long)c * kp + r] = __float_as_uint(v - __uint_as_float(h));
+  const TsplitJob j = jobs[blockIdx.z];
+  const int c0 = blockIdx.y * 32, w = j.w;
+  if (c0 >= w) return;
+  const float* __restrict__ src = (j.src ? j.src : x) + r0 * w;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  float s = 0.f;
+  for (int b = 0; b < kTrows && blockIdx.x * kTrows + b < nbc; b += 32) {
+    const int rb = blockIdx.x * kTrows + b;
+#pragma unroll
+    for (int i = ty; i < 32; i += 8) {
+      const int r = rb + i, c = c0 + tx;
+      const float v = (r < n && c < w) ? src[(long)r * w + c] : 0.f;
+      t[i][tx] = v;
+      s += v;
     }
+    __syncthreads();
+#pragma unroll
+    for (int i = ty; i < 32; i += 8) {
+      const int c = c0 + i, r = rb + tx;
+      if (c < w && r < nbc) {
+        const float v = t[tx][i];
+        const uint32_t h = (__float_as_uint(v) + 0x1000u) & 0xFFFFE000u;  // nearest TF32, ties away
+        j.dh[(long)c * kp + r] = h;
+        j.dl[(long)c * kp + r] = __float_as_uint(v - __uint_as_float(h));
+      }
+    }
+    __syncthreads();
+  }
+  if (j.boff < 0) return;  // uniform over the CTA
+  t[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && c0 + tx < w) {
+    float v = 0.f;
+#pragma unroll
+    for (int y = 0; y < 8; ++y) v += t[y][tx];
+    bpart[(r0 / kTrows + blockIdx.x) * nbias + j.boff + c0 + tx] = v;
   }
 }
-// dW [fo][fi] = the sum of the slices' partial tiles [Mp][Np], in slice order
-__global__ void k_wsum(const float* __restrict__ part, int nsplit, int Mp, int Np, int fo, int fi,
-                       float* __restrict__ dw) {
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)fo * fi; e += (long)gridDim.x * blockDim.x) {
-    const int m = (int)(e / fi), c = (int)(e % fi);
+// the packed gradient: weights from the slices' partial tiles, biases from
+// their partial sums, each added in order
+__global__ void k_wsum(const WgradLayer* __restrict__ lay, int nlayer, long np, const float* __restrict__ part,
+                       long pstride, int nsplit, const float* __restrict__ bpart, int nbias, int nblk,
+                       float* __restrict__ grad) {
+  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < np; e += (long)gridDim.x * blockDim.x) {
+    int l = 0;
+    while (l + 1 < nlayer && e >= lay[l + 1].offw) ++l;
+    const WgradLayer L = lay[l];
     float s = 0.f;
-    for (int q = 0; q < nsplit; ++q) s += part[((long)q * Mp + m) * Np + c];
-    dw[e] = s;
-  }
-}
-// inputs x [n][nin] split to TF32 hi + lo rows of pitch Kp (the padding
-// columns stay zero from allocation)
-__global__ void k_split_in(const float* __restrict__ x, long n, int nin, int Kp, uint32_t* __restrict__ xh,
-                           uint32_t* __restrict__ xl) {
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < n * nin; e += (long)gridDim.x * blockDim.x) {
-    const long m = e / nin;
-    const int k = (int)(e % nin);
-    const float v = x[e];
-    const uint32_t h = (__float_as_uint(v) + 0x1000u) & 0xFFFFE000u;  // nearest TF32, ties away
-    xh[m * Kp + k] = h;
-    xl[m * Kp + k] = __float_as_uint(v - __uint_as_float(h));
+    if (e < L.offb) {
+      const int m = (int)((e - L.offw) / L.fi), c = (int)((e - L.offw) % L.fi);
+      const float* p = part + L.poff + (long)m * L.Np + c;
+#pragma unroll 4
+      for (int q = 0; q < nsplit; ++q) s += p[q * pstride];
+    } else {
+      const float* p = bpart + L.boff + (e - L.offb);
+#pragma unroll 4
+      for (int q = 0; q < nblk; ++q) s += p[(long)q * nbias];
+    }
+    grad[e] = s;
   }
 }
 
@@ -414,204 +454,130 @@ void to_bf16(gd_mlp* p) {
   count_launch();
   GD_LAUNCH_CHECK();
 }
+// after every change of the BF16 weights, on the stream that changed them
+void pack_weights(gd_mlp* p) {
+  if (!p->tc) return;
+  k_pack<<<(unsigned)(p->rowsf + p->rowsb), 64, 0, p->stream>>>(p->w16, p->pack, p->rowsf, p->kpf, p->kpb, p->wpf,
+                                                               p->wpb);
+  count_launch();
+  GD_LAUNCH_CHECK();
+}
 
 }  // namespace
 
 // --------------------------------------------------- shared with the dycore
-// Grows the activation buffers to ncols columns.  The old buffers are kept
-// until the net is destroyed: a context's captured step may still address
-// them (a step graph holds the buffers and tensor maps of its capture).
-void mlp_reserve(gd_mlp* p, int ncols) {
+// Buffers of a forward pass over ncols columns: none on the tensor cores
+// (activations stay on chip), the activations on the SIMT path.  Old buffers
+// are kept until the net is destroyed: a context's captured step may still
+// address them.
+void act_reserve(gd_mlp* p, int ncols) {
   if (ncols <= p->bcap) return;
   GD_CUDA(cudaStreamSynchronize(p->stream));
-  const long w = std::max(p->nh, std::max(p->nin, p->nout));
   p->zb = (float*)p->alloc(sizeof(float) * (size_t)p->nl * ncols * p->nh);
   p->ab = (float*)p->alloc(sizeof(float) * (size_t)p->nl * ncols * p->nh);
-  p->yb = (float*)p->alloc(sizeof(float) * (size_t)ncols * p->nout);
-  p->gy = (float*)p->alloc(sizeof(float) * (size_t)ncols * p->nout);
-  p->g0 = (float*)p->alloc(sizeof(float) * (size_t)ncols * w);
-  p->g1 = (float*)p->alloc(sizeof(float) * (size_t)ncols * w);
   p->bcap = ncols;
-  if (p->tc) {  // tensor-core operands (zero padding) and the layers' tensor maps
-    const int ldh = p->kp.size() > 1 ? p->kp[1] : p->kp[0];
-    auto z = [&](size_t words) {
-      uint32_t* b = (uint32_t*)p->alloc(sizeof(uint32_t) * words);
-      GD_CUDA(cudaMemsetAsync(b, 0, sizeof(uint32_t) * words, p->stream));
-      return b;
-    };
-    p->xh = z((size_t)ncols * p->kp[0]);
-    p->xl = z((size_t)ncols * p->kp[0]);
-    for (int i = 0; i < 2; ++i) {
-      p->hh[i] = z((size_t)ncols * ldh);
-      p->hl[i] = z((size_t)ncols * ldh);
-    }
-    GD_CUDA(cudaStreamSynchronize(p->stream));
-    p->layers.assign(p->nlayer, TcMlpLayer{});
-    for (int l = 0; l < p->nlayer; ++l) {
-      TcMlpLayer& L = p->layers[l];
-      L.M = ncols;
-      L.N = p->fout[l];
-      L.Np = p->npd[l];
-      L.Kp = p->kp[l];
-      L.bias = p->p32 + p->offb[l];
-      L.gelu = l < p->nl;
-      L.err = p->terr;
-      const uint32_t* ah = l == 0 ? p->xh : p->hh[(l - 1) & 1];
-      const uint32_t* al = l == 0 ? p->xl : p->hl[(l - 1) & 1];
-      if (L.gelu) {
-        L.oh = p->hh[l & 1];
-        L.ol = p->hl[l & 1];
-        L.ldo = ldh;
-      }
-      tc_mlp_maps(L, ah, al, p->wtc + p->tcoff[l]);
-    }
-  }
+}
+void mlp_reserve(gd_mlp* p, int ncols) {
+  if (!p->tc) act_reserve(p, ncols);
 }
 
 namespace {
 void forward_simt(gd_mlp* p, const float* x, int n, float* y, cudaStream_t s);
-// the tensor-core forward: weights refreshed from the BF16 copy, inputs
-// split, one k_tc_mlp launch per layer
-void forward_tc(gd_mlp* p, const float* x, int n, float* y, cudaStream_t s) {
-  for (int l = 0; l < p->nlayer; ++l) {
-    const long cnt = (long)p->npd[l] * p->kp[l];
-    k_w_tc<<<std::min(ceil_div(cnt, 256), 1024), 256, 0, s>>>(p->w16 + p->offw[l], p->fout[l], p->fin[l], p->npd[l],
-                                                              p->kp[l], p->wtc + p->tcoff[l]);
-  }
-  k_split_in<<<std::min(ceil_div((long)n * p->nin, 256), 8192), 256, 0, s>>>(x, n, p->nin, p->kp[0], p->xh, p->xl);
-  count_launch(p->nlayer + 1);
-  GD_LAUNCH_CHECK();
-  for (int l = 0; l < p->nlayer; ++l) {
-    TcMlpLayer L = p->layers[l];
-    L.M = n;  // rows past n are neither needed nor stored
-    if (!L.gelu) {
-      L.y = y;
-      L.ldy = p->nout;
-    }
-    tc_mlp_layer(L, s);
-  }
+template <typename X>
+X* to_device(gd_mlp* p, const std::vector<X>& h) {
+  X* d = (X*)p->alloc(sizeof(X) * h.size());
+  GD_CUDA(cudaMemcpy(d, h.data(), sizeof(X) * h.size(), cudaMemcpyHostToDevice));
+  return d;
 }
 }  // namespace
 
-// Training buffers (tensor-core path): the split gradients, the transposed
-// operands of the weight gradients and the slices' partial tiles for
-// batches of up to ncols, and the training layers over them and over the
-// activation buffers of mlp_reserve (rebuilt when those move).
+// Training buffers for batches of up to ncols columns, and on the tensor
+// cores the layer tables over them.
 void train_reserve(gd_mlp* p, int ncols) {
-  if (!p->tcb || (ncols <= p->tcap && p->tbcap == p->bcap)) return;
+  if (ncols <= p->tcap) return;
+  if (p->tcb && p->nin > 256)
+    throw std::invalid_argument("gd_mlp: training on the tensor cores takes at most 256 inputs");
+  act_reserve(p, ncols);
   GD_CUDA(cudaStreamSynchronize(p->stream));
-  auto z = [&](size_t words) {
-    uint32_t* b = (uint32_t*)p->alloc(sizeof(uint32_t) * words);
-    GD_CUDA(cudaMemsetAsync(b, 0, sizeof(uint32_t) * words, p->stream));
-    return b;
-  };
-  const int L1 = p->nlayer - 1;
-  const int ldd = (p->nh + 31) / 32 * 32;  // pitch of a hidden gradient's split (= kpt of a hidden layer)
-  if (ncols > p->tcap) {
-    const int cap = (ncols + 31) / 32 * 32;
-    int mp = 0, np = 0;
-    for (int l = 0; l < p->nlayer; ++l) {
-      mp = std::max(mp, (p->fout[l] + 127) / 128 * 128);
-      np = std::max(np, (p->fin[l] + 15) / 16 * 16);
-    }
-    int nsm = 0;
-    GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
-    p->wsplit_max = std::max(1, 2 * nsm);
-    p->gyh = z((size_t)cap * p->kpt[L1]);
-    p->gyl = z((size_t)cap * p->kpt[L1]);
-    for (int i = 0; i < 2; ++i) {
-      p->dzh[i] = z((size_t)cap * ldd);
-      p->dzl[i] = z((size_t)cap * ldd);
-    }
-    p->zth = z((size_t)mp * cap);
-    p->ztl = z((size_t)mp * cap);
-    p->ath = z((size_t)np * cap);
-    p->atl = z((size_t)np * cap);
-    p->wpart = (float*)p->alloc(sizeof(float) * (size_t)p->wsplit_max * mp * np);
-    p->tcap = cap;
+  const int cap = p->bcap;
+  p->yb = (float*)p->alloc(sizeof(float) * (size_t)cap * p->nout);
+  p->gy = (float*)p->alloc(sizeof(float) * (size_t)cap * p->nout);
+  p->tcap = cap;
+  if (!p->tcb) {
+    const long w = std::max(p->nh, std::max(p->nin, p->nout));
+    p->g0 = (float*)p->alloc(sizeof(float) * (size_t)cap * w);
+    p->g1 = (float*)p->alloc(sizeof(float) * (size_t)cap * w);
+    return;
   }
-  GD_CUDA(cudaStreamSynchronize(p->stream));
-  const int ncb = p->bcap;
-  p->tlayers = p->layers;
-  for (int l = 0; l < p->nl; ++l) {
-    TcMlpLayer& T = p->tlayers[l];
-    T.mode = 2;
-    T.z = p->zb + (size_t)l * ncb * p->nh;
-    T.act = p->ab + (size_t)l * ncb * p->nh;
-    T.ldz = p->nh;
-  }
-  p->tlayers[L1].y = p->yb;
-  p->tlayers[L1].ldy = p->nout;
-  // backward product of layer l: A = split dZ_l (the output gradient, or
-  // what layer l + 1 wrote), writes dZ_{l-1} to g0 / g1 and its split
-  p->blayers.assign(p->nlayer, TcMlpLayer{});
-  for (int l = 1; l < p->nlayer; ++l) {
-    TcMlpLayer& B = p->blayers[l];
-    const int out = (L1 - l) & 1;
-    B.M = p->tcap;  // the A operand's rows: the split gradients hold tcap
-    B.N = p->fin[l];
-    B.Np = p->npt[l];
-    B.Kp = p->kpt[l];
-    B.mode = 3;
-    B.err = p->terr;
-    B.zin = p->zb + (size_t)(l - 1) * ncb * p->nh;
-    B.ldz = p->nh;
-    B.y = out ? p->g1 : p->g0;
-    B.ldy = p->fin[l];
-    B.oh = p->dzh[out];
-    B.ol = p->dzl[out];
-    B.ldo = ldd;
-    const uint32_t* ah = l == L1 ? p->gyh : p->dzh[out ^ 1];
-    const uint32_t* al = l == L1 ? p->gyl : p->dzl[out ^ 1];
-    tc_mlp_maps(B, ah, al, p->wtct + p->tctoff[l]);
-  }
-  // weight gradients: A = dZ_l transposed (fout rows), B = the layer's input transposed (fin rows)
-  p->wgl.assign(p->nlayer, TcWgrad{});
+  const size_t act = (size_t)cap * p->nh;
+  p->dzb = (float*)p->alloc(sizeof(float) * (size_t)p->nl * act);
+  std::vector<TcChainLayer> f, b;
   for (int l = 0; l < p->nlayer; ++l) {
-    TcWgrad& W = p->wgl[l];
-    W.Mp = (p->fout[l] + 127) / 128 * 128;
-    W.Np = (p->fin[l] + 15) / 16 * 16;
-    W.part = p->wpart;
-    W.err = p->terr;
-    tc_wgrad_maps(W, p->zth, p->ztl, p->ath, p->atl, p->tcap);
+    TcChainLayer L{};
+    L.N = p->fout[l], L.K = p->fin[l], L.wrow = p->wrowf[l], L.bias = p->p32 + p->offb[l];
+    if (l < p->nl) L.act = 1, L.z = p->zb + l * act, L.out = p->ab + l * act, L.ldz = p->nh;
+    f.push_back(L);
   }
-  p->tbcap = p->bcap;
+  for (int l = p->nlayer - 1; l >= 1; --l) {  // dZ_{l-1} = (dZ_l W_l) GELU'(Z_{l-1})
+    TcChainLayer L{};
+    L.N = p->fin[l], L.K = p->fout[l], L.wrow = p->wrowb[l], L.act = 2;
+    L.zin = p->zb + (l - 1) * act, L.out = p->dzb + (l - 1) * act, L.ldz = p->nh;
+    b.push_back(L);
+  }
+  p->trn_layers = to_device(p, f);
+  p->bwd_layers = to_device(p, b);
+  // weight gradients: stacked transposed operands over a slab of the batch
+  const int cols = std::min((cap + 31) / 32 * 32, kSlab);
+  long ar = 0, br = 0, po = 0;
+  int bo = 0;
+  std::vector<TcWgradItem> items;
+  std::vector<WgradLayer> lay;
+  std::vector<long> arow, brow;
+  for (int l = 0; l < p->nlayer; ++l) {
+    const int Mp = (p->fout[l] + 127) / 128 * 128, Np = (p->fin[l] + 15) / 16 * 16;
+    arow.push_back(ar), brow.push_back(br);
+    for (int m = 0; m < Mp; m += 128) items.push_back({(int)ar + m, (int)br, Np, po + (long)m * Np});
+    lay.push_back({p->offw[l], p->offb[l], po, p->fout[l], p->fin[l], Np, bo});
+    ar += Mp, br += (p->fin[l] + 63) / 64 * 64, po += (long)Mp * Np, bo += p->fout[l];
+  }
+  if (cols > p->opcols) {  // rows past a layer's outputs or inputs stay zero
+    auto z = [&](size_t words) {
+      uint32_t* q = (uint32_t*)p->alloc(sizeof(uint32_t) * words);
+      GD_CUDA(cudaMemsetAsync(q, 0, sizeof(uint32_t) * words, p->stream));
+      return q;
+    };
+    p->zth = z((size_t)ar * cols), p->ztl = z((size_t)ar * cols);
+    p->ath = z((size_t)br * cols), p->atl = z((size_t)br * cols);
+    p->opcols = cols;
+    GD_CUDA(cudaStreamSynchronize(p->stream));
+  }
+  std::vector<TsplitJob> jobs;
+  for (int l = 0; l < p->nlayer; ++l) {
+    const size_t za = (size_t)arow[l] * p->opcols, ba = (size_t)brow[l] * p->opcols;
+    jobs.push_back({l == p->nlayer - 1 ? p->gy : p->dzb + l * act, p->fout[l], lay[l].boff, p->zth + za, p->ztl + za});
+    jobs.push_back({l == 0 ? nullptr : p->ab + (l - 1) * act, p->fin[l], -1, p->ath + ba, p->atl + ba});
+  }
+  p->jobs = to_device(p, jobs);
+  p->wlay = to_device(p, lay);
+  p->nbias = bo;
+  p->wg.items = to_device(p, items);
+  p->wg.nitems = (int)items.size();
+  p->wg.pstride = po;
+  p->wg.err = p->terr;
+  const int nslab = ceil_div(cap, kSlab);
+  p->wpart = (float*)p->alloc(sizeof(float) * (size_t)nslab * std::max(1, p->nsm / p->wg.nitems) * po);
+  p->wg.part = p->wpart;
+  p->bpart = (float*)p->alloc(sizeof(float) * (size_t)ceil_div(cap, kTrows) * bo);
+  tc_wgrad_maps(p->wg, p->zth, p->ztl, p->ath, p->atl, ar, br, p->opcols);
 }
-
-namespace {
-// the tensor-core forward of a training step: the hidden layers also keep
-// their pre-activations and activations (FP32) for the backward pass; the
-// transposed weights of the backward products are refreshed with the others
-void forward_tc_train(gd_mlp* p, const float* x, int n) {
-  cudaStream_t s = p->stream;
-  for (int l = 0; l < p->nlayer; ++l) {
-    const long cnt = (long)p->npd[l] * p->kp[l];
-    k_w_tc<<<std::min(ceil_div(cnt, 256), 1024), 256, 0, s>>>(p->w16 + p->offw[l], p->fout[l], p->fin[l], p->npd[l],
-                                                              p->kp[l], p->wtc + p->tcoff[l]);
-    if (l >= 1) {
-      const long ct = (long)p->npt[l] * p->kpt[l];
-      k_w_tc_t<<<std::min(ceil_div(ct, 256), 1024), 256, 0, s>>>(p->w16 + p->offw[l], p->fout[l], p->fin[l],
-                                                                  p->npt[l], p->kpt[l], p->wtct + p->tctoff[l]);
-    }
-  }
-  k_split_in<<<std::min(ceil_div((long)n * p->nin, 256), 8192), 256, 0, s>>>(x, n, p->nin, p->kp[0], p->xh, p->xl);
-  count_launch(2 * p->nlayer);
-  GD_LAUNCH_CHECK();
-  for (int l = 0; l < p->nlayer; ++l) {
-    TcMlpLayer L = p->tlayers[l];
-    L.M = n;
-    tc_mlp_layer(L, s);
-  }
-}
-}  // namespace
 
 // y [n][nout] = net(x [n][nin]) on stream s, on the tensor cores when the
-// shape allows (every layer at most 256 wide).  No allocation when n <= bcap.
+// shape allows (every layer at most 256 wide).  No allocation.
 void mlp_forward_on(gd_mlp* p, const float* x, int n, float* y, cudaStream_t s) {
-  if (n > p->bcap) throw std::invalid_argument("gd_mlp: batch above the reserved capacity");
+  if (!p->tc && n > p->bcap) throw std::invalid_argument("gd_mlp: batch above the reserved capacity");
   if (n <= 0) return;
   if (p->tc)
-    forward_tc(p, x, n, y, s);
+    tc_chain(p->mapf, p->inf_layers, p->nlayer, x, p->nin, n, y, p->nout, p->terr, s);
   else
     forward_simt(p, x, n, y, s);
 }
@@ -667,7 +633,7 @@ namespace {
 void loss_grad(gd_mlp* p, const float* x, const float* t, int n) {
   cudaStream_t s = p->stream;
   if (p->tcb)
-    forward_tc_train(p, x, n);
+    tc_chain(p->mapf, p->trn_layers, p->nlayer, x, p->nin, n, p->yb, p->nout, p->terr, s);
   else
     forward_simt(p, x, n, p->yb, s);
   const long cnt = (long)n * p->nout;
@@ -676,11 +642,32 @@ void loss_grad(gd_mlp* p, const float* x, const float* t, int n) {
   k_mse_final<<<1, KPART, 0, s>>>(p->partial, nb, cnt, p->lossd);
   count_launch(2);
   GD_LAUNCH_CHECK();
-  if (p->tcb) {  // the output gradient split, the A operand of the last layer's backward product
-    k_split_in<<<std::min(ceil_div(cnt, 256), 8192), 256, 0, s>>>(p->gy, n, p->nout, p->kpt[p->nlayer - 1], p->gyh,
-                                                                    p->gyl);
+  if (p->tcb) {
+    // dZ of every hidden layer, then all weight gradients, slab by slab of
+    // the batch: operands transposed and split (with the bias gradients'
+    // partial sums), partial tiles of slices of at least four chunks, as many
+    // as one wave of CTAs takes; last the sums over slices
+    tc_chain(p->mapb, p->bwd_layers, p->nl, p->gy, p->nout, n, p->dzb, p->nh, p->terr, s);
+    int wmax = 0, slices = 0;
+    for (int l = 0; l < p->nlayer; ++l) wmax = std::max(wmax, std::max(p->fout[l], p->fin[l]));
+    for (int r0 = 0; r0 < n; r0 += kSlab) {
+      const int m = std::min(kSlab, n - r0), nbc = (m + 31) / 32 * 32, nk = nbc / 32;
+      k_tsplit<<<dim3(ceil_div(nbc, kTrows), ceil_div(wmax, 32), 2 * p->nlayer), 256, 0, s>>>(
+          p->jobs, x, (long)r0, m, nbc, p->opcols, p->bpart, p->nbias);
+      count_launch();
+      GD_LAUNCH_CHECK();
+      int ns = std::max(1, std::min(nk / 4, std::max(1, p->nsm / p->wg.nitems)));
+      const int cps = (nk + ns - 1) / ns;
+      ns = (nk + cps - 1) / cps;  // every slice non-empty
+      tc_wgrad(p->wg, nk, cps, ns, slices, s);
+      slices += ns;
+    }
+    k_wsum<<<std::min(ceil_div(p->np, 256), 1024), 256, 0, s>>>(p->wlay, p->nlayer, p->np, p->wpart, p->wg.pstride,
+                                                               slices, p->bpart, p->nbias, ceil_div(n, kTrows),
+                                                               p->grad);
     count_launch();
     GD_LAUNCH_CHECK();
+    return;
   }
   // backward: dZ of layer l in cur; dW_l = dZ^T A_{l-1}, db_l = colsum dZ,
   // dZ_{l-1} = (dZ W_l) * GELU'(Z_{l-1})
@@ -688,33 +675,11 @@ void loss_grad(gd_mlp* p, const float* x, const float* t, int n) {
   for (int l = p->nlayer - 1; l >= 0; --l) {
     const int fi = p->fin[l], fo = p->fout[l];
     const float* Ain = l == 0 ? x : p->ab + (size_t)(l - 1) * p->bcap * p->nh;
-    if (p->tcb) {  // dW_l on the tensor cores: dZ and the input transposed and split, K = the batch in slices
-      const int nbc = (n + 31) / 32 * 32, nk = nbc / 32;
-      const TcWgrad& W = p->wgl[l];
-      int ns = std::max(1, std::min(nk / 4, std::max(1, p->wsplit_max / (W.Mp / 128))));  // >= 4 chunks per slice
-      const int cps = (nk + ns - 1) / ns;
-      ns = (nk + cps - 1) / cps;  // every slice non-empty
-      k_tsplit<<<dim3(nbc / 32, ceil_div(fo, 32)), dim3(32, 8), 0, s>>>(cur, n, fo, nbc, p->tcap, p->zth, p->ztl);
-      k_tsplit<<<dim3(nbc / 32, ceil_div(fi, 32)), dim3(32, 8), 0, s>>>(Ain, n, fi, nbc, p->tcap, p->ath, p->atl);
-      count_launch(2);
-      GD_LAUNCH_CHECK();
-      tc_wgrad(W, nk, cps, ns, s);
-      k_wsum<<<std::min(ceil_div((long)fo * fi, 256), 1024), 256, 0, s>>>(p->wpart, ns, W.Mp, W.Np, fo, fi,
-                                                                        p->grad + p->offw[l]);
-      count_launch();
-      GD_LAUNCH_CHECK();
-    } else {
-      gemm_splitk(fo, fi, n, cur, 1L, (long)fo, Ain, (long)fi, 1L, p->kpart, p->grad + p->offw[l], s);
-    }
+    gemm_splitk(fo, fi, n, cur, 1L, (long)fo, Ain, (long)fi, 1L, p->kpart, p->grad + p->offw[l], s);
     k_colsum<<<ceil_div(fo, 32), dim3(32, 8), 0, s>>>(cur, n, fo, p->grad + p->offb[l]);
     count_launch();
     GD_LAUNCH_CHECK();
-    if (l > 0 && p->tcb) {  // dZ_{l-1} on the tensor cores, stored and split for layer l - 1
-      TcMlpLayer B = p->blayers[l];
-      B.M = n;
-      tc_mlp_layer(B, s);
-      cur = B.y;
-    } else if (l > 0) {
+    if (l > 0) {
       float* nxt = (cur == p->g0) ? p->g1 : p->g0;
       const float* Zp = p->zb + (size_t)(l - 1) * p->bcap * p->nh;
       gemm(n, fi, fo, cur, (long)fo, 1L, p->w16 + p->offw[l], (long)fi, 1L, EpiGeluD{Zp, nxt, fi}, s);
@@ -755,32 +720,31 @@ int gd_mlp_init(int nin, int nhidden, int nlayers, int nout, unsigned long long 
     off += fo;
   }
   p->np = off;
-  // tensor-core inference when every layer is at most 256 wide
-  p->tc = true;
-  long toff = 0;
-  for (int l = 0; l < p->nlayer; ++l) {
-    p->kp.push_back((p->fin[l] + 31) / 32 * 32);
-    p->npd.push_back((p->fout[l] + 15) / 16 * 16);
-    if (p->npd[l] > 256) p->tc = false;
-    p->tcoff.push_back(toff);
-    toff += (long)p->npd[l] * p->kp[l];
-  }
-  // tensor-core training when the backward products dZ_l W_l fit as well
-  // (every layer's input at most 256 wide); GD_MLP_TRAIN_TC=0 keeps it on
-  // the SIMT kernels (a comparison knob)
+  // tensor cores when every layer is at most 256 wide (training too: the
+  // backward products' outputs are the hidden widths); GD_MLP_TRAIN_TC=0
+  // keeps training on the SIMT kernels (a comparison knob)
+  p->tc = nhidden <= 256 && nout <= 256;
   {
     const char* e = getenv("GD_MLP_TRAIN_TC");
     p->tcb = p->tc && !(e && e[0] == '0');
   }
-  long ttoff = 0;
+  std::vector<PackRow> pack;
+  auto block = [&](std::vector<int>& first, long& rows, int n, long off0, long offn, int stride, int cnt) {
+    first.push_back((int)rows);
+    for (int i = 0; i < (n + 63) / 64 * 64; ++i, ++rows)
+      pack.push_back(i < n ? PackRow{off0 + i * offn, stride, cnt} : PackRow{0, 0, 0});
+  };
   for (int l = 0; l < p->nlayer; ++l) {
-    p->kpt.push_back((p->fout[l] + 31) / 32 * 32);
-    p->npt.push_back((p->fin[l] + 15) / 16 * 16);
-    p->tctoff.push_back(ttoff);
-    if (l >= 1) {
-      if (p->npt[l] > 256) p->tcb = false;
-      ttoff += (long)p->npt[l] * p->kpt[l];
-    }
+    p->kpf = std::max(p->kpf, (p->fin[l] + 63) / 64 * 64);
+    block(p->wrowf, p->rowsf, p->fout[l], p->offw[l], p->fin[l], 1, p->fin[l]);
+  }
+  p->kpb = 64;
+  for (int l = 0; l < p->nlayer; ++l) {
+    p->kpb = std::max(p->kpb, (p->fout[l] + 63) / 64 * 64);
+    if (l == 0 || !p->tcb)
+      p->wrowb.push_back(0);
+    else
+      block(p->wrowb, p->rowsb, p->fin[l], p->offw[l], 1, p->fin[l], p->fout[l]);
   }
   // He-normal hidden weights, the output layer scaled by 0.1 (the net starts
   // close to no correction), zero biases
@@ -808,17 +772,32 @@ int gd_mlp_init(int nin, int nhidden, int nlayers, int nout, unsigned long long 
     p->in_sd = (float*)p->alloc(sizeof(float) * nin);
     p->out_mu = (float*)p->alloc(sizeof(float) * nout);
     p->out_sd = (float*)p->alloc(sizeof(float) * nout);
-    if (p->tcb) p->wtct = (float*)p->alloc(sizeof(float) * std::max(ttoff, 1L));
     if (p->tc) {
-      p->wtc = (float*)p->alloc(sizeof(float) * toff);
+      p->wpf = (__nv_bfloat16*)p->alloc(sizeof(__nv_bfloat16) * (size_t)p->rowsf * p->kpf);
+      tc_chain_map(&p->mapf, p->wpf, p->kpf, p->rowsf);
+      if (p->rowsb > 0) {
+        p->wpb = (__nv_bfloat16*)p->alloc(sizeof(__nv_bfloat16) * (size_t)p->rowsb * p->kpb);
+        tc_chain_map(&p->mapb, p->wpb, p->kpb, p->rowsb);
+      }
+      p->pack = to_device(p.get(), pack);
+      std::vector<TcChainLayer> inf;
+      for (int l = 0; l < p->nlayer; ++l) {
+        TcChainLayer L{};
+        L.N = p->fout[l], L.K = p->fin[l], L.wrow = p->wrowf[l], L.act = l < p->nl ? 1 : 0;
+        L.bias = p->p32 + p->offb[l];
+        inf.push_back(L);
+      }
+      p->inf_layers = to_device(p.get(), inf);
       p->terr = (int*)p->alloc(sizeof(int));
       GD_CUDA(cudaMemset(p->terr, 0, sizeof(int)));
+      GD_CUDA(cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, p->device));
     }
     GD_CUDA(cudaMemcpy(p->p32, h.data(), sizeof(float) * off, cudaMemcpyHostToDevice));
     GD_CUDA(cudaMemset(p->am, 0, sizeof(float) * off));
     GD_CUDA(cudaMemset(p->av, 0, sizeof(float) * off));
     GD_CUDA(cudaMemset(p->grad, 0, sizeof(float) * off));
     to_bf16(p.get());
+    pack_weights(p.get());
     GD_CUDA(cudaStreamSynchronize(p->stream));
   });
   if (rc != GD_OK) {
@@ -855,6 +834,7 @@ int gd_mlp_set_params(gd_mlp* p, const float* params) {
     GD_CUDA(cudaStreamSynchronize(p->stream));
     GD_CUDA(cudaMemcpy(p->p32, params, sizeof(float) * p->np, cudaMemcpyHostToDevice));
     to_bf16(p);
+    pack_weights(p);
     GD_CUDA(cudaStreamSynchronize(p->stream));
   });
 }
@@ -890,7 +870,6 @@ int gd_mlp_loss_grad(gd_mlp* p, const float* x, const float* t, int ncols, float
   return mguard(p, [&] {
     need_device(p, x, "x");
     need_device(p, t, "t");
-    mlp_reserve(p, ncols);
     train_reserve(p, ncols);
     loss_grad(p, x, t, ncols);
     mlp_check(p, p->stream);
@@ -904,7 +883,6 @@ int gd_mlp_train_step(gd_mlp* p, const float* x, const float* t, int ncols, floa
   return mguard(p, [&] {
     need_device(p, x, "x");
     need_device(p, t, "t");
-    mlp_reserve(p, ncols);
     train_reserve(p, ncols);
     loss_grad(p, x, t, ncols);
     ++p->adam_t;
@@ -914,6 +892,7 @@ int gd_mlp_train_step(gd_mlp* p, const float* x, const float* t, int ncols, floa
                                                                          lr, b1, b2, 1e-8f, c1, c2);
     count_launch();
     GD_LAUNCH_CHECK();
+    pack_weights(p);
     if (loss) {
       GD_CUDA(cudaMemcpyAsync(loss, p->lossd, sizeof(float), cudaMemcpyDeviceToHost, p->stream));
       mlp_check(p, p->stream);  // synchronises; raises a tensor-core wait that gave up

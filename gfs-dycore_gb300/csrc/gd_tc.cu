@@ -1575,218 +1575,337 @@ int tc_check(TcPlan& p, cudaStream_t s) {
 }
 
 
-// ------------------------------------------- closure network layers --
-// One CTA per 128 rows (grid columns of the closure); warp 0's first thread
-// issues the TMA copies of A hi, A lo and W per 32-wide K chunk into a
-// 3-stage ring, warp 1's first thread issues two MMAs per K step (hi W and
-// lo W; W is exact in TF32), all four warps drain the accumulator (warp w
-// holds TMEM lanes 32w..32w+31 = rows).  Every wait is bounded.
-struct TcMlpArgs {
-  int M, N, Np, nk;  // Np: this launch's N tile (each CTA covers columns blockIdx.y * Np ...)
-  const float* bias;
-  int gelu;
-  int mode;
-  float* z;
-  float* act;
-  const float* zin;
-  int ldz;
-  uint32_t* oh;
-  uint32_t* ol;
-  int ldo;
-  float* y;
+// ------------------------------------------------- closure network --
+// A chain of dense layers over 128 rows (grid columns of the closure) per
+// CTA, every activation kept on chip: the A operand of each layer sits in
+// tensor memory as three BF16 slices hi + mid + lo of the FP32 values (24
+// bits; the BF16 weights are exact), the accumulator beside it (TMEM: 128
+// columns of FP32 accumulator, 3 x 128 columns of A, K <= 256).  A layer's
+// outputs go in halves of 128: while the MMAs of the second half run, the
+// epilogue warps finish the first (bias, GELU, or the GELU derivative of the
+// backward chain) and hold it in shared memory; the split of all outputs then
+// overwrites A, whose last reader has completed.  Warp 0 streams the packed weights (TMA,
+// 128 outputs x 64 inputs per ring stage), one thread of warp 1 issues the
+// MMAs, warps 2-17 load the input rows, run the epilogues and feed tensor
+// memory (warp w: lane quadrant w % 4, 32-column group (w - 2) / 4).  A
+// first layer wider than 256 goes in K passes, its input rows read once per
+// half.  Every wait is bounded.
+//
+// One launch takes the place of a split of the inputs, a weight conversion
+// and a GEMM launch per layer with the activations through HBM as TF32 hi +
+// lo words: bound by the epilogues' GELU issue.
+constexpr int TCC_NS = 5;            // weight ring stages of 128 x 64 BF16 (16 KB)
+constexpr int TCC_EPI = 16;          // epilogue warps
+constexpr int TCC_THREADS = 64 + 32 * TCC_EPI;
+constexpr uint32_t TCC_STAGE = 128 * 128;
+constexpr int TCC_TP = 33;           // pitch of a warp's 32 x 32 staging tile (words)
+constexpr size_t TCC_SMEM = (size_t)TCC_NS * TCC_STAGE + (size_t)TCC_EPI * 2 * 32 * TCC_TP * 4 + 256 + 1024;
+
+struct TcChainArgs {
+  const TcChainLayer* layers;
+  int nl, M;
+  const float* x;
+  int ldx;
+  float* y;  // output of the last layer ([M][ldy])
   int ldy;
   int* err;
-  uint32_t idesc, tmem_cols;
 };
 
 __device__ __forceinline__ float tc_gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float tc_gelu_d(float z) {
   return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
+__device__ __forceinline__ void mma_bf16_ta(uint32_t dtmem, uint32_t atmem, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(dtmem),
+      "r"(atmem), "l"(b), "r"(idesc), "r"(acc));
+}
+// 32 consecutive K entries of a row (this thread's TMEM lane) as BF16 hi +
+// mid + lo, two entries per TMEM column, to columns t, t + 128, t + 256
+__device__ __forceinline__ void tc_split3_st(uint32_t t, const float* v) {
+  uint32_t h[16], m[16], l[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float x0 = v[2 * i], x1 = v[2 * i + 1];
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h[i]) : "f"(x1), "f"(x0));
+    const float r0 = x0 - __uint_as_float(h[i] << 16), r1 = x1 - __uint_as_float(h[i] & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(m[i]) : "f"(r1), "f"(r0));
+    const float q0 = r0 - __uint_as_float(m[i] << 16), q1 = r1 - __uint_as_float(m[i] & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l[i]) : "f"(q1), "f"(q0));
+  }
+  tmem_st16(t, h);
+  tmem_st16(t + 128, m);
+  tmem_st16(t + 256, l);
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 
-__global__ void __launch_bounds__(TC_THREADS, 1)
-    k_tc_mlp(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
-             const __grid_constant__ CUtensorMap mW, TcMlpArgs a) {
+__global__ void __launch_bounds__(TCC_THREADS, 1)
+    k_tc_chain(const __grid_constant__ CUtensorMap mW, TcChainArgs a) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~(uintptr_t)1023);
-  const uint32_t bytesA = TC_M * 128, bytesW = (uint32_t)a.Np * 128;
-  const uint32_t stage_bytes = 2 * bytesA + bytesW;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sm + TC_NS * stage_bytes);
-  uint64_t* empty = full + TC_NS;
-  uint64_t* done = empty + TC_NS;
+  float* tiles = reinterpret_cast<float*>(sm + TCC_NS * TCC_STAGE);
+  uint64_t* full = reinterpret_cast<uint64_t*>(tiles + TCC_EPI * 2 * 32 * TCC_TP);
+  uint64_t* empty = full + TCC_NS;
+  uint64_t* go = empty + TCC_NS;  // A written and accumulator free: the next batch of MMAs may start
+  uint64_t* mdone = go + 1;       // a batch of MMAs completed
+  uint64_t* done = mdone + 1;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * TC_M, c0 = blockIdx.y * a.Np;  // rows, and the first of the CTA's Np columns
+  const int m0 = blockIdx.x * TC_M;
 
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"(a.tmem_cols));
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    for (int s = 0; s < TC_NS; ++s) {
+    for (int s = 0; s < TCC_NS; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
       mbar_init(smem_u32(&empty[s]), 1);
     }
+    mbar_init(smem_u32(go), TCC_EPI);
+    mbar_init(smem_u32(mdone), 1);
     mbar_init(smem_u32(done), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tbase = *tslot;
+  const uint32_t tbase = *tslot, tA = tbase + 128u;
 
-  if (tid == 0) {  // ---- TMA producer
-    int fills[TC_NS] = {0, 0, 0};
-    for (int i = 0; i < a.nk; ++i) {
-      const int s = i % TC_NS, u = i / TC_NS;
-      if (u >= 1 && !mbar_wait(smem_u32(&empty[s]), (u - 1) & 1, a.err, 31)) break;
-      unsigned char* st = sm + s * stage_bytes;
-      const uint32_t fb = smem_u32(&full[s]);
-      mbar_expect_tx(fb, stage_bytes);
-      tma_2d(smem_u32(st), &mAh, i * 32, m0, fb);
-      tma_2d(smem_u32(st + bytesA), &mAl, i * 32, m0, fb);
-      tma_2d(smem_u32(st + 2 * bytesA), &mW, i * 32, c0, fb);
-      ++fills[s];
+  // every role walks the same batches: layer l, output half h, K pass p
+  // (only a first layer wider than 256 has more than one)
+  if (tid == 0) {  // ------------------------------------------- producer
+    int fills[TCC_NS] = {};
+    long g = 0;
+    TcRing rs;
+    bool bad = false;
+    for (int l = 0; l < a.nl && !bad; ++l) {
+      const int N = a.layers[l].N, K = a.layers[l].K, wrow = a.layers[l].wrow;
+      for (int h = 0; h * 128 < N && !bad; ++h)
+        for (int k = 0; k < K; k += 64, ++g) {  // passes are runs of four chunks
+          const int s = rs.slot;
+          if (g >= TCC_NS && !mbar_wait(smem_u32(&empty[s]), rs.ph ^ 1u, a.err, 31)) {
+            bad = true;
+            break;
+          }
+          const bool two = N - h * 128 > 64;
+          const uint32_t fb = smem_u32(&full[s]), st = smem_u32(sm + (size_t)s * TCC_STAGE);
+          mbar_expect_tx(fb, two ? TCC_STAGE : TCC_STAGE / 2);
+          tma_2d(st, &mW, k, wrow + h * 128, fb);
+          if (two) tma_2d(st + TCC_STAGE / 2, &mW, k, wrow + h * 128 + 64, fb);
+          ++fills[s];
+          rs.next(TCC_NS);
+        }
     }
-    for (int s = 0; s < TC_NS; ++s)  // never leave with copies in flight
+    for (int s = 0; s < TCC_NS; ++s)  // no copies left in flight at exit
       if (fills[s] > 0) mbar_wait(smem_u32(&full[s]), (fills[s] - 1) & 1, a.err, 32);
-  } else if (tid == 32) {  // ---- MMA issuer
-    for (int i = 0; i < a.nk; ++i) {
-      const int s = i % TC_NS, u = i / TC_NS;
-      if (!mbar_wait(smem_u32(&full[s]), u & 1, a.err, 33)) break;
-      tc_fence_after();
-      unsigned char* st = sm + s * stage_bytes;
-      const uint64_t dah = smem_desc(smem_u32(st)), dal = smem_desc(smem_u32(st + bytesA));
-      const uint64_t dw = smem_desc(smem_u32(st + 2 * bytesA));
-#pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4) {  // 4 MMAs of K = 8 per 128-byte row
-        const uint64_t o = (uint64_t)(2 * k4);
-        mma<TC_TF32>(tbase, dah + o, dw + o, a.idesc, (i > 0 || k4 > 0) ? 1u : 0u);
-        mma<TC_TF32>(tbase, dal + o, dw + o, a.idesc, 1u);
+  } else if (tid == 32) {  // ------------------------------------ MMA issuer
+    TcRing rs;
+    uint32_t batch = 0;
+    bool bad = false;
+    for (int l = 0; l < a.nl && !bad; ++l) {
+      const int N = a.layers[l].N, K = a.layers[l].K;
+      for (int h = 0; h * 128 < N && !bad; ++h) {
+        const int nn = (min(128, N - h * 128) + 15) & ~15;
+        const uint32_t idesc =
+            (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nn >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+        for (int kp = 0; kp < K && !bad; kp += 256, ++batch) {
+          if (!mbar_wait(smem_u32(go), batch & 1u, a.err, 33)) {
+            bad = true;
+            break;
+          }
+          tc_fence_after();
+          const int kn = min(256, K - kp);
+          for (int c = 0; c < kn; c += 64) {
+            const int s = rs.slot;
+            if (!mbar_wait(smem_u32(&full[s]), rs.ph, a.err, 34)) {
+              bad = true;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t db = smem_desc(smem_u32(sm + (size_t)s * TCC_STAGE));
+            const int steps = min(4, (kn - c + 15) >> 4);
+            for (int k4 = 0; k4 < steps; ++k4) {  // K = 16: 8 TMEM columns of A, 32 bytes of B
+              const uint32_t ta = tA + (uint32_t)(c / 2 + 8 * k4);
+              const uint64_t o = db + (uint64_t)(2 * k4);
+              mma_bf16_ta(tbase, ta, o, idesc, (kp > 0 || c > 0 || k4 > 0) ? 1u : 0u);
+              mma_bf16_ta(tbase, ta + 128u, o, idesc, 1u);
+              mma_bf16_ta(tbase, ta + 256u, o, idesc, 1u);
+            }
+            mma_commit(smem_u32(&empty[s]));
+            rs.next(TCC_NS);
+          }
+          if (!bad) mma_commit(smem_u32(mdone));
+        }
       }
-      mma_commit(smem_u32(&empty[s]));
     }
     mma_commit(smem_u32(done));  // every issued MMA has completed at done
+  } else if (warp >= 2) {  // -------------------------- rows and epilogues
+    const int q4 = warp & 3, cg = (warp - 2) >> 2;
+    float* tile = tiles + (warp - 2) * 2 * 32 * TCC_TP;
+    float* held = tile + 32 * TCC_TP + lane * TCC_TP;  // the thread's first half
+    const uint32_t lq = (uint32_t)(q4 * 32) << 16;
+    const int mr = m0 + q4 * 32;  // this warp's first row; the thread's own is mr + lane
+    uint32_t batch = 0;
+    bool bad = false;
+    // 32 rows x 32 columns, coalesced, through the warp's tile to the
+    // thread's own row (zero past the rows and columns there are)
+    auto load = [&](const float* __restrict__ src, int ld, int c0, int ncol, float* v) {
+      float t[32];
+#pragma unroll
+      for (int r = 0; r < 32; ++r)
+        t[r] = (mr + r < a.M && c0 + lane < ncol) ? src[(long)(mr + r) * ld + c0 + lane] : 0.f;
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < 32; ++r) tile[r * TCC_TP + lane] = t[r];
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 32; ++c) v[c] = tile[lane * TCC_TP + c];
+    };
+    auto store = [&](float* __restrict__ dst, int ld, int c0, int ncol, const float* v) {
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 32; ++c) tile[lane * TCC_TP + c] = v[c];
+      __syncwarp();
+      const int nr = min(32, a.M - mr);
+      if (c0 + lane < ncol)
+        for (int r = 0; r < nr; ++r) dst[(long)(mr + r) * ld + c0 + lane] = tile[r * TCC_TP + lane];
+    };
+    auto signal = [&] {  // this warp's TMEM stores and loads precede the next batch
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(go));
+    };
+    auto input = [&](int p, int K) {  // K pass p of the input rows into A
+#pragma unroll 1
+      for (int hh = 0; hh < 2; ++hh) {
+        if (256 * p + 128 * hh + 32 * cg >= ((K + 15) & ~15)) break;  // columns no K step reads
+        float v[32];
+        load(a.x, a.ldx, 256 * p + 128 * hh + 32 * cg, K, v);
+        tc_split3_st(tA + lq + (uint32_t)(64 * hh + 16 * cg), v);
+      }
+    };
+    const int K0 = a.layers[0].K, np0 = (K0 + 255) / 256;
+    input(0, K0);
+    signal();
+    for (int l = 0; l < a.nl && !bad; ++l) {
+      const TcChainLayer L = a.layers[l];
+      const int nhalf = (L.N + 127) / 128;
+      const bool last = l == a.nl - 1;
+#pragma unroll 1
+      for (int h = 0; h < nhalf && !bad; ++h) {
+        const int n0 = 128 * h + 32 * cg;
+        float v[32], zi[32];
+        if (L.act == 2) load(L.zin, L.ldz, n0, L.N, zi);
+        for (int p = 0; p < (l == 0 ? np0 : 1); ++p) {
+          if (p > 0) {  // the next K pass of a wide first layer
+            input(p, K0);
+            signal();
+          }
+          const bool ok = mbar_wait(smem_u32(mdone), batch & 1u, a.err, 35);
+          ++batch;
+          if (!__all_sync(0xffffffffu, ok)) {
+            bad = true;
+            break;
+          }
+          tc_fence_after();
+        }
+        if (bad) break;
+        tmem_ld16(tbase + lq + (uint32_t)(32 * cg), v);
+        tmem_ld16(tbase + lq + (uint32_t)(32 * cg + 16), v + 16);
+        if (h + 1 < nhalf) {  // the accumulator is drained: the next half may start
+          if (l == 0 && np0 > 1) input(0, K0);
+          signal();
+        }
+        if (L.bias) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c)
+            if (n0 + c < L.N) v[c] += __ldg(L.bias + n0 + c);
+        }
+        if (L.z) store(L.z, L.ldz, n0, L.N, v);
+        if (L.act == 1) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] = tc_gelu(v[c]);
+        } else if (L.act == 2) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] *= tc_gelu_d(zi[c]);
+        }
+        if (last) {
+          store(a.y, a.ldy, n0, L.N, v);
+          continue;
+        }
+        if (L.out) store(L.out, L.ldz, n0, L.N, v);
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+          if (n0 + c >= L.N) v[c] = 0.f;
+        if (h + 1 < nhalf) {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) held[c] = v[c];
+        } else {  // every MMA of this layer has read A
+          tc_split3_st(tA + lq + (uint32_t)(64 * h + 16 * cg), v);
+          if (h > 0) {
+#pragma unroll
+            for (int c = 0; c < 32; ++c) v[c] = held[c];
+            tc_split3_st(tA + lq + (uint32_t)(16 * cg), v);
+          }
+          signal();
+        }
+      }
+    }
   }
   __syncwarp();
-  // ---- epilogue
-  const bool ok = mbar_wait(smem_u32(done), 0, a.err, 34);
-  tc_fence_after();
-  const bool go = __all_sync(0xffffffffu, ok && *(volatile int*)a.err == 0);
-  if (go && a.mode >= 2) {
-    // training: each lane stages 64 accumulator columns of its row (plus the
-    // bias in the forward), then the warp finishes row after row with
-    // coalesced loads and stores: the forward stores z, gelu(z) and the split
-    // of gelu(z); the backward reads z of the layer below and stores
-    // dZ = acc * gelu'(z) and its split
-    constexpr int TP = 65;
-    uint32_t* th = reinterpret_cast<uint32_t*>(sm) + warp * (2 * 32 * TP);
-    const uint32_t tw = tbase + ((uint32_t)(warp * 32) << 16);
-    const int mw = m0 + warp * 32;
-    for (int g0 = 0; g0 < a.Np; g0 += 64) {
-      for (int g = g0; g < g0 + 64 && g < a.Np; g += 16) {
-        float v[16];
-        tmem_ld16(tw + g, v);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const int n = c0 + g + q;
-          th[lane * TP + (g + q - g0)] = __float_as_uint(v[q] + (a.mode == 2 && n < a.N ? a.bias[n] : 0.f));
-        }
-      }
-      __syncwarp();
-      for (int r = 0; r < 32; ++r) {
-        const int m = mw + r;
-        if (m >= a.M) break;
-#pragma unroll
-        for (int c = 0; c < 64; c += 32) {
-          const int n = c0 + g0 + c + lane;
-          if (g0 + c + lane < a.Np && n < a.N) {
-            const float v = __uint_as_float(th[r * TP + c + lane]);
-            const long iz = (long)m * a.ldz + n;
-            float o;  // the value the next product takes, split hi + lo
-            if (a.mode == 2) {
-              o = tc_gelu(v);
-              a.z[iz] = v;
-              a.act[iz] = o;
-            } else {
-              o = v * tc_gelu_d(a.zin[iz]);
-              a.y[(long)m * a.ldy + n] = o;
-            }
-            uint32_t h, l;
-            Elem<TC_TF32>::splitf(o, h, l);
-            a.oh[(long)m * a.ldo + n] = h;
-            a.ol[(long)m * a.ldo + n] = l;
-          }
-        }
-      }
-      __syncwarp();
-    }
-  } else if (go) {
-    // each lane finishes 64 columns of its row into the warp's part of the
-    // (now idle) ring, then the warp stores row after row: 128 contiguous
-    // bytes per store instead of 32 rows' scattered words
-    constexpr int TP = 65;  // tile pitch (words): conflict-free column writes
-    uint32_t* th = reinterpret_cast<uint32_t*>(sm) + warp * (2 * 32 * TP);
-    uint32_t* tl = th + 32 * TP;
-    const uint32_t tw = tbase + ((uint32_t)(warp * 32) << 16);
-    const int mw = m0 + warp * 32;
-    for (int g0 = 0; g0 < a.Np; g0 += 64) {
-      for (int g = g0; g < g0 + 64 && g < a.Np; g += 16) {
-        float v[16];
-        tmem_ld16(tw + g, v);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const int n = c0 + g + q;
-          const float z = v[q] + (n < a.N ? a.bias[n] : 0.f);
-          uint32_t h, l = 0;
-          if (a.gelu)
-            Elem<TC_TF32>::splitf(tc_gelu(z), h, l);
-          else
-            h = __float_as_uint(z);
-          th[lane * TP + (g + q - g0)] = h;
-          tl[lane * TP + (g + q - g0)] = l;
-        }
-      }
-      __syncwarp();
-      for (int r = 0; r < 32; ++r) {
-        const int m = mw + r;
-        if (m >= a.M) break;
-#pragma unroll
-        for (int c = 0; c < 64; c += 32) {
-          const int n = c0 + g0 + c + lane;
-          if (g0 + c + lane < a.Np && n < a.N) {
-            if (a.gelu) {
-              a.oh[(long)m * a.ldo + n] = th[r * TP + c + lane];
-              a.ol[(long)m * a.ldo + n] = tl[r * TP + c + lane];
-            } else {
-              a.y[(long)m * a.ldy + n] = __uint_as_float(th[r * TP + c + lane]);
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
+  mbar_wait(smem_u32(done), 0, a.err, 36);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(a.tmem_cols));
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(512u));
 }
 
-// Weight gradient of a closure layer (see TcWgrad): one CTA per 128 rows of
-// dZ^T and one slice of the batch; the producer loads A hi, A lo, B hi, B lo
-// per 32-deep K chunk into a 2-stage ring, the MMA thread issues three
-// products per K step into one accumulator, the four warps stage the
-// accumulator through the idle ring and store the slice's partial tile row
-// by row.  Every wait is bounded.
+void tc_chain_map(CUtensorMap* m, const void* w, int kpitch, long rows) {
+  if (kpitch < 64 || kpitch % 64 || rows < 64 || rows % 64) throw std::invalid_argument("tc_chain_map: bad shape");
+  const uint64_t d[2] = {(uint64_t)kpitch, (uint64_t)rows};
+  make_map(m, const_cast<void*>(w), TC_BF16, 2, d, 64, 64);
+}
+
+void tc_chain(const CUtensorMap& w, const TcChainLayer* layers, int nl, const float* x, int ldx, int M, float* y,
+              int ldy, int* err, cudaStream_t s) {
+  TcChainArgs a;
+  a.layers = layers;
+  a.nl = nl;
+  a.M = M;
+  a.x = x;
+  a.ldx = ldx;
+  a.y = y;
+  a.ldy = ldy;
+  a.err = err;
+  static bool attr = false;
+  if (!attr) {
+    GD_CUDA(cudaFuncSetAttribute(k_tc_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TCC_SMEM));
+    attr = true;
+  }
+  k_tc_chain<<<(M + TC_M - 1) / TC_M, TCC_THREADS, TCC_SMEM, s>>>(w, a);
+  count_launch();
+  GD_LAUNCH_CHECK();
+}
+
+// Weight gradients of all layers (see TcWgrad): one CTA per item -- 128 rows
+// of a layer's dZ^T and one slice of the batch; the producer loads A hi, A
+// lo, B hi, B lo per 32-deep K chunk into a 2-stage ring, the MMA thread
+// issues three products per K step into one accumulator, the four warps
+// stage the accumulator through the idle ring and store the slice's partial
+// tile row by row.  Every wait is bounded.
 constexpr int TCW_NS = 2;
 struct TcWgradArgs {
-  int Np, cps, nkt;  // chunks per slice, chunks in all
+  const TcWgradItem* items;
+  int cps, nkt;  // chunks per slice, chunks in all
+  int slice0;    // slices of earlier slabs of the batch
   float* part;
   long pstride;  // floats per slice
   int* err;
-  uint32_t idesc, tmem_cols;
 };
 
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -1794,20 +1913,21 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                const __grid_constant__ CUtensorMap mBh, const __grid_constant__ CUtensorMap mBl, TcWgradArgs a) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~(uintptr_t)1023);
-  const uint32_t bytesA = TC_M * 128, bytesB = (uint32_t)a.Np * 128;
+  const TcWgradItem it = a.items[blockIdx.x];
+  const int nb = (it.Np + 63) / 64;  // 64-row boxes of the B operand
+  const uint32_t bytesA = TC_M * 128, bytesB = (uint32_t)nb * 64 * 128;
   const uint32_t stage_bytes = 2 * bytesA + 2 * bytesB;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sm + TCW_NS * stage_bytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + TCW_NS * (2 * TC_M * 128 + 2 * 256 * 128));
   uint64_t* empty = full + TCW_NS;
   uint64_t* done = empty + TCW_NS;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * TC_M;
   const int ks = blockIdx.y * a.cps;           // this slice's first K chunk
   const int nk = max(0, min(a.cps, a.nkt - ks));  // its chunks (every slice has at least one)
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"(a.tmem_cols));
+                 "r"(256u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
@@ -1828,19 +1948,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     for (int i = 0; i < nk; ++i) {
       const int s = i % TCW_NS, u = i / TCW_NS;
       if (u >= 1 && !mbar_wait(smem_u32(&empty[s]), (u - 1) & 1, a.err, 41)) break;
-      unsigned char* st = sm + s * stage_bytes;
-      const uint32_t fb = smem_u32(&full[s]);
+      const uint32_t st = smem_u32(sm + s * stage_bytes), fb = smem_u32(&full[s]);
       const int x = (ks + i) * 32;
       mbar_expect_tx(fb, stage_bytes);
-      tma_2d(smem_u32(st), &mAh, x, m0, fb);
-      tma_2d(smem_u32(st + bytesA), &mAl, x, m0, fb);
-      tma_2d(smem_u32(st + 2 * bytesA), &mBh, x, 0, fb);
-      tma_2d(smem_u32(st + 2 * bytesA + bytesB), &mBl, x, 0, fb);
+      tma_2d(st, &mAh, x, it.arow, fb);
+      tma_2d(st + bytesA, &mAl, x, it.arow, fb);
+      for (int b = 0; b < nb; ++b) {
+        tma_2d(st + 2 * bytesA + b * 8192, &mBh, x, it.brow + 64 * b, fb);
+        tma_2d(st + 2 * bytesA + bytesB + b * 8192, &mBl, x, it.brow + 64 * b, fb);
+      }
       ++fills[s];
     }
     for (int s = 0; s < TCW_NS; ++s)  // never leave with copies in flight
       if (fills[s] > 0) mbar_wait(smem_u32(&full[s]), (fills[s] - 1) & 1, a.err, 42);
   } else if (tid == 32) {  // ---- MMA issuer
+    const uint32_t idesc =
+        (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(it.Np >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
     for (int i = 0; i < nk; ++i) {
       const int s = i % TCW_NS, u = i / TCW_NS;
       if (!mbar_wait(smem_u32(&full[s]), u & 1, a.err, 43)) break;
@@ -1851,16 +1974,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll
       for (int k4 = 0; k4 < 4; ++k4) {  // 4 K steps of 8 per 128-byte row
         const uint64_t o = (uint64_t)(2 * k4);
-        mma<TC_TF32>(tbase, dah + o, dbh + o, a.idesc, (i > 0 || k4 > 0) ? 1u : 0u);
-        mma<TC_TF32>(tbase, dah + o, dbl + o, a.idesc, 1u);
-        mma<TC_TF32>(tbase, dal + o, dbh + o, a.idesc, 1u);
+        mma<TC_TF32>(tbase, dah + o, dbh + o, idesc, (i > 0 || k4 > 0) ? 1u : 0u);
+        mma<TC_TF32>(tbase, dah + o, dbl + o, idesc, 1u);
+        mma<TC_TF32>(tbase, dal + o, dbh + o, idesc, 1u);
       }
       mma_commit(smem_u32(&empty[s]));
     }
     mma_commit(smem_u32(done));  // every issued MMA has completed at done
   }
   __syncwarp();
-  // ---- epilogue: the slice's partial tile, rows m0 + 32 w + r
+  // ---- epilogue: the slice's partial tile, rows 32 w + r of the item
   const bool ok = mbar_wait(smem_u32(done), 0, a.err, 44);
   tc_fence_after();
   const bool go = __all_sync(0xffffffffu, ok && *(volatile int*)a.err == 0);
@@ -1868,9 +1991,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     constexpr int TP = 65;
     uint32_t* th = reinterpret_cast<uint32_t*>(sm) + warp * (32 * TP);
     const uint32_t tw = tbase + ((uint32_t)(warp * 32) << 16);
-    float* out = a.part + (long)blockIdx.y * a.pstride + (long)(m0 + warp * 32) * a.Np;
-    for (int g0 = 0; g0 < a.Np; g0 += 64) {
-      for (int g = g0; g < g0 + 64 && g < a.Np; g += 16) {
+    float* out = a.part + (long)(a.slice0 + blockIdx.y) * a.pstride + it.poff + (long)(warp * 32) * it.Np;
+    for (int g0 = 0; g0 < it.Np; g0 += 64) {
+      for (int g = g0; g < g0 + 64 && g < it.Np; g += 16) {
         float v[16];
         tmem_ld16(tw + g, v);
 #pragma unroll
@@ -1881,7 +2004,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll
         for (int c = 0; c < 64; c += 32) {
           const int n = g0 + c + lane;
-          if (n < a.Np) out[(long)r * a.Np + n] = __uint_as_float(th[r * TP + c + lane]);
+          if (n < it.Np) out[(long)r * it.Np + n] = __uint_as_float(th[r * TP + c + lane]);
         }
       __syncwarp();
     }
@@ -1889,103 +2012,38 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(a.tmem_cols));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(256u));
 }
 
 void tc_wgrad_maps(TcWgrad& W, const uint32_t* ah, const uint32_t* al, const uint32_t* bh, const uint32_t* bl,
-                   int kpitch) {
-  if (W.Mp < TC_M || W.Mp % TC_M || W.Np < 16 || W.Np > 256 || W.Np % 16 || kpitch < 32 || kpitch % 32)
+                   long arows, long brows, int kpitch) {
+  if (arows < TC_M || arows % TC_M || brows < 64 || brows % 64 || kpitch < 32 || kpitch % 32)
     throw std::invalid_argument("tc_wgrad_maps: bad shape");
-  const uint64_t da[2] = {(uint64_t)kpitch, (uint64_t)W.Mp}, db[2] = {(uint64_t)kpitch, (uint64_t)W.Np};
+  const uint64_t da[2] = {(uint64_t)kpitch, (uint64_t)arows}, db[2] = {(uint64_t)kpitch, (uint64_t)brows};
   make_map(&W.ah, const_cast<uint32_t*>(ah), TC_TF32, 2, da, 32, TC_M);
   make_map(&W.al, const_cast<uint32_t*>(al), TC_TF32, 2, da, 32, TC_M);
-  make_map(&W.bh, const_cast<uint32_t*>(bh), TC_TF32, 2, db, 32, W.Np);
-  make_map(&W.bl, const_cast<uint32_t*>(bl), TC_TF32, 2, db, 32, W.Np);
+  make_map(&W.bh, const_cast<uint32_t*>(bh), TC_TF32, 2, db, 32, 64);
+  make_map(&W.bl, const_cast<uint32_t*>(bl), TC_TF32, 2, db, 32, 64);
 }
 
-void tc_wgrad(const TcWgrad& W, int nk, int cps, int nsplit, cudaStream_t s) {
+void tc_wgrad(const TcWgrad& W, int nk, int cps, int nsplit, int slice0, cudaStream_t s) {
   if (nk < 1 || cps < 1 || nsplit < 1 || (long)(nsplit - 1) * cps >= nk || (long)nsplit * cps < nk || !W.part)
     throw std::invalid_argument("tc_wgrad: bad K split");
   TcWgradArgs a;
-  a.Np = W.Np;
+  a.items = W.items;
   a.cps = cps;
   a.nkt = nk;
+  a.slice0 = slice0;
   a.part = W.part;
-  a.pstride = (long)W.Mp * W.Np;
+  a.pstride = W.pstride;
   a.err = W.err;
-  a.idesc = make_idesc(TC_TF32, W.Np);
-  a.tmem_cols = tmem_cols_for(W.Np / 2);  // a power of two >= Np (and >= 32)
-  const size_t sm = (size_t)TCW_NS * (2 * TC_M * 128 + 2 * (size_t)W.Np * 128) + 1024 + 256;
+  const size_t sm = (size_t)TCW_NS * (2 * TC_M * 128 + 2 * 256 * 128) + 1024 + 256;
   static bool attr = false;
   if (!attr) {
     GD_CUDA(cudaFuncSetAttribute(k_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     attr = true;
   }
-  k_tc_wgrad<<<dim3(W.Mp / TC_M, nsplit), TC_THREADS, sm, s>>>(W.ah, W.al, W.bh, W.bl, a);
-  count_launch();
-  GD_LAUNCH_CHECK();
-}
-
-void tc_mlp_maps(TcMlpLayer& L, const uint32_t* ah, const uint32_t* al, const float* w) {
-  if (L.Kp % 32 || L.Np % 16 || L.Np < 16 || L.Np > 256 || L.N > L.Np || L.M < 1)
-    throw std::invalid_argument("tc_mlp_maps: bad layer shape");
-  const uint64_t da[2] = {(uint64_t)L.Kp, (uint64_t)L.M}, dw[2] = {(uint64_t)L.Kp, (uint64_t)L.Np};
-  make_map(&L.ah, const_cast<uint32_t*>(ah), TC_TF32, 2, da, 32, TC_M);
-  make_map(&L.al, const_cast<uint32_t*>(al), TC_TF32, 2, da, 32, TC_M);
-  make_map(&L.w, const_cast<float*>(w), TC_TF32, 2, dw, 32, L.Np);
-  L.wbase = w;
-  L.wbox = L.Np;
-}
-
-void tc_mlp_layer(const TcMlpLayer& Lin, cudaStream_t s) {
-  // N tile: the whole padded width, halved (down to 32 columns, a multiple
-  // of 16) while the row tiles alone leave SMs idle; the weights' map is
-  // made again for a narrower box
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    GD_CUDA(cudaGetDevice(&dev));
-    GD_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  }
-  const int mt = (Lin.M + TC_M - 1) / TC_M;
-  int nt = Lin.Np;
-  while (nt >= 64 && (nt / 2) % 16 == 0 && (long)mt * ((Lin.Np + nt - 1) / nt) < nsm) nt /= 2;
-  TcMlpLayer L = Lin;
-  if (nt != L.wbox) {
-    if (!L.wbase) throw std::invalid_argument("tc_mlp_layer: layer without its weight map");
-    const uint64_t dw[2] = {(uint64_t)L.Kp, (uint64_t)L.Np};
-    make_map(&L.w, const_cast<float*>(L.wbase), TC_TF32, 2, dw, 32, nt);
-    L.wbox = nt;
-  }
-  TcMlpArgs a;
-  a.M = L.M;
-  a.N = L.N;
-  a.Np = nt;
-  a.nk = L.Kp / 32;
-  a.bias = L.bias;
-  a.gelu = L.gelu;
-  a.mode = L.mode;
-  a.z = L.z;
-  a.act = L.act;
-  a.zin = L.zin;
-  a.ldz = L.ldz;
-  if (L.mode >= 2 && (!L.oh || !L.ol || L.ldz < L.N || (L.mode == 2 ? (!L.z || !L.act || !L.bias) : (!L.zin || !L.y))))
-    throw std::invalid_argument("tc_mlp_layer: training layer without its buffers");
-  a.oh = L.oh;
-  a.ol = L.ol;
-  a.ldo = L.ldo;
-  a.y = L.y;
-  a.ldy = L.ldy;
-  a.err = L.err;
-  a.idesc = make_idesc(TC_TF32, nt);
-  a.tmem_cols = tmem_cols_for(nt / 2);  // a power of two >= nt (and >= 32)
-  const size_t sm = (size_t)TC_NS * (2 * TC_M * 128 + (size_t)nt * 128) + 1024 + 256;
-  static bool attr = false;
-  if (!attr) {
-    GD_CUDA(cudaFuncSetAttribute(k_tc_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    attr = true;
-  }
-  k_tc_mlp<<<dim3(mt, (L.Np + nt - 1) / nt), TC_THREADS, sm, s>>>(L.ah, L.al, L.w, a);
+  k_tc_wgrad<<<dim3(W.nitems, nsplit), TC_THREADS, sm, s>>>(W.ah, W.al, W.bh, W.bl, a);
   count_launch();
   GD_LAUNCH_CHECK();
 }

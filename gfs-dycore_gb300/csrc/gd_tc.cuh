@@ -89,59 +89,53 @@ int tc_anal_segments(const TcPlan& p);
 // returns and clears the device error flag (nonzero: a bounded wait gave up)
 int tc_check(TcPlan& p, cudaStream_t s);
 
-// One dense layer of the closure network on the tensor cores: for m < M,
-// n < N, acc[m][n] = sum_k (Ah[m][k] + Al[m][k]) W[n][k], A split to TF32 hi +
-// lo (row pitch Kp, a multiple of 32 with zeros past the layer's inputs), W
-// exact in TF32 ([Np][Kp], Np = N rounded up to 16, zero rows past N), FP32
-// accumulation in TMEM.  The epilogue adds the bias, then either applies GELU
-// and writes the next layer's split operands (oh, ol, row pitch ldo) or
-// writes FP32 outputs y (row pitch ldy).  N <= 256.
-struct TcMlpLayer {
-  CUtensorMap ah, al, w;
-  int M = 0, N = 0, Np = 0, Kp = 0;
-  const float* wbase = nullptr;  // the weights the map w covers ([Np][Kp])
-  int wbox = 0;                  // N rows of the map's box (the N tile it was made for)
-  const float* bias = nullptr;
-  int gelu = 0;
-  uint32_t* oh = nullptr;
-  uint32_t* ol = nullptr;
-  int ldo = 0;
-  float* y = nullptr;
-  int ldy = 0;
-  int* err = nullptr;  // device flag: nonzero when a bounded wait gave up
-  // training: mode 2, a hidden layer of the forward pass that also stores its
-  // pre-activation z = A W^T + b and activation gelu(z) in FP32 ([M][ldz]);
-  // mode 3, the backward product dZ_prev = (dZ W) * gelu'(zin) (no bias),
-  // stored in FP32 to y and split hi + lo to oh / ol.  Mode 0: inference
-  // (gelu selects a hidden layer or the output).
-  int mode = 0;
-  float* z = nullptr;
-  float* act = nullptr;
-  const float* zin = nullptr;
-  int ldz = 0;
+// A chain of dense layers of the closure network on the tensor cores, one
+// launch: layer l takes the rows of the layer before it (the first x [M][ldx])
+// to acc[m][n] = sum_k A[m][k] W[n][k] (+ bias[n]), W in BF16, A carried as BF16
+// hi + mid + lo (the FP32 value), FP32 accumulation in TMEM, then
+//   act 0: acc; 1: GELU(acc); 2: acc GELU'(zin[m][n]) (the backward chain).
+// Optional copies in FP32, row pitch ldz: z (acc), out (the layer's result).
+// The last layer's result goes to y.  N <= 256 (every layer), K <= 256 but for
+// the first.  wrow: the layer's first row in the packed weights, rows of
+// kpitch BF16 zero-padded past K, each layer's block a multiple of 64 rows.
+struct TcChainLayer {
+  int N, K, wrow, act;
+  const float* bias;
+  float* z;
+  float* out;
+  const float* zin;
+  int ldz;
 };
-// tensor maps of a layer over its operand buffers (rows M of A)
-void tc_mlp_maps(TcMlpLayer& L, const uint32_t* ah, const uint32_t* al, const float* w);
-void tc_mlp_layer(const TcMlpLayer& L, cudaStream_t s);
+void tc_chain_map(CUtensorMap* m, const void* w, int kpitch, long rows);
+// layers: device array
+void tc_chain(const CUtensorMap& w, const TcChainLayer* layers, int nl, const float* x, int ldx, int M, float* y,
+              int ldy, int* err, cudaStream_t s);
 
-// Weight gradient of a closure layer: part[s][m][n] = sum over the K chunks
-// of slice s of A(m, k) B(n, k), both operands TF32 hi + lo rows with the
-// batch (K) contiguous: A = dZ^T (Mp rows, a multiple of 128), B = the
-// layer's input transposed (Np <= 256 rows).  Three products per K step
-// (hi hi, hi lo, lo hi), FP32 accumulation in TMEM; the slices' partial
+// Weight gradients of the closure's layers, one launch: item i, slice q:
+// part[q][poff + m Np + n] = sum over the slice's K chunks of A(arow + m, k)
+// B(brow + n, k), m < 128, n < Np; both operands TF32 hi + lo rows with the
+// batch (K) contiguous: A the layers' dZ^T stacked (blocks of 128 rows), B
+// their inputs transposed (Np <= 256, blocks of 64 rows).  Three products per K
+// step (hi hi, hi lo, lo hi), FP32 accumulation in TMEM; the slices' partial
 // tiles are summed afterwards in a fixed order.
+struct TcWgradItem {
+  int arow, brow, Np;
+  long poff;
+};
 struct TcWgrad {
   CUtensorMap ah, al, bh, bl;
-  int Mp = 0, Np = 0;
-  float* part = nullptr;  // [nsplit][Mp][Np]
+  const TcWgradItem* items = nullptr;  // device array
+  int nitems = 0;
+  float* part = nullptr;
+  long pstride = 0;
   int* err = nullptr;
 };
-// maps over the transposed operands; kpitch = their row length (batch
-// capacity, a multiple of 32)
+// maps over the stacked transposed operands; kpitch = their row length (a
+// multiple of 32)
 void tc_wgrad_maps(TcWgrad& W, const uint32_t* ah, const uint32_t* al, const uint32_t* bh, const uint32_t* bl,
-                   int kpitch);
+                   long arows, long brows, int kpitch);
 // nk = K chunks of 32 in use, split over nsplit slices of cps chunks each
-// (every slice non-empty)
-void tc_wgrad(const TcWgrad& W, int nk, int cps, int nsplit, cudaStream_t s);
+// (every slice non-empty), the partial tiles from slice0 on
+void tc_wgrad(const TcWgrad& W, int nk, int cps, int nsplit, int slice0, cudaStream_t s);
 
 }  // namespace gd
