@@ -419,6 +419,7 @@ class Dycore : public DycoreBase {
     free_plan(anaSimple);
     free_fft_plan(r2cSimple);
     free_fft_plan(r2cClos);
+    for (auto& kv : api_plans_) free_fft_plan(kv.second);
     if (stream) cudaStreamSynchronize(stream);
     for (void* p : allocs) cudaFree(p);
     if (stream && own_stream) cudaStreamDestroy(stream);
@@ -1503,44 +1504,73 @@ class Dycore : public DycoreBase {
     return anal_cache[ncr] = make_anal_plan(T, ncr, stream);
   }
   int chunk_cols() const { return std::max(1, std::min(sc.ncol / 2, ar.total / 2)); }
-  // synthesis of ncs complex columns X[nlm][ldS] with descriptors -> host grids
+  // Longitude plans of the transform API by (operation, fields of a call),
+  // made once: a call then neither allocates nor waits for its plan's upload.
+  enum { OP_SPECTOGRD, OP_GETUV, OP_GETGRAD, OP_GRDTOSPEC, OP_GETVRTDIV };
+  std::map<std::pair<int, int>, FftPlan> api_plans_;
+  template <typename D>
+  const FftPlan& api_plan(int op, int k, const std::vector<D>& ds) {
+    auto it = api_plans_.find({op, k});
+    if (it != api_plans_.end()) return it->second;
+    if constexpr (std::is_same<D, SynthDesc>::value)
+      return api_plans_[{op, k}] = mk_c2r(ds.data(), (int)ds.size());
+    else
+      return api_plans_[{op, k}] = mk_r2c(ds.data(), (int)ds.size());
+  }
+  // Device scratch of the host copies (fields in the host layout, rows in the
+  // host type), kept between calls up to kXferKeep bytes.
+  static constexpr size_t kXferKeep = 512u << 20;
+  char* xfer_ = nullptr;
+  size_t xfer_cap_ = 0;
   template <typename H>
-  void api_synth(const R* X, int ncs, bool needH, const std::vector<SynthDesc>& ds, int nrows, H* out) {
+  H* xfer(size_t n) {
+    if (n * sizeof(H) > xfer_cap_) {
+      GD_CUDA(cudaStreamSynchronize(stream));
+      if (xfer_) release(xfer_);
+      xfer_ = nullptr;
+      xfer_cap_ = 0;
+      xfer_ = dalloc<char>(n * sizeof(H));
+      xfer_cap_ = n * sizeof(H);
+    }
+    return reinterpret_cast<H*>(xfer_);
+  }
+  // the end of a transform call: every copy has completed
+  void api_done() {
+    GD_CUDA(cudaStreamSynchronize(stream));
+    if (xfer_cap_ > kXferKeep) {
+      release(xfer_);
+      xfer_ = nullptr;
+      xfer_cap_ = 0;
+    }
+  }
+  // synthesis of ncs complex columns X[nlm][ldS] to grid rows in gS
+  void api_synth(const R* X, int ncs, bool needH, const FftPlan& p) {
     const GemmPlan* plan = tcp ? nullptr : &synth_plan(2 * ncs);
     const Leg h{true, plan, X, ldS, 2 * ncs, FHb, ldS};
     do_synth(Leg{false, plan, X, ldS, 2 * ncs, FPb, ldS}, needH ? &h : nullptr);
-    FftPlan p = mk_c2r(ds.data(), (int)ds.size());
     c2r(p, FPb, ldS, FHb, ldS, gS);
-    grid_out(gS, nrows, out);
-    free_fft_plan(p);
   }
   // device grid rows (R) -> host (H), converted on the device when the types differ
   template <typename H>
   void grid_out(const R* g, int nrows, H* out) {
-    long n = (long)nrows * ng;
+    const long n = (long)nrows * ng;
     if constexpr (std::is_same<R, H>::value) {
       GD_CUDA(cudaMemcpyAsync(out, g, sizeof(H) * n, cudaMemcpyDeviceToHost, stream));
     } else {
-      H* tmp = dalloc<H>(n);
+      H* tmp = xfer<H>(n);
       launch_convert2d<R, H>(g, ng, tmp, ng, nrows, (int)ng, stream);
       GD_CUDA(cudaMemcpyAsync(out, tmp, sizeof(H) * n, cudaMemcpyDeviceToHost, stream));
-      GD_CUDA(cudaStreamSynchronize(stream));
-      release(tmp);
     }
-    GD_CUDA(cudaStreamSynchronize(stream));
   }
   template <typename H>
   void grid_in(const H* in, int nrows, R* g) {
-    long n = (long)nrows * ng;
+    const long n = (long)nrows * ng;
     if constexpr (std::is_same<R, H>::value) {
       GD_CUDA(cudaMemcpyAsync(g, in, sizeof(H) * n, cudaMemcpyHostToDevice, stream));
-      GD_CUDA(cudaStreamSynchronize(stream));
     } else {
-      H* tmp = dalloc<H>(n);
+      H* tmp = xfer<H>(n);
       GD_CUDA(cudaMemcpyAsync(tmp, in, sizeof(H) * n, cudaMemcpyHostToDevice, stream));
       launch_convert2d<H, R>(tmp, ng, g, ng, nrows, (int)ng, stream);
-      GD_CUDA(cudaStreamSynchronize(stream));
-      release(tmp);
     }
   }
   R* X_ = nullptr;
@@ -1553,11 +1583,15 @@ class Dycore : public DycoreBase {
   }
   template <typename H>
   void spec_in(const H* h, int nb, R* X, int col) {
-    H* tmp = dalloc<H>(2L * nb * nlm);
+    H* tmp = xfer<H>(2L * nb * nlm);
     GD_CUDA(cudaMemcpyAsync(tmp, h, sizeof(H) * 2 * (long)nb * nlm, cudaMemcpyHostToDevice, stream));
     launch_ref2int<R>(tmp, nb, nlm, X, ldS, col, stream);
-    GD_CUDA(cudaStreamSynchronize(stream));
-    release(tmp);
+  }
+  template <typename H>
+  void spec_out_to(int col, int nb, H* h) {  // columns of AP
+    H* tmp = xfer<H>(2L * nb * nlm);
+    launch_int2ref<R>(AP, ldAP, col, nb, nlm, tmp, stream);
+    GD_CUDA(cudaMemcpyAsync(h, tmp, sizeof(H) * 2 * (long)nb * nlm, cudaMemcpyDeviceToHost, stream));
   }
   void spectogrd(int nb, const double* spec, double* grid) override { spectogrd_t(nb, spec, grid); }
   void spectogrd(int nb, const float* spec, float* grid) override { spectogrd_t(nb, spec, grid); }
@@ -1579,9 +1613,10 @@ class Dycore : public DycoreBase {
     for (int b0 = 0; b0 < nb; b0 += chunk_cols()) {
       int k = std::min(chunk_cols(), nb - b0);
       spec_in(spec + 2L * b0 * nlm, k, X, 0);
-      std::vector<SynthDesc> ds = {{k, 0, 0, 0, -1, 0, 1.0, 0.0}};
-      api_synth(X, k, false, ds, k, grid + (long)b0 * ng);
+      api_synth(X, k, false, api_plan(OP_SPECTOGRD, k, std::vector<SynthDesc>{{k, 0, 0, 0, -1, 0, 1.0, 0.0}}));
+      grid_out(gS, k, grid + (long)b0 * ng);
     }
+    api_done();
   }
   template <typename H>
   void getuv_t(int nb, const H* vrt, const H* div, H* u, H* v) {
@@ -1593,12 +1628,12 @@ class Dycore : public DycoreBase {
       spec_in(div + 2L * b0 * nlm, k, X, k);
       // s = a invlap vrt, c = a invlap div (shtns.f90:259-260)
       launch_scale_cols<R>(X, ldS, 0, 2 * k, nlm, invlap_a(), R(1), stream);
-      std::vector<SynthDesc> ds = {{k, 0, 1, 0, 0, k, -1.0, 1.0}, {k, k, 1, k, 0, 0, 1.0, 1.0}};
-      std::vector<H> out(2L * k * ng);
-      api_synth(X, 2 * k, true, ds, 2 * k, out.data());
-      memcpy(u + (long)b0 * ng, out.data(), sizeof(H) * k * ng);
-      memcpy(v + (long)b0 * ng, out.data() + (long)k * ng, sizeof(H) * k * ng);
+      api_synth(X, 2 * k, true,
+                api_plan(OP_GETUV, k, std::vector<SynthDesc>{{k, 0, 1, 0, 0, k, -1.0, 1.0}, {k, k, 1, k, 0, 0, 1.0, 1.0}}));
+      grid_out(gS, k, u + (long)b0 * ng);
+      grid_out(gS + (long)k * ng, k, v + (long)b0 * ng);
     }
+    api_done();
   }
   R* invlap_ = nullptr;
   const R* invlap_a() {  // rerth * invlap, 0 for n = 0
@@ -1617,60 +1652,47 @@ class Dycore : public DycoreBase {
     for (int b0 = 0; b0 < nb; b0 += ch) {
       int k = std::min(ch, nb - b0);
       spec_in(spec + 2L * b0 * nlm, k, X, 0);
-      std::vector<SynthDesc> ds = {{k, 0, -1, 0, 0, 0, 0.0, ai}, {k, k, 1, 0, -1, 0, ai, 0.0}};
-      std::vector<H> out(2L * k * ng);
-      api_synth(X, k, true, ds, 2 * k, out.data());
-      memcpy(gx + (long)b0 * ng, out.data(), sizeof(H) * k * ng);
-      memcpy(gy + (long)b0 * ng, out.data() + (long)k * ng, sizeof(H) * k * ng);
+      api_synth(X, k, true,
+                api_plan(OP_GETGRAD, k, std::vector<SynthDesc>{{k, 0, -1, 0, 0, 0, 0.0, ai}, {k, k, 1, 0, -1, 0, ai, 0.0}}));
+      grid_out(gS, k, gx + (long)b0 * ng);
+      grid_out(gS + (long)k * ng, k, gy + (long)b0 * ng);
     }
+    api_done();
   }
-  void api_anal(const std::vector<AnalDesc>& ds, int ncP, int ncH) {
-    FftPlan p = mk_r2c(ds.data(), (int)ds.size());
+  void api_anal(const FftPlan& p, int ncP, int ncH) {
     r2c(p, gA, FPb, ldS, FHb, ldS);
     const Leg h{true, tcp || ncH <= 0 ? nullptr : &anal_plan(2 * ncH), FHb, ldS, 2 * ncH, AH, ldAH};
     do_anal(Leg{false, tcp ? nullptr : &anal_plan(2 * ncP), FPb, ldS, 2 * ncP, AP, ldAP}, ncH > 0 ? &h : nullptr);
-    free_fft_plan(p);
   }
   int achunk() const { return std::max(1, std::min(ap.ncol / 2, ar.total / 2)); }
   template <typename H>
   void grdtospec_t(int nb, const H* grid, H* spec) {
     const int ch = achunk();
-    H* tmp = dalloc<H>(2L * ch * nlm);
     for (int b0 = 0; b0 < nb; b0 += ch) {
       int k = std::min(ch, nb - b0);
       grid_in(grid + (long)b0 * ng, k, gA);
-      api_anal({{k, 0, 0, 0, -1, 1.0, 0.0}}, k, 0);
-      launch_int2ref<R>(AP, ldAP, 0, k, nlm, tmp, stream);
-      GD_CUDA(cudaMemcpyAsync(spec + 2L * b0 * nlm, tmp, sizeof(H) * 2 * (long)k * nlm, cudaMemcpyDeviceToHost,
-                              stream));
-      GD_CUDA(cudaStreamSynchronize(stream));
+      api_anal(api_plan(OP_GRDTOSPEC, k, std::vector<AnalDesc>{{k, 0, 0, 0, -1, 1.0, 0.0}}), k, 0);
+      spec_out_to(0, k, spec + 2L * b0 * nlm);
     }
-    release(tmp);
+    api_done();
   }
   template <typename H>
   void getvrtdivspec_t(int nb, const H* u, const H* v, H* vrt, H* div) {
     const int ch = std::max(1, std::min(ah.ncol / 2, achunk()));
-    H* tmp = dalloc<H>(2L * ch * nlm);
     const R ai = (R)(1.0 / Phys::rerth);
     for (int b0 = 0; b0 < nb; b0 += ch) {
       int k = std::min(ch, nb - b0);
       grid_in(u + (long)b0 * ng, k, gA);
       grid_in(v + (long)b0 * ng, k, gA + (long)k * ng);
       // GP: [i m/cos V | i m/cos U], GH: [U | -V]
-      std::vector<AnalDesc> ds = {{k, 0, k, 1, 0, 1.0, 1.0}, {k, k, 0, 1, k, 1.0, -1.0}};
-      api_anal(ds, 2 * k, 2 * k);
+      api_anal(api_plan(OP_GETVRTDIV, k, std::vector<AnalDesc>{{k, 0, k, 1, 0, 1.0, 1.0}, {k, k, 0, 1, k, 1.0, -1.0}}),
+               2 * k, 2 * k);
       // vrt = (AP[0:k] + AH[0:k]) / a, div = (AP[k:2k] + AH[k:2k]) / a
       launch_combine<R>(AP, ldAP, 0, AH, ldAH, 0, AP, ldAP, 0, 2 * k, nlm, ai, stream);
-      launch_int2ref<R>(AP, ldAP, 0, k, nlm, tmp, stream);
-      GD_CUDA(cudaMemcpyAsync(vrt + 2L * b0 * nlm, tmp, sizeof(H) * 2 * (long)k * nlm, cudaMemcpyDeviceToHost,
-                              stream));
-      GD_CUDA(cudaStreamSynchronize(stream));
-      launch_int2ref<R>(AP, ldAP, k, k, nlm, tmp, stream);
-      GD_CUDA(cudaMemcpyAsync(div + 2L * b0 * nlm, tmp, sizeof(H) * 2 * (long)k * nlm, cudaMemcpyDeviceToHost,
-                              stream));
-      GD_CUDA(cudaStreamSynchronize(stream));
+      spec_out_to(0, k, vrt + 2L * b0 * nlm);
+      spec_out_to(k, k, div + 2L * b0 * nlm);
     }
-    release(tmp);
+    api_done();
   }
 
   void grid_info(double* lats, double* gauwts, double* areawts, int* degree, int* order, double* lap,
@@ -1711,6 +1733,7 @@ class Dycore : public DycoreBase {
     else if (n == "pwat") src = pwat, rows = 1;
     if (!src || rows == 0) return GD_ERR_ARG;
     grid_out(src, rows, out);
+    api_done();
     return GD_OK;
   }
   double get_pdryini() override {

@@ -112,6 +112,7 @@ struct gd_mlp {
   int tcap = 0;               // batch capacity of the training buffers
   int nsm = 0;
   int* terr = nullptr;
+  float* hres = nullptr;  // page-locked: error flag and loss on their way out
   cudaStream_t stream = nullptr;  // the stream the net's work runs on
   cudaStream_t own = nullptr;     // the net's own stream (destroyed with it)
   std::string err;
@@ -128,6 +129,7 @@ struct gd_mlp {
     if (stream) cudaStreamSynchronize(stream);
     for (void* p : allocs)
       if (p) cudaFree(p);
+    if (hres) cudaFreeHost(hres);
     if (own) cudaStreamDestroy(own);
     if (cur != device) cudaSetDevice(cur);
   }
@@ -603,17 +605,34 @@ void forward_simt(gd_mlp* p, const float* x, int n, float* y, cudaStream_t s) {
 }
 }  // namespace
 
-// raises (and clears) a bounded wait's timeout in the tensor-core forward
+// a bounded wait of a tensor-core kernel gave up: clears the flag and raises it
+[[noreturn]] static void mlp_timeout(gd_mlp* p, cudaStream_t s, int code) {
+  GD_CUDA(cudaMemsetAsync(p->terr, 0, sizeof(int), s));
+  GD_CUDA(cudaStreamSynchronize(s));
+  throw CudaError("closure net: a tensor-core wait timed out (code " + std::to_string(code) + ")");
+}
+// the end of an entry point of the net itself: copies the error flag and the
+// loss through page-locked memory, the gradient straight to the caller (a
+// second host copy of 0.9 MB costs more than it saves), waits once, and
+// raises a timeout
+void mlp_results(gd_mlp* p, cudaStream_t s, float* loss, float* grad) {
+  int* e = reinterpret_cast<int*>(p->hres);
+  *e = 0;
+  if (p->terr) GD_CUDA(cudaMemcpyAsync(e, p->terr, sizeof(int), cudaMemcpyDeviceToHost, s));
+  if (loss) GD_CUDA(cudaMemcpyAsync(p->hres + 1, p->lossd, sizeof(float), cudaMemcpyDeviceToHost, s));
+  if (grad) GD_CUDA(cudaMemcpyAsync(grad, p->grad, sizeof(float) * p->np, cudaMemcpyDeviceToHost, s));
+  GD_CUDA(cudaStreamSynchronize(s));
+  if (*e) mlp_timeout(p, s, *e);
+  if (loss) *loss = p->hres[1];
+}
+// for a context the net is attached to: another thread may be using the net's
+// own page-locked results
 void mlp_check(gd_mlp* p, cudaStream_t s) {
   if (!p->terr) return;
   int e = 0;
   GD_CUDA(cudaMemcpyAsync(&e, p->terr, sizeof(int), cudaMemcpyDeviceToHost, s));
   GD_CUDA(cudaStreamSynchronize(s));
-  if (e) {
-    GD_CUDA(cudaMemsetAsync(p->terr, 0, sizeof(int), s));
-    GD_CUDA(cudaStreamSynchronize(s));
-    throw CudaError("closure net: a tensor-core wait timed out (code " + std::to_string(e) + ")");
-  }
+  if (e) mlp_timeout(p, s, e);
 }
 
 int mlp_nin(const gd_mlp* p) { return p->nin; }
@@ -758,6 +777,7 @@ int gd_mlp_init(int nin, int nhidden, int nlayers, int nout, unsigned long long 
   const int rc = mguard(p.get(), [&] {
     GD_CUDA(cudaStreamCreateWithFlags(&p->own, cudaStreamNonBlocking));
     p->stream = p->own;
+    GD_CUDA(cudaMallocHost(&p->hres, sizeof(float) * 2));
     p->p32 = (float*)p->alloc(sizeof(float) * off);
     p->w16 = (__nv_bfloat16*)p->alloc(sizeof(__nv_bfloat16) * off);
     p->grad = (float*)p->alloc(sizeof(float) * off);
@@ -861,7 +881,7 @@ int gd_mlp_forward(gd_mlp* p, const float* x, int ncols, float* y) {
     need_device(p, y, "y");
     mlp_reserve(p, ncols);
     mlp_forward_on(p, x, ncols, y, p->stream);
-    mlp_check(p, p->stream);
+    mlp_results(p, p->stream, nullptr, nullptr);
   });
 }
 
@@ -872,9 +892,7 @@ int gd_mlp_loss_grad(gd_mlp* p, const float* x, const float* t, int ncols, float
     need_device(p, t, "t");
     train_reserve(p, ncols);
     loss_grad(p, x, t, ncols);
-    mlp_check(p, p->stream);
-    if (loss) GD_CUDA(cudaMemcpy(loss, p->lossd, sizeof(float), cudaMemcpyDeviceToHost));
-    if (grad) GD_CUDA(cudaMemcpy(grad, p->grad, sizeof(float) * p->np, cudaMemcpyDeviceToHost));
+    mlp_results(p, p->stream, loss, grad);
   });
 }
 
@@ -893,10 +911,7 @@ int gd_mlp_train_step(gd_mlp* p, const float* x, const float* t, int ncols, floa
     count_launch();
     GD_LAUNCH_CHECK();
     pack_weights(p);
-    if (loss) {
-      GD_CUDA(cudaMemcpyAsync(loss, p->lossd, sizeof(float), cudaMemcpyDeviceToHost, p->stream));
-      mlp_check(p, p->stream);  // synchronises; raises a tensor-core wait that gave up
-    }
+    if (loss) mlp_results(p, p->stream, loss, nullptr);  // waits; raises a tensor-core wait that gave up
   });
 }
 
@@ -908,9 +923,7 @@ int gd_mlp_set_stream(gd_mlp* p, void* stream) {
 }
 
 int gd_mlp_sync(gd_mlp* p) {
-  return mguard(p, [&] {
-    mlp_check(p, p->stream);
-  });
+  return mguard(p, [&] { mlp_results(p, p->stream, nullptr, nullptr); });
 }
 
 const char* gd_mlp_last_error(gd_mlp* p) { return p ? p->err.c_str() : g_mlp_init_error.c_str(); }

@@ -357,7 +357,7 @@ class Dycore:
         return np.asarray(a).dtype in (np.complex64, np.float32)
 
     def _g(self, nb, single=False):
-        return np.zeros((nb, self.nlat, self.nlon), np.float32 if single else np.float64)
+        return np.empty((nb, self.nlat, self.nlon), np.float32 if single else np.float64)
 
     def spectogrd(self, spec):
         f = self._single(spec)
@@ -370,7 +370,7 @@ class Dycore:
     def grdtospec(self, grid):
         f = self._single(grid)
         grid = np.ascontiguousarray(grid, np.float32 if f else np.float64).reshape(-1, self.nlat, self.nlon)
-        s = np.zeros((grid.shape[0], self.nlm), np.complex64 if f else np.complex128)
+        s = np.empty((grid.shape[0], self.nlm), np.complex64 if f else np.complex128)
         fn = load().gd_grdtospec_f if f else load().gd_grdtospec
         self._chk(fn(self.h, grid.shape[0], _p(grid), _p(s)))
         return s
@@ -390,8 +390,8 @@ class Dycore:
         rt = np.float32 if f else np.float64
         u = np.ascontiguousarray(u, rt).reshape(-1, self.nlat, self.nlon)
         v = np.ascontiguousarray(v, rt).reshape(-1, self.nlat, self.nlon)
-        vrt = np.zeros((u.shape[0], self.nlm), np.complex64 if f else np.complex128)
-        div = np.zeros_like(vrt)
+        vrt = np.empty((u.shape[0], self.nlm), np.complex64 if f else np.complex128)
+        div = np.empty_like(vrt)
         fn = load().gd_getvrtdivspec_f if f else load().gd_getvrtdivspec
         self._chk(fn(self.h, u.shape[0], _p(u), _p(v), _p(vrt), _p(div)))
         return vrt, div
@@ -574,8 +574,7 @@ class Mlp:
         self._batch(x, self.nin, "x")
         y = torch.empty((x.shape[0], self.nout), dtype=torch.float32, device=x.device)
         self._chk(load().gd_mlp_forward(self.h, ctypes.c_void_p(x.data_ptr()), int(x.shape[0]),
-                                        ctypes.c_void_p(y.data_ptr())))
-        self.sync()
+                                        ctypes.c_void_p(y.data_ptr())))  # returns when y is written
         return y
 
     def loss_grad(self, x, t):

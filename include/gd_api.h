@@ -458,7 +458,7 @@ int gd_mlp_set_params(gd_mlp* net, const float* params);
 /* Normalisation of a closure's raw inputs ((x - in_mu) / in_sd) and outputs
    (y out_sd + out_mu), host arrays of nin and nout. */
 int gd_mlp_set_norm(gd_mlp* net, const float* in_mu, const float* in_sd, const float* out_mu, const float* out_sd);
-/* y = net(x) on the net's stream (asynchronous). */
+/* y = net(x) on the net's stream; returns when y is written. */
 int gd_mlp_forward(gd_mlp* net, const float* x, int ncols, float* y);
 /* Mean-squared error of net(x) against t and its gradient with respect to
    the parameters (host float[nparams], may be NULL); synchronous. */
