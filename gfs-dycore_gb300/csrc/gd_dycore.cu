@@ -26,6 +26,7 @@
 #include "gd_dcmip.h"
 #include "gd_physics.cuh"
 #include "gd_mlp.cuh"
+#include "gd_oz.cuh"
 #include "gd_spec.cuh"
 #include "gd_tc.cuh"
 #include <type_traits>
@@ -193,6 +194,9 @@ class Dycore : public DycoreBase {
   // tensor-core split-precision Legendre path: FP32 state (TF32x3, BF16x3)
   // or FP64 state with FP32 staging copies around the GEMM (F64_TF32X3)
   std::unique_ptr<TcPlan> tcp;
+  // FP64 tensor-core Legendre path of the plain FP64 mode (exact splitting)
+  std::unique_ptr<OzPlan> ozp;
+  bool simt() const { return !split_mode() && !ozp; }
   double *P64keep = nullptr, *H64keep = nullptr;
   bool split_mode() const {
     return c.precision == GD_PREC_TF32X3 || c.precision == GD_PREC_BF16X3 || c.precision == GD_PREC_F64_TF32X3 ||
@@ -252,7 +256,7 @@ class Dycore : public DycoreBase {
   // orders m >= 1, both tables' order 0 in one launch.
   struct Leg {
     bool useH;
-    const GemmPlan* plan;  // all-orders SIMT work list (not used by the split modes)
+    const GemmPlan* plan;  // all-orders SIMT work list (null on the tensor-core paths)
     const R* in;
     long ldin;
     int ncr;
@@ -261,17 +265,36 @@ class Dycore : public DycoreBase {
     Order0<R> order0() const { return Order0<R>{in, ldin, out, ldout, ncr / 2, useH ? 1 : 0, nullptr}; }
   };
   void do_synth(const Leg& a, const Leg* b = nullptr) {
-    if (tcp) {
+    if (!simt()) {
       const Order0<R> g[2] = {a.order0(), b ? b->order0() : a.order0()};
       launch_synth0<R>(sd, g, b ? 2 : 1, stream);
+    }
+    if constexpr (std::is_same<R, double>::value) {
+      if (ozp) {  // both tables read the same columns: one split serves them
+        oz_split_x(*ozp, moff, a.in, a.ldin, a.ncr, stream);
+        oz_synth(*ozp, moff, a.useH, 0, a.ncr, a.out, a.ldout, stream);
+        if (!b) return;
+        const long off = b->in - a.in;
+        const bool shared = b->ldin == a.ldin && off >= 0 && off + b->ncr <= a.ncr;
+        if (!shared) oz_split_x(*ozp, moff, b->in, b->ldin, b->ncr, stream);
+        oz_synth(*ozp, moff, b->useH, shared ? (int)off : 0, b->ncr, b->out, b->ldout, stream);
+        return;
+      }
     }
     synth_orders(a);
     if (b) synth_orders(*b);
   }
   void do_anal(const Leg& a, const Leg* b = nullptr) {
-    if (tcp) {
+    if (!simt()) {
       const Order0<R> g[2] = {a.order0(), b ? b->order0() : a.order0()};
       launch_anal0<R>(sd, g, b ? 2 : 1, stream);
+    }
+    if constexpr (std::is_same<R, double>::value) {
+      if (ozp) {
+        oz_anal(*ozp, moff, a.useH, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
+        if (b) oz_anal(*ozp, moff, b->useH, b->in, b->ldin, b->ncr, b->out, b->ldout, stream);
+        return;
+      }
     }
     anal_orders(a);
     if (b) anal_orders(*b);
@@ -325,7 +348,7 @@ class Dycore : public DycoreBase {
     if (closure) mlp_check(closure, stream);
   }
   void tc_status() {
-    if (tcp && tc_check(*tcp, stream))
+    if ((tcp && tc_check(*tcp, stream)) || (ozp && oz_check(*ozp, stream)))
       throw CudaError("tensor-core Legendre pipeline: a bounded wait gave up (results invalid)");
   }
 
@@ -366,6 +389,20 @@ class Dycore : public DycoreBase {
     init_grid();
     init_vertical(ak_, bk_);
     init_buffers();
+    if constexpr (std::is_same<R, double>::value) {
+      if (c.precision == GD_PREC_FP64) {
+        // the digits take 4 to 8 times the FP64 tables and operands: contexts
+        // where that is more than a quarter of the device's memory (T1148 with
+        // 64 levels; GD_FP64_TC_GB sets the line, 0: none) keep the FP64 pipe
+        size_t free_b = 0, total_b = 0;
+        GD_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        const int gb = env_int("GD_FP64_TC_GB", -1);
+        ozp.reset(new OzPlan());
+        if (!oz_init(*ozp, T, nh, nlat, 2 * std::max(sc.ncol, ap.ncol), gb < 0 ? total_b / 4 : (size_t)gb << 30, moff,
+                     toff, P, H, stream))
+          ozp.reset();
+      }
+    }
     init_plans();
     if (split_mode()) {
       tcp.reset(new TcPlan());
@@ -404,6 +441,7 @@ class Dycore : public DycoreBase {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (gstep) cudaGraphDestroy(gstep);
     if (tcp) tc_free(*tcp);
+    if (ozp) oz_free(*ozp);
     for (auto e : evpool) cudaEventDestroy(e);
     free_plan(synP);
     free_plan(synH);
@@ -740,11 +778,13 @@ class Dycore : public DycoreBase {
   }
 
   void init_plans() {
-    synP = make_synth_plan(T, nh, 2 * sc.ncol, stream);
-    synH = make_synth_plan(T, nh, 2 * (sc.ncol - 2 * L), stream);
-    anaP = make_anal_plan(T, 2 * ap.ncol, stream);
-    anaH = make_anal_plan(T, 2 * ah.ncol, stream);
-    anaPhys = make_anal_plan(T, 2 * (3 * L + 1), stream);
+    if (simt()) {
+      synP = make_synth_plan(T, nh, 2 * sc.ncol, stream);
+      synH = make_synth_plan(T, nh, 2 * (sc.ncol - 2 * L), stream);
+      anaP = make_anal_plan(T, 2 * ap.ncol, stream);
+      anaH = make_anal_plan(T, 2 * ah.ncol, stream);
+      anaPhys = make_anal_plan(T, 2 * (3 * L + 1), stream);
+    }
     const double ai = 1.0 / Phys::rerth;
     const int h0 = 2 * L;  // FH column = S column - 2L
     std::vector<SynthDesc> full = {
@@ -793,7 +833,7 @@ class Dycore : public DycoreBase {
       };
       if (c.massfix) sd_.push_back({1, 4 * L, 2 * L, 0, -1, 1.0, 0.0});
       r2cSimple = mk_r2c(sd_.data(), (int)sd_.size());
-      anaSimple = make_anal_plan(T, 2 * (4 * L + 1), stream);
+      if (simt()) anaSimple = make_anal_plan(T, 2 * (4 * L + 1), stream);
     }
   }
 
@@ -1116,7 +1156,7 @@ class Dycore : public DycoreBase {
         };
         r2cClos = mk_r2c(cd.data(), (int)cd.size());
       }
-      if (!anaSimple.items) anaSimple = make_anal_plan(T, 2 * (4 * L + 1), stream);
+      if (simt() && !anaSimple.items) anaSimple = make_anal_plan(T, 2 * (4 * L + 1), stream);
       GD_CUDA(cudaStreamSynchronize(stream));
     }
     closure = net;
@@ -1545,7 +1585,7 @@ class Dycore : public DycoreBase {
   }
   // synthesis of ncs complex columns X[nlm][ldS] to grid rows in gS
   void api_synth(const R* X, int ncs, bool needH, const FftPlan& p) {
-    const GemmPlan* plan = tcp ? nullptr : &synth_plan(2 * ncs);
+    const GemmPlan* plan = !simt() ? nullptr : &synth_plan(2 * ncs);
     const Leg h{true, plan, X, ldS, 2 * ncs, FHb, ldS};
     do_synth(Leg{false, plan, X, ldS, 2 * ncs, FPb, ldS}, needH ? &h : nullptr);
     c2r(p, FPb, ldS, FHb, ldS, gS);
@@ -1661,8 +1701,8 @@ class Dycore : public DycoreBase {
   }
   void api_anal(const FftPlan& p, int ncP, int ncH) {
     r2c(p, gA, FPb, ldS, FHb, ldS);
-    const Leg h{true, tcp || ncH <= 0 ? nullptr : &anal_plan(2 * ncH), FHb, ldS, 2 * ncH, AH, ldAH};
-    do_anal(Leg{false, tcp ? nullptr : &anal_plan(2 * ncP), FPb, ldS, 2 * ncP, AP, ldAP}, ncH > 0 ? &h : nullptr);
+    const Leg h{true, !simt() || ncH <= 0 ? nullptr : &anal_plan(2 * ncH), FHb, ldS, 2 * ncH, AH, ldAH};
+    do_anal(Leg{false, !simt() ? nullptr : &anal_plan(2 * ncP), FPb, ldS, 2 * ncP, AP, ldAP}, ncH > 0 ? &h : nullptr);
   }
   int achunk() const { return std::max(1, std::min(ap.ncol / 2, ar.total / 2)); }
   template <typename H>

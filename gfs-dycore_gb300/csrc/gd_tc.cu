@@ -29,6 +29,7 @@
 #include <cstring>
 #include <vector>
 
+#include "gd_ptx.cuh"
 #include "gd_tc.cuh"
 
 namespace gd {
@@ -36,76 +37,6 @@ namespace gd {
 constexpr int TC_NS = 3;          // pipeline stages
 constexpr int TC_M = 128;         // MMA M (batch columns per CTA)
 constexpr int TC_THREADS = 128;   // 4 warps
-constexpr unsigned long long TC_WAIT_NS = 2000000000ull;  // bounded waits: 2 s
-
-// ------------------------------------------------------------ PTX helpers --
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait: false (and the error flag set) if the phase does not
-// complete within TC_WAIT_NS
-__device__ __noinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* err, int code) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer();
-  for (;;) {
-    for (int i = 0; i < 64; ++i)
-      if (mbar_try(bar, parity)) return true;
-    if (globaltimer() - t0 > TC_WAIT_NS) {
-      atomicCAS(err, 0, code);
-      return false;
-    }
-    __nanosleep(64);
-  }
-}
-__device__ __forceinline__ void tma_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          dst),
-      "l"(map), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-      "[%5];" ::"r"(dst),
-      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row
-// groups 1024 bytes apart (SBO), descriptor version 1 (sm_100 family)
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;              // LBO (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;    // SBO
-  d |= (uint64_t)1 << 46;              // version
-  d |= (uint64_t)2 << 61;              // SWIZZLE_128B
-  return d;
-}
 template <int KIND>
 __device__ __forceinline__ void mma(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
   if (KIND == TC_TF32)
@@ -119,23 +50,6 @@ __device__ __forceinline__ void mma(uint32_t dtmem, uint64_t a, uint64_t b, uint
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // ------------------------------------------------------------ splitting --
 template <int KIND>
 struct Elem;
@@ -695,29 +609,12 @@ constexpr int TCF_MAXNS = 6;
 constexpr int TCF_MAXA = 4;  // A slots in tensor memory at most (64 columns each)
 constexpr int TCF_MAXN = 192;  // widest N tile (single-buffered E|O, 2N + 128 TMEM columns)
 
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
 __device__ __forceinline__ void mma_tf32_ta(uint32_t dtmem, uint32_t atmem, uint64_t b, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(dtmem),
       "r"(atmem), "l"(b), "r"(idesc), "r"(acc));
 }
-
-// Position of K chunk g in a ring of n slots, advanced once per chunk: the
-// slot g mod n and the parity (g / n) & 1 of its use count, without the
-// 64-bit division per chunk on the single-thread issue paths.
-struct TcRing {
-  int slot = 0;
-  uint32_t ph = 0;
-  __device__ __forceinline__ void next(int n) {
-    if (++slot == n) {
-      slot = 0;
-      ph ^= 1u;
-    }
-  }
-};
 
 __global__ void __launch_bounds__(TCF_THREADS, 1)
     k_tc_gemm_f(const __grid_constant__ CUtensorMap mRaw, const __grid_constant__ CUtensorMap mBh,
@@ -1063,7 +960,7 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
 }
 
 // ------------------------------------------------------------ host side --
-static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   if (!fn) {
     cudaDriverEntryPointQueryResult q;
@@ -1086,7 +983,7 @@ static void make_map(CUtensorMap* m, void* base, int kind, int rank, const uint6
   bx[0] = box_inner;
   bx[1] = box_rows;
   bx[2] = 1;
-  CUresult r = encode_fn()(m, kind == TC_TF32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+  CUresult r = tensor_map_encoder()(m, kind == TC_TF32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
                            rank, base, gd, gs, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
@@ -1097,7 +994,7 @@ static void make_raw_map(CUtensorMap* m, const void* base, const uint64_t* dims,
                          const uint32_t* box) {
   cuuint64_t gd[3] = {dims[0], dims[1], dims[2]}, gs[2] = {strides[0], strides[1]};
   cuuint32_t bx[3] = {box[0], box[1], box[2]}, estr[3] = {1, 1, 1};
-  CUresult r = encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), gd, gs, bx, estr,
+  CUresult r = tensor_map_encoder()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), gd, gs, bx, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled (raw) failed: " + std::to_string((int)r));
@@ -1638,10 +1535,6 @@ __device__ __forceinline__ void tc_split3_st(uint32_t t, const float* v) {
   tmem_st16(t + 128, m);
   tmem_st16(t + 256, l);
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
 __global__ void __launch_bounds__(TCC_THREADS, 1)
     k_tc_chain(const __grid_constant__ CUtensorMap mW, TcChainArgs a) {
   extern __shared__ __align__(1024) unsigned char smraw[];

@@ -2,12 +2,16 @@
 // sm_103a tensor cores (tcgen05 + TMEM + TMA).  Declarations.
 #pragma once
 #include <cuda.h>
+#include <cudaTypedefs.h>
 
 #include <array>
 
 #include "gd_kernels.h"
 
 namespace gd {
+
+// the driver's cuTensorMapEncodeTiled
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
 enum TcKind { TC_TF32 = 0, TC_BF16 = 1 };
 
