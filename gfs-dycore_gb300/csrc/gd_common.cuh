@@ -77,6 +77,27 @@ __host__ __device__ inline typename C2<R>::T mk2(R x, R y) {
 
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
+// Reciprocal in FP64 for kernels that the FP64 pipe (two lanes per clock and
+// SM) bounds: one step of Halley's third-order iteration r (1 + e + e^2), e = 1
+// - x r, on the hardware's approximation (relative error 2^-20 at worst; e^3 is
+// below 2^-59): three multiply-adds, last-bit differences from the IEEE
+// quotient.  For normal numbers below 2^1022.
+__device__ __forceinline__ double crcp(double a) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
+  const double e = fma(-a, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// sum of c[k] w^k, k < N
+template <typename R, int N>
+__device__ __forceinline__ R series(const R* c, R w) {
+  R v = c[N - 1];
+#pragma unroll
+  for (int k = N - 2; k >= 0; --k) v = v * w + c[k];
+  return v;
+}
+
 // float to double with integer operations: the conversion instruction runs on
 // the FP64 pipe (two lanes per clock and SM) and bounds a kernel that does
 // little else.  The same result; zero, subnormal numbers, infinities and NaN

@@ -10,6 +10,7 @@
 // interface quantities (ak, bk, pk, dpk, rlnp, alfa, etadot) top (t=0) to
 // bottom; b = L-1-t.
 #include <cfloat>
+#include <vector>
 
 #include "gd_grid.cuh"
 
@@ -19,18 +20,8 @@ constexpr int LMAX = 128;
 
 // Division, reciprocal and logarithm of the column kernel: the hardware
 // approximations for the FP32 state (relative error ~1e-7, below the FP32
-// state's own rounding).  In the FP64 state the FP64 pipe (two lanes per clock
-// and SM) bounds the kernel, so its reciprocal is one step of Halley's
-// third-order iteration r (1 + e + e^2), e = 1 - x r, on the hardware's
-// approximation (relative error 2^-20 at worst; e^3 is below 2^-59): three
-// multiply-adds, last-bit differences from the IEEE quotient.  Operands here
-// are pressures, layer thicknesses and tracer differences, normal numbers.
-__device__ __forceinline__ double crcp(double a) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(a));
-  const double e = fma(-a, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
+// state's own rounding), the FP64 state's crcp in gd_common.cuh (operands here
+// are pressures, layer thicknesses and tracer differences, normal numbers).
 __device__ __forceinline__ double cdiv(double a, double b) {
   const double r = crcp(b), q = a * r;
   return fma(fma(-b, q, a), r, q);
@@ -498,13 +489,6 @@ template void launch_dyn_columns<float>(const ColumnArgs<float>&, bool, cudaStre
 // of 32.  Physics phase of a step (this kernel, the mass fixer and the
 // update), before -> after: T254L64 FP64 state 7.77 -> 3.82 ms, T126L64 FP64
 // 1.97 -> 0.97 ms, T42L20 FP64 0.330 -> 0.088 ms, T574L64 FP32 0.563 -> 0.467 ms.
-template <typename R, int N>
-__device__ __forceinline__ R hs_series(const R* c, R w) {
-  R v = c[N - 1];
-#pragma unroll
-  for (int k = N - 2; k >= 0; --k) v = v * w + c[k];
-  return v;
-}
 template <typename R>
 __global__ void __launch_bounds__(128) k_hs(const __grid_constant__ HsArgs<R> a) {
   const long ng = (long)a.nlon * a.nlat;
@@ -541,9 +525,9 @@ __global__ void __launch_bounds__(128) k_hs(const __grid_constant__ HsArgs<R> a)
       const bool low = !(pkt1 < psbot);  // prs < pkt1: above this level the drag profile is zero
       R lp, bl = R(0);                // ln(prs / p0), (prs / ps - sigbot) / (1 - sigbot)
       if (w <= R(0.16)) {
-        lp = log(pm * rp0) + (w <= R(0.015625) ? hs_series<R, 9>(a.lns, w) : hs_series<R, HsArgs<R>::NS>(a.lns, w));
+        lp = log(pm * rp0) + (w <= R(0.015625) ? series<R, 9>(a.lns, w) : series<R, HsArgs<R>::NS>(a.lns, w));
         if (low)
-          bl = pm * ips * (w <= R(0.015625) ? hs_series<R, 9>(a.prss, w) : hs_series<R, HsArgs<R>::NS>(a.prss, w));
+          bl = pm * ips * (w <= R(0.015625) ? series<R, 9>(a.prss, w) : series<R, HsArgs<R>::NS>(a.prss, w));
       } else {
         const R x = (pow(pkt1, a.kappa) * pkt1 - pow(pkt, a.kappa) * pkt) / ((a.kappa + R(1)) * dp);
         const R lx = log(x) / a.kappa;
@@ -563,32 +547,39 @@ __global__ void __launch_bounds__(128) k_hs(const __grid_constant__ HsArgs<R> a)
   }
 }
 template <typename R>
-void launch_hs_forcing(const HsArgs<R>& in, cudaStream_t s) {
-  HsArgs<R> a = in;
-  const long ng = (long)a.nlon * a.nlat;
-  constexpr int NS = HsArgs<R>::NS;
+void phillips_series(R kappa, int n, R* lns, R* prss) {
   // g(w) = ((1+z)^(k+1) - (1-z)^(k+1)) / (2 (k+1) z) = sum_i C(k+1, 2i+1) / (k+1) w^i,
   // h = ln(g) / k and exp(h), each series from the one before by its derivative
-  const double kap = (double)a.kappa;
-  double c[NS], h[NS], e[NS];
+  const double kap = (double)kappa;
+  std::vector<double> c(n), h(n), e(n);
   double bin = 1.0;  // C(k+1, 2i+1) / (k+1)
-  for (int i = 0; i < NS; ++i) {
+  for (int i = 0; i < n; ++i) {
     if (i > 0) bin *= (kap + 2.0 - 2 * i) * (kap + 1.0 - 2 * i) / ((2.0 * i) * (2.0 * i + 1.0));
     c[i] = bin;
   }
   h[0] = 0.0;
-  for (int i = 1; i < NS; ++i) {
+  for (int i = 1; i < n; ++i) {
     double v = i * c[i];
     for (int q = 1; q < i; ++q) v -= q * h[q] * kap * c[i - q];
     h[i] = v / (i * kap);
   }
   e[0] = 1.0;
-  for (int i = 1; i < NS; ++i) {
+  for (int i = 1; i < n; ++i) {
     double v = 0.0;
     for (int q = 1; q <= i; ++q) v += q * h[q] * e[i - q];
     e[i] = v / i;
   }
-  for (int i = 0; i < NS; ++i) a.lns[i] = (R)h[i], a.prss[i] = (R)e[i];
+  for (int i = 0; i < n; ++i) lns[i] = (R)h[i], prss[i] = (R)e[i];
+}
+template void phillips_series<double>(double, int, double*, double*);
+template void phillips_series<float>(float, int, float*, float*);
+
+template <typename R>
+void launch_hs_forcing(const HsArgs<R>& in, cudaStream_t s) {
+  HsArgs<R> a = in;
+  const long ng = (long)a.nlon * a.nlat;
+  constexpr int NS = HsArgs<R>::NS;
+  phillips_series(a.kappa, NS, a.lns, a.prss);
   // eight levels per thread share the column's exp and profiles; four while
   // that leaves fewer than eight CTAs per SM
   const int nx = ceil_div(ng, 128);

@@ -40,6 +40,12 @@ template <typename R>
 // lb: levels per warp, 4 or 8 (0: 4 up to 64 levels, else 8)
 void launch_dyn_columns(const ColumnArgs<R>& a, bool inverse_only, cudaStream_t s, int lb = 0);
 
+// First n coefficients of the power series in ((p1 - p0) / (p1 + p0))^2 of
+// ln(prs / pm) and prs / pm, prs the Phillips pressure of the layer p0..p1 and pm
+// its mean pressure.
+template <typename R>
+void phillips_series(R kappa, int n, R* lns, R* prss);
+
 template <typename R>
 struct HsArgs {
   int L, nlon, nlat;
@@ -56,9 +62,7 @@ struct HsArgs {
   const R* vfact;  // [L] bottom to top
   R kappa;
   R sigbot, kdrag, krada, kradb, expo;
-  // filled in by the launcher: levels per thread, and the power series in
-  // ((p1 - p0) / (p1 + p0))^2 of ln(prs / pm) and prs / pm, prs the Phillips
-  // pressure of the layer p0..p1 and pm its mean pressure
+  // filled in by the launcher: levels per thread, phillips_series
   static constexpr int NS = 20;
   int lt;
   R lns[NS], prss[NS];

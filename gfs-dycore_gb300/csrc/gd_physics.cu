@@ -58,14 +58,33 @@ struct SimpleConst {
   static constexpr double pi = 3.14159265358979323846, a = 6371220.0, omega = 7.29212e-5;
 };
 
+// quotients; by the short reciprocal in the FP64 state
+__device__ __forceinline__ float quot(float a, float b) { return a / b; }
+__device__ __forceinline__ double quot(double a, double b) { return a * crcp(b); }
+// (1 / x)^(2/7), the Exner factor of x = p / p0, FP64: one step of the
+// third-order iteration y (1 + e/7 + (4/49) e^2), e = 1 - x^2 y^7, on the FP32
+// power (e below 4e-5; the next term, 0.06 e^3, is below 4e-15 e).  A dozen
+// multiply-adds in place of a quotient and a power.
+__device__ __forceinline__ double exner(double x) {
+  static_assert(SimpleConst<double>::rair * 7 == SimpleConst<double>::cpair * 2, "kappa is 2/7");
+  const double y = (double)exp2f(-2.f / 7.f * log2f((float)x));
+  const double y2 = y * y, y4 = y2 * y2, y7 = y4 * y2 * y;
+  const double e = fma(-(x * x), y7, 1.0);
+  return fma(y * e, fma(e, 4.0 / 49.0, 1.0 / 7.0), y);
+}
+
 }  // namespace
 
 // Thread per column; LMAX bounds the level count of the per-thread arrays.
 // The sweeps are dependent chains per thread, so the kernel lives on
 // occupancy: 16 CTAs of 128 threads per SM for the FP32 state (32
-// registers), 5 for FP64.
+// registers), 5 for FP64.  The FP64 state is bound by the FP64 pipe: layer
+// pressures by their power series (k_hs), the Exner factor by iteration and
+// short reciprocals in place of three powers and some fifteen quotients per
+// level: T126L64 4.37 -> 1.56 ms of a step.
 template <typename R, int LMAX>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics(SimpleArgs<R> a) {
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5)
+    k_simple_physics(const __grid_constant__ SimpleArgs<R> a) {
   typedef SimpleConst<R> K;
   const long ng = (long)a.nlon * a.nlat;
   const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -79,8 +98,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics
   const R* gS = a.gS;
   auto IN = [&](int row, int t) -> R { return gS[(long)(row + (L - 1 - t)) * ng + p]; };  // top-down t
   auto PK = [&](int t) -> R { return a.ak[t] + a.bk[t] * ps; };
-  auto PMID = [&](int t) -> R {  // prs of calc_pressdata (pressure_data.f90:87-88)
-    const R pu = PK(t), pl = PK(t + 1);
+  auto PMID = [&](R pu, R pl) -> R {  // prs of calc_pressdata (pressure_data.f90:87-88), layer pu..pl
+    if (sizeof(R) == 8) {
+      const R sum = pl + pu, z = quot(pl - pu, sum), w = z * z;
+      if (w <= R(0.16))
+        return R(0.5) * sum *
+               (w <= R(0.015625) ? series<R, 9>(a.prss, w) : series<R, SimpleArgs<R>::NS>(a.prss, w));
+    }
     return pow((pow(pl, a.kappa) * pl - pow(pu, a.kappa) * pu) / ((a.kappa + R(1)) * (pl - pu)), R(1) / a.kappa);
   };
   // Layer thickness: the reference differences interface pressures; in
@@ -91,13 +115,14 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics
     return PK(t + 1) - PK(t);
   };
   auto PDELX = [&](int t) -> R { return PK(t + 1) - PK(t); };  // as in PMID
-  auto TEMP = [&](R tv, R q) -> R { return tv / (R(1) + a.fvirt * max(a.qmin, q)); };
+  auto TEMP = [&](R tv, R q) -> R { return quot(tv, R(1) + a.fvirt * max(a.qmin, q)); };
   // large-scale condensation of one level (simple_physics_v5_1.f90:226-255)
   R precl = R(0);
   auto condense = [&](R& t, R& q, R pm, R pdel) {
-    const R qsat = epsilo * e0 / pm * exp(-latvap / rh2o * ((R(1) / t) - R(1) / T0));
+    const R qsat = quot(epsilo * e0, pm) * exp(-latvap / rh2o * (quot(R(1), t) - R(1) / T0));
     if (q > qsat) {
-      const R tmp = R(1) / dt * (q - qsat) / (R(1) + (latvap / cpair) * (epsilo * latvap * qsat / (rair * (t * t))));
+      const R tmp = quot(R(1) / dt * (q - qsat),
+                         R(1) + (latvap / cpair) * quot(epsilo * latvap * qsat, rair * (t * t)));
       t = t + (latvap / cpair * tmp) * dt;
       q = q + (-tmp) * dt;
       precl = precl + tmp * pdel / (gravit * rhow);
@@ -118,7 +143,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics
   if (!a.turbflux) {
     for (int t = 0; t < L; ++t) {
       R q = IN(a.s.trc, t), tt = TEMP(IN(a.s.tv, t), q);
-      condense(tt, q, PMID(t), PDEL(t));
+      condense(tt, q, PMID(PK(t), PK(t + 1)), PDEL(t));
       emit(t, tt, q, IN(a.s.u, t), IN(a.s.v, t));
     }
   } else {
@@ -160,16 +185,26 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics
       const R pint = PK(i);
       if (pint >= R(K::pbltop)) return R(1);
       const R x = R(K::pbltop) - pint;
-      return exp(-(x * x) / (R(K::pblconst) * R(K::pblconst)));
+      return exp(sizeof(R) == 8 ? -(x * x) * R(1 / (K::pblconst * K::pblconst))
+                                : -(x * x) / (R(K::pblconst) * R(K::pblconst)));
     };
     const R qsats = epsilo * e0 / ps * exp(-latvap / rh2o * ((R(1) / Tsurf) - R(1) / T0));
-    // pk^kappa pk at interface i, each computed once (layer pressures of two layers)
+    // pk^kappa pk at interface i, each computed once (layer pressures of two
+    // layers); the FP64 state's layer pressures need none
     auto PKK = [&](int i) -> R {
+      if (sizeof(R) == 8) return R(0);
       const R pk = PK(i);
       return pow(pk, a.kappa) * pk;
     };
     auto PMID2 = [&](int t, R kku, R kkl) -> R {  // Phillips layer pressure from the interface terms
+      if (sizeof(R) == 8) return PMID(PK(t), PK(t + 1));
       return pow((kkl - kku) / ((a.kappa + R(1)) * PDELX(t)), R(1) / a.kappa);
+    };
+    auto EXNER = [&](R pm) -> R {
+      if constexpr (sizeof(R) == 8)
+        return exner(pm * (1 / K::p0));
+      else
+        return pow(p0 / pm, rk);
     };
     // sweep 1: bottom to top, level k with the level below (k+1) and above (k-1)
     R ce[LMAX], cem[LMAX], cfu[LMAX], cfv[LMAX], cft[LMAX], cfq[LMAX], exv[LMAX];
@@ -196,23 +231,23 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics
         pdu = PDEL(k - 1);
         condense(tu, qu, pmu, pdu);
         // interface k, between k-1 and k
-        const R rho = (PK(k) / (rair * (tk + tu) / R(2)));
-        const R x = dt * gravit * gravit * rho * rho / (pmk - pmu);
+        const R rho = quot(PK(k), rair * (tk + tu) / R(2));
+        const R x = quot(dt * gravit * gravit * rho * rho, pmk - pmu);
         const R tp = TAPER(k);
         xm = x * (Kmn * tp);
         xe = x * (Ken * tp);
       }
-      const R rpd = R(1) / pdk;
+      const R rpd = quot(R(1), pdk);
       const R CAm = rpd * xm1, CA = rpd * xe1, CCm = rpd * xm, CC = rpd * xe;
       const R de = R(1) + CA + CC - CA * ce1;
       const R dm = R(1) + CAm + CCm - CAm * cem1;
-      const R ex = pow(p0 / pmk, rk);
-      ce[k] = CC / de;
-      cem[k] = CCm / dm;
-      cfu[k] = (uk + CAm * fu1) / dm;
-      cfv[k] = (vk + CAm * fv1) / dm;
-      cft[k] = (ex * tk + CA * ft1) / de;
-      cfq[k] = (qk + CA * fq1) / de;
+      const R ex = EXNER(pmk);
+      ce[k] = quot(CC, de);
+      cem[k] = quot(CCm, dm);
+      cfu[k] = quot(uk + CAm * fu1, dm);
+      cfv[k] = quot(vk + CAm * fv1, dm);
+      cft[k] = quot(ex * tk + CA * ft1, de);
+      cfq[k] = quot(qk + CA * fq1, de);
       exv[k] = ex;
       xm1 = xm, xe1 = xe;
       ce1 = ce[k], cem1 = cem[k], fu1 = cfu[k], fv1 = cfv[k], ft1 = cft[k], fq1 = cfq[k];
@@ -224,7 +259,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics
     for (int k = 1; k < L; ++k) {
       un = cem[k] * un + cfu[k];
       vn = cem[k] * vn + cfv[k];
-      tn = (ce[k] * tn * exv[k - 1] + cft[k]) / exv[k];
+      tn = quot(ce[k] * tn * exv[k - 1] + cft[k], exv[k]);
       qn = ce[k] * qn + cfq[k];
       emit(k, tn, qn, un, vn);
     }
@@ -236,9 +271,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 16 : 5) k_simple_physics
 }
 
 template <typename R>
-void launch_simple_physics(const SimpleArgs<R>& a, cudaStream_t s) {
-  const long ng = (long)a.nlon * a.nlat;
+void launch_simple_physics(const SimpleArgs<R>& in, cudaStream_t s) {
+  const long ng = (long)in.nlon * in.nlat;
   const int nblk = ceil_div(ng, 128);
+  SimpleArgs<R> a = in;
+  phillips_series(a.kappa, a.NS, a.lns, a.prss);
   if (a.L <= 32)
     k_simple_physics<R, 32><<<nblk, 128, 0, s>>>(a);
   else if (a.L <= 64)

@@ -26,6 +26,8 @@ struct SimpleArgs {
   int test;      // 1: latitude-dependent SST (dcmip 4x); 0: constant SST (5x)
   int turbflux;  // surface fluxes and boundary-layer mixing (dcmip 43 and 5x)
   R fvirt, qmin, grav, kappa;  // con_fvirt, qmin of phy_run_simple.f90:38, con_g, con_rocp
+  static constexpr int NS = 20;
+  R lns[NS], prss[NS];  // filled in by the launcher: phillips_series
 };
 template <typename R>
 void launch_simple_physics(const SimpleArgs<R>& a, cudaStream_t s);
