@@ -22,10 +22,7 @@ constexpr int LMAX = 128;
 // approximations for the FP32 state (relative error ~1e-7, below the FP32
 // state's own rounding), the FP64 state's crcp in gd_common.cuh (operands here
 // are pressures, layer thicknesses and tracer differences, normal numbers).
-__device__ __forceinline__ double cdiv(double a, double b) {
-  const double r = crcp(b), q = a * r;
-  return fma(fma(-b, q, a), r, q);
-}
+__device__ __forceinline__ double cdiv(double a, double b) { return a * crcp(b); }
 __device__ __forceinline__ float cdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float crcp(float a) { return __fdividef(1.f, a); }
 __device__ __forceinline__ float clog(float a) { return __logf(a); }
@@ -34,16 +31,22 @@ __device__ __forceinline__ float clog(float a) { return __logf(a); }
 // p0) in the FP64 state: 2 atanh(z) = 2 z (1 + s), z = dp / (p1 + p0), s = w
 // (1/3 + w/5 + ...), w = z^2, and alfa = z - (1 - z) s.  For thin layers this
 // is both cheaper than a quotient and a logarithm and free of alfa's
-// cancellation.  w <= 1/64: 8 terms, w <= 0.16: 19 terms (remainders below
-// 3e-18); thicker layers take the logarithm.
+// cancellation.  w < 2^-10: 5 terms, w < 1/64: 8, w < 0.16: 19 (remainders
+// below 3e-18); thicker layers take the logarithm.  The ranges are told apart by
+// w's high word (comparisons run on the FP64 pipe).
 __device__ __forceinline__ void layer_log(double p0, double p1, double dp, double& rl, double& al) {
   const double z = dp * crcp(p1 + p0), w = z * z;
+  const int hw = __double2hiint(w);
   double s;
-  if (w <= 0.015625) {
+  if (hw < 0x3f500000) {
+    s = 1.0 / 11;
+#pragma unroll
+    for (int k = 9; k >= 3; k -= 2) s = fma(s, w, 1.0 / k);
+  } else if (hw < 0x3f900000) {
     s = 1.0 / 17;
 #pragma unroll
     for (int k = 15; k >= 3; k -= 2) s = fma(s, w, 1.0 / k);
-  } else if (w <= 0.16) {
+  } else if (hw < 0x3fc47ae1) {  // 0.16
     s = 1.0 / 39;
 #pragma unroll
     for (int k = 37; k >= 3; k -= 2) s = fma(s, w, 1.0 / k);
@@ -294,17 +297,19 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
   const R dphx = a.dphisdx[p], dphy = a.dphisdy[p];
   R uu[LB], vv[LB], idpa[LB];
   R pkb3 = PK(L - b0), bpb3 = __ldg(bk + L - b0) * crcp(pkb3);
+  // the level's values and the differences across its bottom interface (from
+  // the level below)
   R um = R(0), vm = R(0), tm = R(0);
   R uc = R(0), vc = R(0), tc = R(0);
   if (nb > 0) {
-    if (b0 > 0) {
-      um = S(a.s.u + b0 - 1);
-      vm = S(a.s.v + b0 - 1);
-      tm = S(a.s.tv + b0 - 1);
-    }
     uc = S(a.s.u + b0);
     vc = S(a.s.v + b0);
     tc = S(a.s.tv + b0);
+    if (b0 > 0) {
+      um = S(a.s.u + b0 - 1) - uc;
+      vm = S(a.s.v + b0 - 1) - vc;
+      tm = S(a.s.tv + b0 - 1) - tc;
+    }
   }
 #pragma unroll
   for (int i = 0; i < LB; ++i) {
@@ -365,9 +370,13 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
       const R e1 = ETA(t + 1), e0 = ETA(t);
       const R h = R(0.5) * idp;
       const R h1 = b > 0 ? h * e1 : R(0), h0 = b + 1 < L ? h * e0 : R(0);
-      const R vu = h1 * (um - uc) + h0 * (uc - up);
-      const R vvv = h1 * (vm - vc) + h0 * (vc - vp);
-      const R vt = h1 * (tm - tc) + h0 * (tc - tp);
+      const R du = uc - up, dw = vc - vp, dt = tc - tp;
+      const R vu = h1 * um + h0 * du;
+      const R vvv = h1 * vm + h0 * dw;
+      const R vt = h1 * tm + h0 * dt;
+      um = du;
+      vm = dw;
+      tm = dt;
       R vq = a.kappa * dlnpdt * tc;
       if (a.nt > 0) vq = cdiv(vq, R(1) + a.cvap_cp * S(a.s.trc + b));
       const R vr = S(a.s.vrt + b);
@@ -381,9 +390,6 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
         SV += rl * dty;
       }
     }
-    um = uc;
-    vm = vc;
-    tm = tc;
     uc = up;
     vc = vp;
     tc = tp;
@@ -460,7 +466,14 @@ static void launch_cols_lb(const ColumnArgs<R>& a, bool inverse_only, cudaStream
 template <typename R>
 void launch_dyn_columns(const ColumnArgs<R>& a, bool inverse_only, cudaStream_t s, int lb) {
   if (a.L < 1 || a.L > LMAX) throw std::runtime_error("nlev out of range for the column kernel");
-  // levels per warp (at most 16 warps per CTA): 4, or 8 when asked or above 64 levels
+  // Levels per warp (at most 16 warps per CTA): 8 above 64 levels, else as
+  // asked.  By default 4 in the FP32 state (8: T574L64 4.49 -> 5.07 ms of a step,
+  // T62L28 0.081 -> 0.093).  The FP64 state with more than 32 levels takes 8, which
+  // halves the work at the blocks' edges (4 -> 8: T254L64 19.8 -> 18.1 ms,
+  // T126L64 4.91 -> 4.52, T42L64 0.558 -> 0.522), once every SM has a CTA; with
+  // fewer levels neither is the better one throughout (T126L28 2.16 -> 2.07,
+  // T94L28 1.07 -> 1.14, T42L20 0.201 -> 0.212).
+  if (lb == 0) lb = sizeof(R) == 8 && a.L > 32 && (long)a.nlon * a.nlat >= 152 * 32 ? 8 : 4;
   if (a.L <= 64 && lb != 8)
     launch_cols_lb<R, 4, 16>(a, inverse_only, s);
   else

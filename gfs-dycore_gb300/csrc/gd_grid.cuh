@@ -37,7 +37,7 @@ struct ColumnArgs {
 };
 
 template <typename R>
-// lb: levels per warp, 4 or 8 (0: 4 up to 64 levels, else 8)
+// lb: levels per warp, 4 or 8 (0: by the levels, the grid and the type; 8 above 64 levels)
 void launch_dyn_columns(const ColumnArgs<R>& a, bool inverse_only, cudaStream_t s, int lb = 0);
 
 // First n coefficients of the power series in ((p1 - p0) / (p1 + p0))^2 of
