@@ -281,8 +281,35 @@ class Dycore : public DycoreBase {
         return;
       }
     }
-    synth_orders(a);
-    if (b) synth_orders(*b);
+    Leg c[2] = {a, b ? *b : a};
+    TailJob t[2];
+    int nt = 0;
+    for (int i = 0; i < (b ? 2 : 1); ++i)
+      if (take_tail(c[i], &t[nt])) ++nt;
+    if (nt) synth_tail(t, nt);
+    synth_orders(c[0]);
+    if (b) synth_orders(c[1]);
+  }
+  // The last two columns of an FP32 transform go beside the GEMM where they
+  // would be a 128-column tile of their own and a tile's work items are several
+  // per SM: with 64 levels, a step's Legendre phases T574 14.9 -> 14.2 ms, T382 6.33
+  // -> 5.96, T254 2.33 -> 2.25, T170 1.27 -> 1.25, but T126 0.79 -> 0.80 and T62 0.33 -> 0.37.
+  bool take_tail(Leg& l, TailJob* t) const {
+    if constexpr (std::is_same<R, float>::value) {
+      const int n = l.ncr - kTail;
+      if (!tcp || n <= 0 || n % 128 || T < kTailT || nh > 2048) return false;
+      l.ncr = n;
+      *t = TailJob{l.in + n, l.ldin, l.out + n, l.ldout, l.useH ? 1 : 0, nullptr};
+      return true;
+    }
+    return false;
+  }
+  static constexpr int kTailT = 150;
+  void synth_tail(const TailJob* t, int n) {
+    if constexpr (std::is_same<R, float>::value) launch_synth_tail(sd, t, n, stream);
+  }
+  void anal_tail(const TailJob& t) {
+    if constexpr (std::is_same<R, float>::value) launch_anal_tail(sd, t, stream);
   }
   void do_anal(const Leg& a, const Leg* b = nullptr) {
     if (!simt()) {
@@ -296,8 +323,13 @@ class Dycore : public DycoreBase {
         return;
       }
     }
-    anal_orders(a);
-    if (b) anal_orders(*b);
+    for (const Leg* l : {&a, b}) {
+      if (!l) continue;
+      Leg c = *l;
+      TailJob t;
+      if (take_tail(c, &t)) anal_tail(t);
+      anal_orders(c);
+    }
   }
   void synth_orders(const Leg& a) {
     if (!tcp) {

@@ -73,6 +73,21 @@ void launch_synth0(const ShtDev<R>& d, const Order0<R>* jobs, int njobs, cudaStr
 template <typename R>
 void launch_anal0(const ShtDev<R>& d, const Order0<R>* jobs, int njobs, cudaStream_t s);
 
+// The last two columns of a transform of orders m >= 1, FP32, beside the
+// tensor-core GEMMs of the columns before them; up to two tables' jobs per
+// synthesis launch
+constexpr int kTail = 2;
+struct TailJob {
+  const float* in;  // first of the columns
+  long ldin;
+  float* out;
+  long ldout;
+  int parityH;
+  const float* tab;  // filled in by the launcher
+};
+void launch_synth_tail(const ShtDev<float>& d, const TailJob* jobs, int njobs, cudaStream_t s);
+void launch_anal_tail(const ShtDev<float>& d, const TailJob& job, cudaStream_t s);
+
 // Longitude stage.
 struct SynthDesc {  // a run of output grid rows
   int count;        // rows in the run

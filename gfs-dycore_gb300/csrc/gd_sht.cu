@@ -400,6 +400,119 @@ template void launch_anal<double>(const ShtDev<double>&, bool, const GemmPlan&, 
 template void launch_anal<float>(const ShtDev<float>&, bool, const GemmPlan&, const float*, long, int, float*,
                                  long, cudaStream_t);
 
+// The two columns past the last full 128-column tile of the tensor-core GEMMs (a
+// state's ln ps beside 64 levels of everything else): a tile of their own would
+// cost them a full tile's time.  Orders m >= 1, IEEE FP32.
+// Bound by the read of the table (T574: 0.38 GB in 0.115 ms for both tables'
+// synthesis, 0.19 GB in 0.065 ms for an analysis; the tile took 0.22 and 0.13).  Synthesis: a warp takes four latitude pairs,
+// its lanes the degrees (a lane's all of one parity), and one butterfly at
+// the end.  Analysis: a lane takes four degrees 32 apart, a warp an eighth of
+// the latitudes; the warps' sums meet in shared memory.
+__global__ void __launch_bounds__(256) k_synth_tail(int T, int nh, int nlat, const long* __restrict__ moff,
+                                                    const long* __restrict__ toff, TailJob jobP, TailJob jobH) {
+  const TailJob g = blockIdx.z ? jobH : jobP;
+  extern __shared__ float xs[];  // [K][kTail]
+  constexpr int NJ = 4;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = blockIdx.y + 1, K = T - m + 1;
+  const float* in = g.in + moff[m] * g.ldin;
+  for (int i = threadIdx.x; i < K * kTail; i += 256) xs[i] = in[(long)(i / kTail) * g.ldin + i % kTail];
+  __syncthreads();
+  const int j0 = (blockIdx.x * 8 + w) * NJ;
+  if (j0 >= nh) return;
+  const float* tab[NJ];
+#pragma unroll
+  for (int r = 0; r < NJ; ++r) tab[r] = g.tab + toff[m] + (long)min(j0 + r, nh - 1) * K;
+  float acc[NJ][kTail] = {};
+#pragma unroll 4
+  for (int q = lane; q < K; q += 32) {
+    float x[kTail];
+#pragma unroll
+    for (int c = 0; c < kTail; ++c) x[c] = xs[q * kTail + c];
+#pragma unroll
+    for (int r = 0; r < NJ; ++r) {
+      const float t = __ldg(tab[r] + q);
+#pragma unroll
+      for (int c = 0; c < kTail; ++c) acc[r][c] += t * x[c];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NJ; ++r)
+#pragma unroll
+    for (int c = 0; c < kTail; ++c) {
+      float v = acc[r][c];
+#pragma unroll
+      for (int o = 16; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      const float u = __shfl_xor_sync(0xffffffffu, v, 1);  // lane 0: v = E, u = O; lane 1: v = O, u = E
+      const int j = j0 + r;
+      if (j < nh && lane == 0) g.out[((long)m * nlat + j) * g.ldout + c] = v + u;
+      if (j < nh && lane == 1) g.out[((long)m * nlat + (nlat - 1 - j)) * g.ldout + c] = g.parityH ? v - u : u - v;
+    }
+}
+__global__ void __launch_bounds__(256) k_anal_tail(int T, int nh, int nlat, const long* __restrict__ moff,
+                                                   const long* __restrict__ toff, TailJob g) {
+  extern __shared__ float eo[];  // [nh][2][kTail]: what pairs with the even degrees, with the odd ones
+  __shared__ float red[8][128][kTail];
+  constexpr int NQ = 4;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = blockIdx.y + 1, K = T - m + 1, q0 = blockIdx.x * 128;
+  if (q0 >= K) return;
+  const float* in = g.in + (long)m * nlat * g.ldin;
+  for (int i = threadIdx.x; i < nh * kTail; i += 256) {
+    const int j = i / kTail, c = i % kTail;
+    const float n = in[(long)j * g.ldin + c], s = in[(long)(nlat - 1 - j) * g.ldin + c];
+    const float p = n + s, d = n - s;
+    eo[(2 * j) * kTail + c] = g.parityH ? d : p;
+    eo[(2 * j + 1) * kTail + c] = g.parityH ? p : d;
+  }
+  __syncthreads();
+  const float* tab = g.tab + toff[m];
+  int q[NQ];
+#pragma unroll
+  for (int i = 0; i < NQ; ++i) q[i] = min(q0 + 32 * i + lane, K - 1);
+  const int par = lane & 1;
+  float acc[NQ][kTail] = {};
+#pragma unroll 8
+  for (int j = w; j < nh; j += 8) {
+    float x[kTail];
+#pragma unroll
+    for (int c = 0; c < kTail; ++c) x[c] = eo[(2 * j + par) * kTail + c];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      const float t = __ldg(tab + (long)j * K + q[i]);
+#pragma unroll
+      for (int c = 0; c < kTail; ++c) acc[i][c] += t * x[c];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NQ; ++i)
+#pragma unroll
+    for (int c = 0; c < kTail; ++c) red[w][32 * i + lane][c] = acc[i][c];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 128 * kTail; i += 256) {
+    const int qq = i / kTail, c = i % kTail;
+    if (q0 + qq >= K) continue;
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v += red[k][qq][c];
+    g.out[(moff[m] + q0 + qq) * g.ldout + c] = v;
+  }
+}
+void launch_synth_tail(const ShtDev<float>& d, const TailJob* jobs, int njobs, cudaStream_t s) {
+  TailJob g[2] = {jobs[0], jobs[njobs - 1]};
+  for (auto& t : g) t.tab = t.parityH ? d.H : d.P;
+  k_synth_tail<<<dim3(ceil_div(d.nh, 32), d.T, njobs), 256, sizeof(float) * kTail * d.T, s>>>(d.T, d.nh, d.nlat, d.moff,
+                                                                                          d.toff, g[0], g[1]);
+  count_launch();
+  GD_LAUNCH_CHECK();
+}
+void launch_anal_tail(const ShtDev<float>& d, const TailJob& job, cudaStream_t s) {
+  TailJob g = job;
+  g.tab = g.parityH ? d.H : d.P;
+  k_anal_tail<<<dim3(ceil_div(d.T, 128), d.T), 256, sizeof(float) * 2 * kTail * d.nh, s>>>(d.T, d.nh, d.nlat, d.moff,
+                                                                                        d.toff, g);
+  count_launch();
+  GD_LAUNCH_CHECK();
+}
+
 // Order 0 of the split modes (the zonal means, on the IEEE path): real
 // coefficients, so only the real parts are summed -- half the multiply-adds of
 // the general kernels above; the imaginary parts (zero for a real field) are
