@@ -416,6 +416,52 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs& a, int idx) {
   return t;
 }
 
+// Columns g..g+15 of an item's E (e) and O (o) sums of batch column c to their
+// rows.  One multiply-add per address: four epilogue warps, one per scheduler,
+// store a whole tile, and with row products and range tests at every element
+// their instructions took longer than the tile's MMAs (T254L64, the largest
+// synthesis GEMM 207 -> 162 us; 112 -> 72 million instructions).
+__device__ __forceinline__ void tc_store16(const TcArgs& a, const TcItem& t, float* out, int g, int c, const float* e,
+                                           const float* o) {
+  const long ld = a.ldout;
+  if (a.mode == 0) {
+    const int j = t.n0 + g, n = a.nh - j;
+    float* const pn = out + ((long)t.m * a.nlat + j) * ld + c;
+    float* const ps = out + ((long)t.m * a.nlat + (a.nlat - 1 - j)) * ld + c;
+    const float sg = a.parityH ? -1.f : 1.f;
+    if (n >= 16) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        pn[q * ld] = e[q] + o[q];
+        ps[-q * ld] = sg * (e[q] - o[q]);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        if (q < n) {
+          pn[q * ld] = e[q] + o[q];
+          ps[-q * ld] = sg * (e[q] - o[q]);
+        }
+    }
+  } else {
+    const int q0 = 2 * (t.n0 + g), n = t.K - q0;  // degrees left
+    float* const p = out + (a.moff[t.m] + q0) * ld + c;
+    if (n >= 32) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        p[2 * q * ld] = e[q];
+        p[(2 * q + 1) * ld] = o[q];
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        if (2 * q < n) p[2 * q * ld] = e[q];
+        if (2 * q + 1 < n) p[(2 * q + 1) * ld] = o[q];
+      }
+    }
+  }
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(TCP_THREADS, 1)
     k_tc_gemm_p(const __grid_constant__ CUtensorMap mA0h, const __grid_constant__ CUtensorMap mA0l,
@@ -552,26 +598,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
         else
 #pragma unroll
           for (int q = 0; q < 16; ++q) o[q] = 0.f;
-        if (c < a.ncols) {
-          if (a.mode == 0) {
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-              const int j = t.n0 + g + q;
-              if (j < a.nh) {
-                a.out[((long)t.m * a.nlat + j) * a.ldout + c] = e[q] + o[q];
-                a.out[((long)t.m * a.nlat + (a.nlat - 1 - j)) * a.ldout + c] = a.parityH ? o[q] - e[q] : e[q] - o[q];
-              }
-            }
-          } else {
-            const long base = a.moff[t.m];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-              const int qe = 2 * (t.n0 + g + q), qo = qe + 1;
-              if (qe < t.K) a.out[(base + qe) * a.ldout + c] = e[q];
-              if (qo < t.K) a.out[(base + qo) * a.ldout + c] = o[q];
-            }
-          }
-        }
+        if (c < a.ncols) tc_store16(a, t, a.out, g, c, e, o);
       }
       tc_fence_before();
       __syncwarp();
@@ -810,17 +837,26 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
         // convert before waiting for the A slot: the loads and the split
         // overlap the MMAs still reading it
         uint32_t h[16], l[16];
+        float v[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const int ii = k0 + e;
-          float v = raw[ii * TC_M + c];
-          if (a.mode == 1) {
-            const float w = raw[(2 * kc - 1 - ii) * TC_M + c];  // mirrored row nlat-1-j
-            v = plus ? v + w : v - w;
+        for (int e = 0; e < 16; ++e) v[e] = raw[(k0 + e) * TC_M + c];
+        if (a.mode == 1) {  // mirrored rows nlat-1-j
+          const float* mir = raw + (2 * kc - 1 - k0) * TC_M + c;
+          if (plus) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] += mir[-e * TC_M];
+          } else {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] -= mir[-e * TC_M];
           }
-          if (ii >= nv) v = 0.f;
-          Elem<TC_TF32>::splitf(v, h[e], l[e]);
         }
+        if (k0 + 16 > nv) {  // the last chunk
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            if (k0 + e >= nv) v[e] = 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) Elem<TC_TF32>::splitf(v[e], h[e], l[e]);
         // the slot's previous contents fed chunk g - na
         if (g >= na) {
           const bool oku = mbar_wait(smem_u32(&used[rp.slot]), rp.ph, a.err, 27);
@@ -865,24 +901,20 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
           const uint32_t ts = lw + (uint32_t)b * bw, tr = lw + rcol + (j < nsE ? 0u : (uint32_t)N);
           const bool first = j == 0 || j == nsE;
           for (int g = 0; g < N; g += 16) {
-            float v[16];
-            uint32_t w[16];
-            tmem_ld16(ts + g, v);
+            uint32_t v[16], x[16], r[16];
+            tmem_ld16_issue(ts + g, v);
+            if (a.sepx) tmem_ld16_issue(ts + N + g, x);
+            if (!first) tmem_ld16_issue(tr + g, r);
+            tmem_ld_wait();
             if (a.sepx) {
-              float x[16];
-              tmem_ld16(ts + N + g, x);
 #pragma unroll
-              for (int q = 0; q < 16; ++q) v[q] += x[q];
+              for (int q = 0; q < 16; ++q) v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(x[q]));
             }
             if (!first) {
-              float r[16];
-              tmem_ld16(tr + g, r);
 #pragma unroll
-              for (int q = 0; q < 16; ++q) v[q] = r[q] + v[q];
+              for (int q = 0; q < 16; ++q) v[q] = __float_as_uint(__uint_as_float(r[q]) + __uint_as_float(v[q]));
             }
-#pragma unroll
-            for (int q = 0; q < 16; ++q) w[q] = __float_as_uint(v[q]);
-            tmem_st16(tr + g, w);
+            tmem_st16(tr + g, v);
           }
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           tc_fence_before();
@@ -902,47 +934,33 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
       const int c = t.c0 + q4 * 32 + lane;
       for (int g = 0; g < N; g += 16) {
         float e[16], o[16];
-        tmem_ld16(tw + g, e);
+        uint32_t re[16], ro[16];
+        tmem_ld16_issue(tw + g, re);
         if (t.nk1 > 0)
-          tmem_ld16(tw + N + g, o);
+          tmem_ld16_issue(tw + N + g, ro);
         else
 #pragma unroll
-          for (int q = 0; q < 16; ++q) o[q] = 0.f;
+          for (int q = 0; q < 16; ++q) ro[q] = 0u;
         if (a.sepx && !fold) {  // add the cross products' accumulator (round to nearest)
-          float xe[16], xo[16];
-          tmem_ld16(tw + 2 * N + g, xe);
+          uint32_t xe[16], xo[16];
+          tmem_ld16_issue(tw + 2 * N + g, xe);
           if (t.nk1 > 0)
-            tmem_ld16(tw + 3 * N + g, xo);
+            tmem_ld16_issue(tw + 3 * N + g, xo);
           else
 #pragma unroll
-            for (int q = 0; q < 16; ++q) xo[q] = 0.f;
+            for (int q = 0; q < 16; ++q) xo[q] = 0u;
+          tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 16; ++q) {
-            e[q] += xe[q];
-            o[q] += xo[q];
+            e[q] = __uint_as_float(re[q]) + __uint_as_float(xe[q]);
+            o[q] = __uint_as_float(ro[q]) + __uint_as_float(xo[q]);
           }
-        }
-        if (c < a.ncols) {
-          if (a.mode == 0) {
+        } else {
+          tmem_ld_wait();
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-              const int j = t.n0 + g + q;
-              if (j < a.nh) {
-                a.out[((long)t.m * a.nlat + j) * a.ldout + c] = e[q] + o[q];
-                a.out[((long)t.m * a.nlat + (a.nlat - 1 - j)) * a.ldout + c] = a.parityH ? o[q] - e[q] : e[q] - o[q];
-              }
-            }
-          } else {
-            const long base = a.moff[t.m];
-            float* const out = a.out + (long)t.seg * a.seg_stride;
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-              const int qe = 2 * (t.n0 + g + q), qo = qe + 1;
-              if (qe < t.K) out[(base + qe) * a.ldout + c] = e[q];
-              if (qo < t.K) out[(base + qo) * a.ldout + c] = o[q];
-            }
-          }
+          for (int q = 0; q < 16; ++q) e[q] = __uint_as_float(re[q]), o[q] = __uint_as_float(ro[q]);
         }
+        if (c < a.ncols) tc_store16(a, t, a.out + (long)t.seg * a.seg_stride, g, c, e, o);
       }
       if (bt >= 0) {
         tc_fence_before();
