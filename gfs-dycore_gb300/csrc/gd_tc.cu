@@ -1064,6 +1064,14 @@ static int tcf_slots(const TcPlan& p, int n) {
   return na;
 }
 
+static bool fused_off() {
+  static const bool off = [] {
+    const char* e = getenv("GD_TC_FUSED");
+    return e && e[0] == '0';
+  }();
+  return off;
+}
+
 int tc_slots(const TcPlan& p, int n) { return tcf_slots(p, n); }
 
 int tc_max_n(const TcPlan& p) {
@@ -1096,9 +1104,13 @@ void tc_init(TcPlan& p, int kind, int T, int nh, int nlat, int ncap, const long*
   // the fused TF32 path also keeps two A slots in TMEM and, as configured,
   // cross-product accumulators and running sums (wider tiles, single-
   // buffered, by the plan's tile cap or the autotuner)
-  const int ncap_n = !p.persistent ? 160 : kind == TC_TF32 ? std::min(tc_max_n(p), p.tile_cap) : 128;
+  const int ncap_n = !p.persistent                     ? 160
+                     : kind == TC_TF32 && !fused_off() ? std::min(tc_max_n(p), p.tile_cap)
+                                                       : 128;
   p.nsyn = tile_n(nh, ncap_n);
-  p.nana = tile_n(kemax, ncap_n);
+  // at most 160 degrees: with the mirrored rows in a stage, wider tiles leave
+  // the ring two stages (T382L64, 192: analyses 2.27 -> 2.50 ms of a step)
+  p.nana = tile_n(kemax, std::min(ncap_n, 160));
   p.kirows = round_up(kemax, p.nana);
   p.ncap = round_up(ncap, 32);
   p.xbase.assign(T + 1, 0);
@@ -1241,11 +1253,7 @@ static int4* cached_items(TcPlan& p, long key, const std::vector<int4>& it) {
 }
 
 static bool fused_ok(const TcPlan& p, const void* base, long ld) {
-  static const bool off = [] {
-    const char* e = getenv("GD_TC_FUSED");
-    return e && e[0] == '0';
-  }();
-  return !off && p.kind == TC_TF32 && p.persistent && p.nsyn <= tc_max_n(p) && p.nana <= tc_max_n(p) &&
+  return !fused_off() && p.kind == TC_TF32 && p.persistent && p.nsyn <= tc_max_n(p) && p.nana <= tc_max_n(p) &&
          ((uintptr_t)base % 16) == 0 && ld % 4 == 0;
 }
 

@@ -40,9 +40,13 @@ struct TcPlan {
   // fused TF32x3 GEMM: A-operand slots in tensor memory requested (2..4; a
   // launch gets as many as fit beside its accumulators)
   int aslots = 2;
-  // widest N tile tc_init chooses for the fused TF32x3 GEMM (tiles above 96
-  // are single-buffered in TMEM); the autotuner may widen the synthesis tile
-  int tile_cap = 96;
+  // widest N tile tc_init chooses for the fused TF32x3 GEMM, as far as tensor
+  // memory holds it (tiles above 96 are single-buffered).  A chunk's operand tile
+  // is read from L2 once per N tile, and that traffic bounds the GEMM: cap 96 ->
+  // 192, one step's syntheses and analyses T574L64 8.22 -> 6.89 and 5.12 -> 4.72
+  // ms, T382L64 3.19 -> 2.90 and (capped at 160) the same, T254L64 1.32 -> 1.20 and
+  // 1.17 -> 1.07, T170L64 0.63 -> 0.54 ms; T126 and below need no wider tile
+  int tile_cap = 192;
   // fused TF32x3 analysis: the latitude sum in aseg segments, each written as
   // FP32 partial sums to its own copy of the output (nlm x ldA floats apart),
   // to be added in the caller's precision; set by the FP64-state modes
