@@ -164,8 +164,13 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
   const bool brief = inverse_only && !a.dlnpdtg;
   auto PART = [&](int q, int ww) -> R& { return part[(q * NW + ww) * 32 + lane]; };
   auto ETA = [&](int t) -> R& { return etas[t * 32 + lane]; };
-  const R* gS = a.gS;
-  auto S = [&](int row) -> R { return __ldg(gS + (long)row * ng + p); };
+  // Rows of the grid arrays at this column.  A 32-bit row pitch in bytes makes
+  // each address one multiply-add: 64-bit products took a good part of the FP32
+  // kernel's 900 instructions per level (its issue slots bound it: T574L64 5.02
+  // -> 4.16 ms of a step, T254L64 2.05 -> 1.72).
+  const int pitch = (int)(ng * sizeof(R));
+  const char* gS = reinterpret_cast<const char*>(a.gS + p);
+  auto S = [&](int row) -> R { return __ldg(reinterpret_cast<const R*>(gS + (long)row * pitch)); };
   const R* ak = a.ak;
   const R* bk = a.bk;
   const R* dbk = a.dbk;
@@ -289,9 +294,9 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
   __syncthreads();
 
   // phase 3
-  R* gA = a.gA;
+  char* gA = reinterpret_cast<char*>(a.gA + p);
   auto A = [&](int row, R v) {
-    if (valid) gA[(long)row * ng + p] = v;
+    if (valid) *reinterpret_cast<R*>(gA + (long)row * pitch) = v;
   };
   const R fcor = a.omega2 * a.sinlat[j];
   const R dphx = a.dphisdx[p], dphy = a.dphisdy[p];

@@ -1682,7 +1682,10 @@ __global__ void __launch_bounds__(((nr4_of<R>() * (M1 > M2 ? M1 : M2) + 31) / 32
   const int col = r0 + r;
   R* pP = ds.dstP >= 0 ? GP + (long)j * ldP + 2 * (ds.dstP + col) : nullptr;
   R* pH = ds.dstH >= 0 ? GH + (long)j * ldH + 2 * (ds.dstH + col) : nullptr;
-  const long sP = (long)nlat * ldP, sH = (long)nlat * ldH;
+  const int sP = (int)(nlat * ldP * sizeof(R)), sH = (int)(nlat * ldH * sizeof(R));  // bytes between orders: 32-bit, one multiply-add per address
+  auto at = [](R* q, int k, int step) -> V& {
+    return *reinterpret_cast<V*>(reinterpret_cast<char*>(q) + (long)k * step);
+  };
   // the quadrature weight and the output's scale in one factor
   const R scP = (R)ds.scaleP * wn * (ds.imcosP ? rc : R(1)), scH = (R)ds.scaleH * wn;
   const V* brow = buf + r * RP;
@@ -1713,9 +1716,9 @@ __global__ void __launch_bounds__(((nr4_of<R>() * (M1 > M2 ? M1 : M2) + 31) / 32
       } else {
         y = mk2<R>(scP * X.x, scP * X.y);
       }
-      *reinterpret_cast<V*>(pP + k * sP) = y;
+      at(pP, k, sP) = y;
     }
-    if (pH) *reinterpret_cast<V*>(pH + k * sH) = mk2<R>(scH * X.x, scH * X.y);
+    if (pH) at(pH, k, sH) = mk2<R>(scH * X.x, scH * X.y);
   };
   for (int kk = kq; kk <= M / 2; kk += KS) {
     // E = Z_k + conj Z_(M-k), D = -i (Z_k - conj Z_(M-k)) w_k, w_k = exp(-2 pi i k
