@@ -1270,8 +1270,8 @@ static void launch_fused(const TcPlan& p, const CUtensorMap& raw, const CUtensor
   }();
   const int ns = (int)std::min<size_t>((size_t)cap, avail / stage);
   args.nbuf = tcf_nbuf(p, args.N);
-  args.na = tcf_slots(p, args.N);
-  if (ns < args.na || args.N > TCF_MAXN || args.N % 16 ||
+  args.na = std::min(tcf_slots(p, args.N), ns);  // a converter is never ahead of the ring
+  if (args.na < 2 || args.N > TCF_MAXN || args.N % 16 ||
       tcf_tmem_cols(args.N, p.sepx, p.cps > 0, args.na, args.nbuf) > 512)
     throw std::runtime_error("tc fused gemm: bad tile");
   const size_t sm = (size_t)ns * stage + 1024 + 256;
