@@ -301,7 +301,7 @@ __device__ __forceinline__ double oz_join(long long hi, long long lo, int k) {
   const double xl = __hiloint2double((int)(lo >> 32) + (0x43380000 + kk), (int)lo);
   const double xh = __hiloint2double((int)(hi >> 32) + (0x45380000 + kk), (int)hi);
   double v = (xh - __hiloint2double(0x45380000 + kk, 0x00180000)) + xl;
-  if (!plain) v = oz_scale(v, k);
+  if (!plain && ((hi | lo) != 0 || k >= OZ_BAD / 2)) v = oz_scale(v, k);  // a zero column's k is out of range too
   return v;
 }
 
