@@ -262,6 +262,7 @@ class Dycore : public DycoreBase {
     int ncr;
     R* out;
     long ldout;
+    OzLeg oz() const { return OzLeg{useH, (const double*)in, ldin, ncr, (double*)out, ldout}; }
     Order0<R> order0() const { return Order0<R>{in, ldin, out, ldout, ncr / 2, useH ? 1 : 0, nullptr}; }
   };
   void do_synth(const Leg& a, const Leg* b = nullptr) {
@@ -270,14 +271,9 @@ class Dycore : public DycoreBase {
       launch_synth0<R>(sd, g, b ? 2 : 1, stream);
     }
     if constexpr (std::is_same<R, double>::value) {
-      if (ozp) {  // both tables read the same columns: one split serves them
-        oz_split_x(*ozp, moff, a.in, a.ldin, a.ncr, stream);
-        oz_synth(*ozp, moff, a.useH, 0, a.ncr, a.out, a.ldout, stream);
-        if (!b) return;
-        const long off = b->in - a.in;
-        const bool shared = b->ldin == a.ldin && off >= 0 && off + b->ncr <= a.ncr;
-        if (!shared) oz_split_x(*ozp, moff, b->in, b->ldin, b->ncr, stream);
-        oz_synth(*ozp, moff, b->useH, shared ? (int)off : 0, b->ncr, b->out, b->ldout, stream);
+      if (ozp) {
+        const OzLeg la = a.oz(), lb = b ? b->oz() : la;
+        oz_synth(*ozp, moff, la, b ? &lb : nullptr, stream);
         return;
       }
     }
@@ -318,8 +314,8 @@ class Dycore : public DycoreBase {
     }
     if constexpr (std::is_same<R, double>::value) {
       if (ozp) {
-        oz_anal(*ozp, moff, a.useH, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
-        if (b) oz_anal(*ozp, moff, b->useH, b->in, b->ldin, b->ncr, b->out, b->ldout, stream);
+        const OzLeg la = a.oz(), lb = b ? b->oz() : la;
+        oz_anal(*ozp, moff, la, b ? &lb : nullptr, stream);
         return;
       }
     }
@@ -430,7 +426,7 @@ class Dycore : public DycoreBase {
         GD_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const int gb = env_int("GD_FP64_TC_GB", -1);
         ozp.reset(new OzPlan());
-        if (!oz_init(*ozp, T, nh, nlat, 2 * std::max(sc.ncol, ap.ncol), gb < 0 ? total_b / 4 : (size_t)gb << 30, moff,
+        if (!oz_init(*ozp, T, nh, nlat, 2 * std::max(sc.ncol, ap.ncol + ah.ncol), gb < 0 ? total_b / 4 : (size_t)gb << 30, moff,
                      toff, P, H, stream))
           ozp.reset();
       }

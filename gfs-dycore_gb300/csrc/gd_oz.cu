@@ -19,11 +19,15 @@
 // through the sets.  The synthesis forms E +- O as integers, before the one
 // rounding; sums over several segments are added in FP64 at the outputs.
 //
-// One step of T126 with 64 levels and 4 tracers (1154 columns; 152 SMs): all its
-// Legendre transforms 18.8 ms on the FP64 pipe (70% of its rate), 4.35 ms here,
-// 0.29 ms the largest GEMM.  That one reads 0.9 GB of operands from L2 and needs 0.13
-// ms for it, 0.11 ms of tensor-core issue and 0.13 ms of FP64 additions; the
-// three overlap in part.  T42 with 20 levels: 0.57 -> 0.46 ms.
+// A launch takes both tables' work (P and dP/dphi), after one split of their
+// operand columns.
+//
+// One step of T126 with 64 levels and 3 tracers (1026 columns; 152 SMs): all its
+// Legendre transforms 18.8 ms on the FP64 pipe (70% of its rate), 3.92 ms here.
+// The syntheses read 0.9 GB of operands from L2 per table and need 0.13 ms for
+// it, 0.11 ms of tensor-core issue and 0.13 ms of FP64 additions; the three
+// overlap in part (0.29 ms).  T42 with 20 levels: 0.57 -> 0.35 ms; with a launch
+// per table 0.47 ms (and 4.35 ms at T126).
 #include <algorithm>
 #include <stdexcept>
 
@@ -122,26 +126,31 @@ __global__ void __launch_bounds__(256) k_oz_table(int mode, int T, int nh, int n
 // in registers between the search for the column's largest exponent and the
 // digits, more are read again.  Bound by integer issue.
 struct OzSplit {
-  int T, nh, nlat, ncols, ncap, nhpad, parityH;
+  int T, nh, nlat, ncap, nhpad;
   const long* moff;
   const long* xbase;
   long xlen;
-  const double* src;
-  long ld;
+  // up to two sources side by side in the operand (blockIdx.z), from column coff
+  const double* src[2];
+  long ld[2];
+  int ncols[2], coff[2], parityH[2];
   uint16_t* out[2];  // mode 0: X (both parities in one row); mode 1: G of each parity
   int* ex[2];        // [(T+1)][ncap]: mode 0 one for both parities, mode 1 per parity
 };
 template <int MODE>
-__global__ void __launch_bounds__(256) k_oz_split(OzSplit a) {
+__global__ void __launch_bounds__(256) k_oz_split(const __grid_constant__ OzSplit a) {
   __shared__ uint32_t t[OZ_S][32][33];
   __shared__ int red[2][8][32];
   constexpr int NU = 8;  // pairs per thread and register block of 128 K entries
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int z = blockIdx.z, ncols = a.ncols[z], parityH = a.parityH[z];
   const int m = blockIdx.x + 1, c0 = blockIdx.y * 32, c = c0 + lane;
+  if (c0 >= ncols) return;  // the grid covers the wider source
+  const long ld = a.ld[z], d0 = a.coff[z] + c0;  // first operand column of the CTA
   const int K = a.T - m + 1, ke = (K + 1) / 2, kp = MODE == 0 ? (ke + 31) / 32 * 32 : a.nhpad;
   const int n0 = MODE == 0 ? ke : a.nh, n1 = MODE == 0 ? K / 2 : a.nh;  // entries of each parity
-  const bool live = c < a.ncols;
-  const double* src = MODE == 0 ? a.src + a.moff[m] * a.ld + c : a.src + (long)m * a.nlat * a.ld + c;
+  const bool live = c < ncols;
+  const double* src = a.src[z] + (MODE == 0 ? a.moff[m] : (long)m * a.nlat) * ld + c;
   double v[2][NU][2];
   // entries k0 + 2 (w + 8 u) + {0, 1} of both parities
   auto load = [&](int k0) {
@@ -152,11 +161,11 @@ __global__ void __launch_bounds__(256) k_oz_split(OzSplit a) {
         const int k = k0 + 2 * (w + 8 * u) + i;
         double x = 0.0, y = 0.0;
         if (MODE == 0) {
-          if (live && k < n0) x = src[(long)(2 * k) * a.ld];
-          if (live && k < n1) y = src[(long)(2 * k + 1) * a.ld];
+          if (live && k < n0) x = src[(long)(2 * k) * ld];
+          if (live && k < n1) y = src[(long)(2 * k + 1) * ld];
         } else if (live && k < n0) {
-          x = src[(long)k * a.ld];
-          y = src[(long)(a.nlat - 1 - k) * a.ld];
+          x = src[(long)k * ld];
+          y = src[(long)(a.nlat - 1 - k) * ld];
         }
         v[0][u][i] = x;
         v[1][u][i] = y;
@@ -167,8 +176,8 @@ __global__ void __launch_bounds__(256) k_oz_split(OzSplit a) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const double p = v[0][u][i] + v[1][u][i], d = v[0][u][i] - v[1][u][i];
-          v[0][u][i] = a.parityH ? d : p;
-          v[1][u][i] = a.parityH ? p : d;
+          v[0][u][i] = parityH ? d : p;
+          v[1][u][i] = parityH ? p : d;
         }
     }
   };
@@ -189,8 +198,8 @@ __global__ void __launch_bounds__(256) k_oz_split(OzSplit a) {
     for (int i = 0; i < 8; ++i) fm[par] = max(fm[par], red[par][i][lane]);
   if (MODE == 0) fm[0] = fm[1] = max(fm[0], fm[1]);
   if (w == 0 && live) {
-    a.ex[0][(long)m * a.ncap + c] = oz_exponent(fm[0]);
-    if (MODE == 1) a.ex[1][(long)m * a.ncap + c] = oz_exponent(fm[1]);
+    a.ex[0][(long)m * a.ncap + d0 + lane] = oz_exponent(fm[0]);
+    if (MODE == 1) a.ex[1][(long)m * a.ncap + d0 + lane] = oz_exponent(fm[1]);
   }
   const long pitch = MODE == 0 ? a.xlen : a.nhpad;
   const long slice = MODE == 0 ? (long)a.ncap * a.xlen : (long)(a.T + 1) * a.ncap * a.nhpad;
@@ -198,8 +207,8 @@ __global__ void __launch_bounds__(256) k_oz_split(OzSplit a) {
     if (n0 > 128) load(k0);
 #pragma unroll
     for (int par = 0; par < 2; ++par) {
-      uint16_t* out = MODE == 0 ? a.out[0] + a.xbase[m] + (long)par * kp + (long)c0 * a.xlen
-                                : a.out[par] + ((long)m * a.ncap + c0) * a.nhpad;
+      uint16_t* out = MODE == 0 ? a.out[0] + a.xbase[m] + (long)par * kp + d0 * a.xlen
+                                : a.out[par] + ((long)m * a.ncap + d0) * a.nhpad;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {  // 64 K entries through shared memory
         if (k0 + 64 * h >= kp) break;
@@ -214,7 +223,7 @@ __global__ void __launch_bounds__(256) k_oz_split(OzSplit a) {
         if (k0 + 64 * h + 2 * lane < kp)
           for (int r = w; r < OZ_S * 32; r += 8) {
             const int b = r >> 5, cc = r & 31;
-            if (c0 + cc < a.ncols)
+            if (c0 + cc < ncols)
               *reinterpret_cast<uint32_t*>(out + b * slice + cc * pitch + k0 + 64 * h + 2 * lane) = t[b][cc][lane];
           }
         __syncthreads();
@@ -231,23 +240,27 @@ struct OzArgs {
   int T, nh, nlat, N, ncap;
   const long* xbase;
   const long* moff;
-  int parityH, ncols, coff;
   const int* ea[2];  // operand exponents [m][ncap] of each parity (synthesis: the same)
-  const int* eb;     // table exponents (synthesis [m nh + j], analysis [spectral row, even degrees first])
-  double* out;
-  long ldout;
+  // up to two tables' jobs on columns [coff, coff + ncols) of the operand
+  struct Job {
+    int parityH, ncols, coff;
+    const int* eb;  // table exponents (synthesis [m nh + j], analysis [spectral row, even degrees first])
+    double* out;
+    long ldout;
+  } job[2];
   int* err;
 };
 // A work item's passes, each through one set of accumulators: a K segment of 128
 // of one parity; in the synthesis a segment's even degrees, then its odd ones (if
 // it has any), in the analysis all segments of the even degrees, then the others'.
 struct OzItem {
-  int m, c0, n0, K, segs, passes;
+  int m, c0, n0, K, segs, passes, job;
   __device__ OzItem(const OzArgs& a, int idx) {
     const int4 it = a.items[idx];
     m = it.x;
     c0 = it.y * OZ_M;
     n0 = it.z * a.N;
+    job = it.w;
     K = a.T - m + 1;
     segs = ((a.mode ? a.nh : degrees(0)) + OZ_SEG - 1) / OZ_SEG;
     passes = a.mode == 0 ? segs + (degrees(1) + OZ_SEG - 1) / OZ_SEG : ncount(a, 1) > 0 ? 2 * segs : segs;
@@ -307,7 +320,8 @@ __device__ __forceinline__ double oz_join(long long hi, long long lo, int k) {
 
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     k_oz_gemm(const __grid_constant__ CUtensorMap mA0, const __grid_constant__ CUtensorMap mA1,
-              const __grid_constant__ CUtensorMap mB, OzArgs a) {
+              const __grid_constant__ CUtensorMap mB0, const __grid_constant__ CUtensorMap mB1,
+              const __grid_constant__ OzArgs a) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~(uintptr_t)1023);
   const uint32_t bbytes = (uint32_t)(OZ_S * a.N * OZ_KC * 2), stage = OZ_ABYTES + bbytes;
@@ -347,7 +361,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     bool bad = false;
     for (int idx = blockIdx.x; idx < a.nitems && !bad; idx += gridDim.x) {
       const OzItem t(a, idx);
-      const int kpx = (t.degrees(0) + 31) / 32 * 32;
+      const int kpx = (t.degrees(0) + 31) / 32 * 32, row = a.job[t.job].coff + t.c0;
       for (int p = 0; p < t.passes && !bad; ++p) {
         const OzPass ps(a, t, p);
         for (int k = ps.k0; k < ps.k0 + ps.kn; k += OZ_KC, ++g) {
@@ -360,14 +374,21 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
           mbar_expect_tx(fb, stage);
           if (a.mode == 0) {
             const int x = (int)a.xbase[t.m] + ps.par * kpx + k;
-            tma_3d(st, &mA0, x, a.coff + t.c0, 0, fb);
-            tma_3d(st + OZ_ABYTES, &mB, x, t.n0, 0, fb);
+            tma_3d(st, &mA0, x, row, 0, fb);
+            if (t.job)
+              tma_3d(st + OZ_ABYTES, &mB1, x, t.n0, 0, fb);
+            else
+              tma_3d(st + OZ_ABYTES, &mB0, x, t.n0, 0, fb);
           } else {
             if (ps.par)
-              tma_3d(st, &mA1, k, t.m * a.ncap + t.c0, 0, fb);
+              tma_3d(st, &mA1, k, t.m * a.ncap + row, 0, fb);
             else
-              tma_3d(st, &mA0, k, t.m * a.ncap + t.c0, 0, fb);
-            tma_3d(st + OZ_ABYTES, &mB, k, (int)a.moff[t.m] + ps.par * t.degrees(0) + t.n0, 0, fb);
+              tma_3d(st, &mA0, k, t.m * a.ncap + row, 0, fb);
+            const int y = (int)a.moff[t.m] + ps.par * t.degrees(0) + t.n0;
+            if (t.job)
+              tma_3d(st + OZ_ABYTES, &mB1, k, y, 0, fb);
+            else
+              tma_3d(st + OZ_ABYTES, &mB0, k, y, 0, fb);
           }
           ++fills[s];
           rs.next(OZ_NS);
@@ -446,18 +467,20 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
     uint32_t lw = 0;
     for (int idx = blockIdx.x; idx < a.nitems && !bad; idx += gridDim.x) {
       const OzItem t(a, idx);
+      const OzArgs::Job& job = a.job[t.job];
       const int c = t.c0 + q4 * 32 + lane;
-      const bool live = c < a.ncols;
+      const bool live = c < job.ncols;
+      const long ldout = job.ldout;
       if (a.mode == 0) {
         // north E + O, south E - O (dP/dphi: O - E), a quarter of the latitudes
         // per warp; E waits in registers as integers, so that the next item's
         // even degrees are multiplied while this one's sums are formed and stored
         const int ng = grp * (a.N / 4), nv = t.ncount(a, 0);
-        const int ea = live ? a.ea[0][(long)t.m * a.ncap + a.coff + c] + 56 : 0;
-        const int* eb = a.eb + (long)t.m * a.nh + t.n0;
-        const int flip = a.parityH ? (int)0x80000000 : 0;
-        double* north = a.out + ((long)t.m * a.nlat + t.n0) * a.ldout + c;
-        double* south = a.out + ((long)t.m * a.nlat + (a.nlat - 1 - t.n0)) * a.ldout + c;
+        const int ea = live ? a.ea[0][(long)t.m * a.ncap + job.coff + c] + 56 : 0;
+        const int* eb = job.eb + (long)t.m * a.nh + t.n0;
+        const int flip = job.parityH ? (int)0x80000000 : 0;
+        double* north = job.out + ((long)t.m * a.nlat + t.n0) * ldout + c;
+        double* south = job.out + ((long)t.m * a.nlat + (a.nlat - 1 - t.n0)) * ldout + c;
         for (int k0 = 0, p = 0; p < t.passes; k0 += OZ_SEG, p += 2) {
           const bool odd = k0 < t.degrees(1), more = k0 > 0;
           if (!begin(&lw)) {
@@ -497,8 +520,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                   double vn = oz_join(eh[i + q] + oh, el[i + q] + ol, k);
                   double vs = oz_join(eh[i + q] - oh, el[i + q] - ol, k);
                   vs = __hiloint2double(__double2hiint(vs) ^ flip, __double2loint(vs));
-                  double* const on = north + n * a.ldout;
-                  double* const os = south - n * a.ldout;
+                  double* const on = north + n * ldout;
+                  double* const os = south - n * ldout;
                   if (more) vn += *on, vs += *os;
                   *on = vn;
                   *os = vs;
@@ -512,10 +535,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         for (int p = 0; p < t.passes; ++p) {
           const OzPass ps(a, t, p);
           const int nv = t.ncount(a, ps.par);
-          const int ea = live ? (ps.par ? a.ea[1] : a.ea[0])[(long)t.m * a.ncap + c] + 56 : 0;
+          const int ea = live ? (ps.par ? a.ea[1] : a.ea[0])[(long)t.m * a.ncap + job.coff + c] + 56 : 0;
           const bool more = ps.k0 > 0;
-          const int* eb = a.eb + a.moff[t.m] + ps.par * t.degrees(0) + t.n0;
-          double* out = a.out + (a.moff[t.m] + 2 * t.n0 + ps.par) * a.ldout + c;
+          const int* eb = job.eb + a.moff[t.m] + ps.par * t.degrees(0) + t.n0;
+          double* out = job.out + (a.moff[t.m] + 2 * t.n0 + ps.par) * ldout + c;
           if (!begin(&lw)) {
             bad = true;
             break;
@@ -527,7 +550,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             for (int q = 0; q < 4; ++q) {
               if (live && n4 + q < nv) {
                 double v = oz_join(oz_int(r, 4, q), oz_int(r, 0, q), ea + __ldg(eb + n4 + q));
-                double* const o = out + 2 * (n4 + q) * a.ldout;
+                double* const o = out + 2 * (n4 + q) * ldout;
                 if (more) v += *o;
                 *o = v;
               }
@@ -557,30 +580,61 @@ void oz_map(CUtensorMap* m, void* base, long k, long rows, int boxrows) {
                                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled (digits) failed: " + std::to_string((int)r));
 }
-const int4* oz_items(OzPlan& p, int ncols, int mode, int* n) {
-  const int ct = (ncols + OZ_M - 1) / OZ_M;
+const int4* oz_items(OzPlan& p, const OzLeg* legs, int nlegs, int mode, int* n) {
+  int ct[2] = {0, 0};
+  for (int i = 0; i < nlegs; ++i) ct[i] = (legs[i].ncols + OZ_M - 1) / OZ_M;
   for (const auto& l : p.items)
-    if (l.ct == ct && l.mode == mode) {
+    if (l.ct[0] == ct[0] && l.ct[1] == ct[1] && l.mode == mode) {
       *n = l.n;
       return l.d;
     }
   std::vector<int4> it;
   for (int m = 1; m <= p.T; ++m) {
     const int nn = mode == 0 ? p.nh : (p.T - m + 2) / 2, N = mode == 0 ? p.nsyn : p.nana;
-    for (int c = 0; c < ct; ++c)
-      for (int b = 0; b * N < nn; ++b) it.push_back(make_int4(m, c, b, 0));
+    for (int i = 0; i < nlegs; ++i)
+      for (int c = 0; c < ct[i]; ++c)
+        for (int b = 0; b * N < nn; ++b) it.push_back(make_int4(m, c, b, i));
   }
-  OzPlan::Items l{ct, mode, (int)it.size(), nullptr};
+  OzPlan::Items l{{ct[0], ct[1]}, mode, (int)it.size(), nullptr};
   GD_CUDA(cudaMalloc(&l.d, sizeof(int4) * it.size()));
   p.items.push_back(l);
   GD_CUDA(cudaMemcpy(l.d, it.data(), sizeof(int4) * it.size(), cudaMemcpyHostToDevice));
   *n = l.n;
   return l.d;
 }
-void oz_launch(OzPlan& p, const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap& b, const OzArgs& a,
-               cudaStream_t s) {
+// the operand's columns of the legs, from `src` if given (analyses: the legs side by side)
+OzSplit oz_split_args(const OzPlan& p, const long* d_moff, const OzLeg* legs, int nlegs, int* widest) {
+  OzSplit a{};
+  a.T = p.T, a.nh = p.nh, a.nlat = p.nlat, a.ncap = p.ncap, a.nhpad = p.nhpad;
+  a.moff = d_moff, a.xbase = p.d_xbase, a.xlen = p.xlen;
+  *widest = 0;
+  int at = 0;
+  for (int i = 0; i < nlegs; ++i) {
+    a.src[i] = legs[i].in, a.ld[i] = legs[i].ldin, a.ncols[i] = legs[i].ncols, a.coff[i] = at;
+    a.parityH[i] = legs[i].useH ? 1 : 0;
+    at += legs[i].ncols;
+    *widest = std::max(*widest, legs[i].ncols);
+  }
+  if (at > p.ncap) throw std::runtime_error("FP64 tensor-core Legendre path: too many columns");
+  return a;
+}
+void oz_gemm(OzPlan& p, const long* d_moff, int mode, const OzLeg* legs, const int* coff, int nlegs, cudaStream_t s) {
+  OzArgs a{};
+  a.mode = mode, a.T = p.T, a.nh = p.nh, a.nlat = p.nlat, a.ncap = p.ncap, a.N = mode ? p.nana : p.nsyn;
+  a.xbase = p.d_xbase, a.moff = d_moff, a.err = p.d_err;
+  for (int t = 0; t < 2; ++t) a.ea[t] = mode ? p.eg[t] : p.ex;
+  const CUtensorMap* mb[2];
+  for (int i = 0; i < 2; ++i) {
+    const OzLeg& l = legs[i < nlegs ? i : 0];
+    const int t = l.useH ? 1 : 0, at = coff[i < nlegs ? i : 0];
+    if (at < 0 || at + l.ncols > p.ncap) throw std::runtime_error("FP64 tensor-core Legendre path: too many columns");
+    a.job[i] = {t, l.ncols, at, mode ? p.eana[t] : p.esyn[t], l.out, l.ldout};
+    mb[i] = mode ? &p.m_tana[t] : &p.m_tsyn[t];
+  }
+  a.items = oz_items(p, legs, nlegs, mode, &a.nitems);
   const size_t sm = (size_t)OZ_NS * (OZ_ABYTES + (size_t)OZ_S * a.N * OZ_KC * 2) + 1024 + 128;
-  k_oz_gemm<<<std::min(a.nitems, p.nsm), OZ_THREADS, sm, s>>>(a0, a1, b, a);
+  k_oz_gemm<<<std::min(a.nitems, p.nsm), OZ_THREADS, sm, s>>>(mode ? p.m_g[0] : p.m_x, mode ? p.m_g[1] : p.m_x, *mb[0],
+                                                             *mb[1], a);
   count_launch();
   GD_LAUNCH_CHECK();
 }
@@ -675,54 +729,45 @@ void oz_free(OzPlan& p) {
   p.mem = nullptr;
 }
 
-static OzSplit oz_split_args(const OzPlan& p, const long* d_moff, const double* src, long ld, int ncols) {
-  if (ncols > p.ncap) throw std::runtime_error("FP64 tensor-core Legendre path: too many columns");
-  OzSplit a{};
-  a.T = p.T, a.nh = p.nh, a.nlat = p.nlat, a.ncols = ncols, a.ncap = p.ncap, a.nhpad = p.nhpad;
-  a.moff = d_moff, a.xbase = p.d_xbase, a.xlen = p.xlen, a.src = src, a.ld = ld;
-  return a;
-}
-static OzArgs oz_args(const OzPlan& p, const long* d_moff, bool useH, int ncols, double* out, long ld) {
-  OzArgs a{};
-  a.T = p.T, a.nh = p.nh, a.nlat = p.nlat, a.ncap = p.ncap;
-  a.xbase = p.d_xbase, a.moff = d_moff, a.parityH = useH ? 1 : 0, a.ncols = ncols;
-  a.out = out, a.ldout = ld, a.err = p.d_err;
-  return a;
-}
-
-void oz_split_x(OzPlan& p, const long* d_moff, const double* B, long ldB, int ncols, cudaStream_t s) {
-  if (ncols <= 0) return;
-  OzSplit a = oz_split_args(p, d_moff, B, ldB, ncols);
-  a.out[0] = (uint16_t*)p.x;
-  a.ex[0] = p.ex;
-  k_oz_split<0><<<dim3(p.T, (ncols + 31) / 32), 256, 0, s>>>(a);
+void oz_synth(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s) {
+  if (a.ncols <= 0) return;
+  // both tables read the same columns: one split serves them
+  const long off = b ? b->in - a.in : 0;
+  if (b && (b->ldin != a.ldin || off < 0 || off + b->ncols > a.ncols)) {
+    oz_synth(p, d_moff, a, nullptr, s);
+    oz_synth(p, d_moff, *b, nullptr, s);
+    return;
+  }
+  int n = 0;
+  OzSplit sp = oz_split_args(p, d_moff, &a, 1, &n);
+  sp.out[0] = (uint16_t*)p.x;
+  sp.ex[0] = p.ex;
+  k_oz_split<0><<<dim3(p.T, (n + 31) / 32), 256, 0, s>>>(sp);
   count_launch();
   GD_LAUNCH_CHECK();
+  const OzLeg legs[2] = {a, b ? *b : a};
+  const int coff[2] = {0, (int)off};
+  oz_gemm(p, d_moff, 0, legs, coff, b && b->ncols > 0 ? 2 : 1, s);
 }
 
-void oz_synth(OzPlan& p, const long* d_moff, bool useH, int coff, int ncols, double* F, long ldF, cudaStream_t s) {
-  if (ncols <= 0) return;
-  if (coff < 0 || coff + ncols > p.ncap) throw std::runtime_error("FP64 tensor-core Legendre path: too many columns");
-  OzArgs a = oz_args(p, d_moff, useH, ncols, F, ldF);
-  a.items = oz_items(p, ncols, 0, &a.nitems);
-  a.N = p.nsyn, a.coff = coff, a.ea[0] = a.ea[1] = p.ex, a.eb = p.esyn[useH ? 1 : 0];
-  oz_launch(p, p.m_x, p.m_x, p.m_tsyn[useH ? 1 : 0], a, s);
-}
-
-void oz_anal(OzPlan& p, const long* d_moff, bool useH, const double* G, long ldG, int ncols, double* A, long ldA,
-             cudaStream_t s) {
-  if (ncols <= 0) return;
-  OzSplit sp = oz_split_args(p, d_moff, G, ldG, ncols);
-  sp.parityH = useH ? 1 : 0;
+void oz_anal(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s) {
+  if (b && b->ncols <= 0) b = nullptr;
+  if (a.ncols <= 0) return;
+  if (b && a.ncols + b->ncols > p.ncap) {
+    oz_anal(p, d_moff, a, nullptr, s);
+    oz_anal(p, d_moff, *b, nullptr, s);
+    return;
+  }
+  const OzLeg legs[2] = {a, b ? *b : a};
+  const int nl = b ? 2 : 1;
+  int n = 0;
+  OzSplit sp = oz_split_args(p, d_moff, legs, nl, &n);
   for (int t = 0; t < 2; ++t) sp.out[t] = (uint16_t*)p.g[t], sp.ex[t] = p.eg[t];
-  k_oz_split<1><<<dim3(p.T, (ncols + 31) / 32), 256, 0, s>>>(sp);
+  k_oz_split<1><<<dim3(p.T, (n + 31) / 32, nl), 256, 0, s>>>(sp);
   count_launch();
   GD_LAUNCH_CHECK();
-  OzArgs a = oz_args(p, d_moff, useH, ncols, A, ldA);
-  a.mode = 1;
-  a.items = oz_items(p, ncols, 1, &a.nitems);
-  a.N = p.nana, a.ea[0] = p.eg[0], a.ea[1] = p.eg[1], a.eb = p.eana[useH ? 1 : 0];
-  oz_launch(p, p.m_g[0], p.m_g[1], p.m_tana[useH ? 1 : 0], a, s);
+  const int coff[2] = {0, a.ncols};
+  oz_gemm(p, d_moff, 1, legs, coff, nl, s);
 }
 
 int oz_check(OzPlan& p, cudaStream_t s) {

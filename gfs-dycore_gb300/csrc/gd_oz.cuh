@@ -33,9 +33,9 @@ struct OzPlan {
   // binary exponents of the rows
   int *esyn[2] = {nullptr, nullptr}, *eana[2] = {nullptr, nullptr}, *ex = nullptr, *eg[2] = {nullptr, nullptr};
   CUtensorMap m_tsyn[2], m_tana[2], m_x, m_g[2];
-  // work lists by column tiles and direction (0 synthesis, 1 analysis)
+  // work lists by the legs' column tiles and the direction (0 synthesis, 1 analysis)
   struct Items {
-    int ct, mode, n;
+    int ct[2], mode, n;
     int4* d;
   };
   std::vector<Items> items;
@@ -49,13 +49,18 @@ struct OzPlan {
 bool oz_init(OzPlan& p, int T, int nh, int nlat, int ncap, size_t limit, const long* d_moff, const long* d_toff,
              const double* P, const double* H, cudaStream_t s);
 void oz_free(OzPlan& p);
-// the columns [0, ncols) of B [nlm][ldB] into the synthesis operand
-void oz_split_x(OzPlan& p, const long* d_moff, const double* B, long ldB, int ncols, cudaStream_t s);
-// F[m][j][c] (orders m >= 1) = Legendre synthesis of the split columns [coff, coff + ncols)
-void oz_synth(OzPlan& p, const long* d_moff, bool useH, int coff, int ncols, double* F, long ldF, cudaStream_t s);
-// A[idx][c] (orders m >= 1) = Legendre analysis of G[m][j][c], columns [0, ncols)
-void oz_anal(OzPlan& p, const long* d_moff, bool useH, const double* G, long ldG, int ncols, double* A, long ldA,
-             cudaStream_t s);
+// Legendre transform of `ncols` real columns through the P or the dP/dphi table, orders m >= 1
+struct OzLeg {
+  bool useH;
+  const double* in;
+  long ldin;
+  int ncols;
+  double* out;
+  long ldout;
+};
+// syntheses F[m][j][c] of B[nlm][c], analyses A[nlm][c] of G[m][j][c]: one or two legs in a launch
+void oz_synth(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s);
+void oz_anal(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s);
 // returns and clears the device error flag (nonzero: a bounded wait gave up)
 int oz_check(OzPlan& p, cudaStream_t s);
 
