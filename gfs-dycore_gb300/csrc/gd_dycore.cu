@@ -262,6 +262,7 @@ class Dycore : public DycoreBase {
     int ncr;
     R* out;
     long ldout;
+    TcLeg tc() const { return TcLeg{useH, (const float*)in, ldin, ncr, (float*)out, ldout}; }
     OzLeg oz() const { return OzLeg{useH, (const double*)in, ldin, ncr, (double*)out, ldout}; }
     Order0<R> order0() const { return Order0<R>{in, ldin, out, ldout, ncr / 2, useH ? 1 : 0, nullptr}; }
   };
@@ -283,6 +284,13 @@ class Dycore : public DycoreBase {
     for (int i = 0; i < (b ? 2 : 1); ++i)
       if (take_tail(c[i], &t[nt])) ++nt;
     if (nt) synth_tail(t, nt);
+    if constexpr (std::is_same<R, float>::value) {
+      if (tcp) {  // both tables in one launch
+        const TcLeg t2[2] = {c[0].tc(), c[1].tc()};
+        tc_synth(*tcp, moff, t2, b ? 2 : 1, nlm_rows, stream);
+        return;
+      }
+    }
     synth_orders(c[0]);
     if (b) synth_orders(c[1]);
   }
@@ -319,27 +327,33 @@ class Dycore : public DycoreBase {
         return;
       }
     }
-    for (const Leg* l : {&a, b}) {
-      if (!l) continue;
-      Leg c = *l;
+    Leg c[2] = {a, b ? *b : a};
+    for (int i = 0; i < (b ? 2 : 1); ++i) {
       TailJob t;
-      if (take_tail(c, &t)) anal_tail(t);
-      anal_orders(c);
+      if (take_tail(c[i], &t)) anal_tail(t);
     }
+    if constexpr (std::is_same<R, float>::value) {
+      if (tcp) {
+        const TcLeg t2[2] = {c[0].tc(), c[1].tc()};
+        tc_anal(*tcp, moff, t2, b ? 2 : 1, stream);
+        return;
+      }
+    }
+    anal_orders(c[0]);
+    if (b) anal_orders(c[1]);
   }
   void synth_orders(const Leg& a) {
     if (!tcp) {
       launch_synth<R>(sd, a.useH, *a.plan, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
       return;
     }
-    if constexpr (std::is_same<R, float>::value) {
-      tc_synth(*tcp, moff, a.useH, a.in, a.ldin, nlm_rows, a.ncr, a.out, a.ldout, stream);
-    } else {
+    if constexpr (std::is_same<R, double>::value) {
       // FP64 state: the GEMM of orders m >= 1 reads an FP32 copy of the
       // spectral columns and writes FP32 Fourier rows, widened after it
       // (the eddy FFT reads the FP32 rows where the GEMM left them)
       launch_convert2d<double, float>(a.in, a.ldin, stSpec, a.ldin, nlm_rows, a.ncr, stream);
-      tc_synth(*tcp, moff, a.useH, stSpec, a.ldin, nlm_rows, a.ncr, stFour(a.out), a.ldout, stream);
+      const TcLeg t{a.useH, stSpec, a.ldin, a.ncr, stFour(a.out), a.ldout};
+      tc_synth(*tcp, moff, &t, 1, nlm_rows, stream);
       if (!eddy_)
         launch_convert2d<float, double>(stFour(a.out) + (long)nlat * a.ldout, a.ldout, a.out + (long)nlat * a.ldout,
                                         a.ldout, (long)T * nlat, a.ncr, stream);
@@ -350,16 +364,15 @@ class Dycore : public DycoreBase {
       launch_anal<R>(sd, a.useH, *a.plan, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
       return;
     }
-    if constexpr (std::is_same<R, float>::value) {
-      tc_anal(*tcp, moff, a.useH, a.in, a.ldin, a.ncr, a.out, a.ldout, stream);
-    } else {
+    if constexpr (std::is_same<R, double>::value) {
       // FP64 state: FP32 copy of every Fourier row (order 0 included, so the
       // GEMM reads no stale staging), FP32 result rows of orders m >= 1
       // (spectral rows T+1.. in the m-major order) widened after it
       // (the eddy FFT already wrote the FP32 rows, with zeros for order 0)
       if (!eddy_)
         launch_convert2d<double, float>(a.in, a.ldin, stFour(a.in), a.ldin, (long)(T + 1) * nlat, a.ncr, stream);
-      tc_anal(*tcp, moff, a.useH, stFour(a.in), a.ldin, a.ncr, stSpec, a.ldout, stream);
+      const TcLeg t{a.useH, stFour(a.in), a.ldin, a.ncr, stSpec, a.ldout};
+      tc_anal(*tcp, moff, &t, 1, stream);
       // the analysis GEMM's K segments are added here in FP64
       launch_sumconvert(stSpec + (long)(T + 1) * a.ldout, a.ldout, (long)nlm * a.ldout, tc_anal_segments(*tcp),
                         a.out + (long)(T + 1) * a.ldout, a.ldout, (long)nlm - (T + 1), a.ncr, stream);

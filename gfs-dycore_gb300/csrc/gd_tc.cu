@@ -222,6 +222,13 @@ struct TcArgs {
   // the segment; segment q writes its FP32 partial sums at out + q * seg_stride
   int nseg;
   long seg_stride;
+  // fused kernel only: the second table's leg (items with job 1): its columns
+  // and rows; the first leg's are above
+  struct Leg {
+    int parityH, ncols;
+    float* out;
+    long ldout;
+  } second;
 };
 
 template <int KIND>
@@ -386,6 +393,7 @@ struct TcItem {
   int m, c0, n0, nk0, nk1, kp, K;
   long xb;
   int kb, seg;  // first K chunk of both parities, K segment (analysis with nseg > 1)
+  int job;      // 1: the second leg's item
 };
 __device__ __forceinline__ TcItem tc_item(const TcArgs& a, int idx) {
   const int4 it = a.items[idx];
@@ -407,9 +415,10 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs& a, int idx) {
   }
   t.kb = 0;
   t.seg = 0;
+  t.job = it.w >> 16;
   if (a.mode == 1 && a.nseg > 1) {  // segment it.w of the latitude chunks (nseg <= chunks)
     const int nk = t.nk0;
-    t.seg = it.w;
+    t.seg = it.w & 0xffff;
     t.kb = t.seg * nk / a.nseg;
     t.nk0 = t.nk1 = (t.seg + 1) * nk / a.nseg - t.kb;
   }
@@ -421,14 +430,13 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs& a, int idx) {
 // store a whole tile, and with row products and range tests at every element
 // their instructions took longer than the tile's MMAs (T254L64, the largest
 // synthesis GEMM 207 -> 162 us; 112 -> 72 million instructions).
-__device__ __forceinline__ void tc_store16(const TcArgs& a, const TcItem& t, float* out, int g, int c, const float* e,
-                                           const float* o) {
-  const long ld = a.ldout;
+__device__ __forceinline__ void tc_store16(const TcArgs& a, const TcItem& t, float* out, long ld, int parityH, int g,
+                                           int c, const float* e, const float* o) {
   if (a.mode == 0) {
     const int j = t.n0 + g, n = a.nh - j;
     float* const pn = out + ((long)t.m * a.nlat + j) * ld + c;
     float* const ps = out + ((long)t.m * a.nlat + (a.nlat - 1 - j)) * ld + c;
-    const float sg = a.parityH ? -1.f : 1.f;
+    const float sg = parityH ? -1.f : 1.f;
     if (n >= 16) {
 #pragma unroll
       for (int q = 0; q < 16; ++q) {
@@ -598,7 +606,7 @@ __global__ void __launch_bounds__(TCP_THREADS, 1)
         else
 #pragma unroll
           for (int q = 0; q < 16; ++q) o[q] = 0.f;
-        if (c < a.ncols) tc_store16(a, t, a.out, g, c, e, o);
+        if (c < a.ncols) tc_store16(a, t, a.out, a.ldout, a.parityH, g, c, e, o);
       }
       tc_fence_before();
       __syncwarp();
@@ -643,9 +651,12 @@ __device__ __forceinline__ void mma_tf32_ta(uint32_t dtmem, uint32_t atmem, uint
       "r"(atmem), "l"(b), "r"(idesc), "r"(acc));
 }
 
+// tensor maps of both legs: raw operand, table hi and lo
+struct TcfMaps {
+  CUtensorMap raw[2], bh[2], bl[2];
+};
 __global__ void __launch_bounds__(TCF_THREADS, 1)
-    k_tc_gemm_f(const __grid_constant__ CUtensorMap mRaw, const __grid_constant__ CUtensorMap mBh,
-                const __grid_constant__ CUtensorMap mBl, TcArgs a, int nitems, int ns, uint32_t raw_bytes) {
+    k_tc_gemm_f(const __grid_constant__ TcfMaps mp, TcArgs a, int nitems, int ns, uint32_t raw_bytes) {
   const int na = a.na;  // A slots (2 <= na <= min(ns, TCF_MAXA))
   extern __shared__ __align__(1024) unsigned char smraw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~(uintptr_t)1023);
@@ -717,21 +728,22 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
         unsigned char* st = sm + (size_t)s * stage_bytes;
         const uint32_t fb = smem_u32(&full[s]);
         mbar_expect_tx(fb, 2 * tab_bytes + raw_bytes);
+        const CUtensorMap *mRaw = &mp.raw[t.job], *mBh = &mp.bh[t.job], *mBl = &mp.bl[t.job];
         if (a.mode == 0) {
           const int xt = acc * a.kepad + kk * kc;
-          tma_3d(smem_u32(st), &mBh, xt, t.n0, t.m, fb);
-          tma_3d(smem_u32(st + tab_bytes), &mBl, xt, t.n0, t.m, fb);
+          tma_3d(smem_u32(st), mBh, xt, t.n0, t.m, fb);
+          tma_3d(smem_u32(st + tab_bytes), mBl, xt, t.n0, t.m, fb);
           // degrees q = acc + 2 (kk kc + i) of order m: spectral rows moff[m] + q,
           // addressed as (row pair, parity slot)
           const long r0 = a.moff[t.m] + acc + 2L * kk * kc;
-          tma_3d(smem_u32(st + raw_off), &mRaw, t.c0, (int)(r0 & 1), (int)(r0 >> 1), fb);
+          tma_3d(smem_u32(st + raw_off), mRaw, t.c0, (int)(r0 & 1), (int)(r0 >> 1), fb);
         } else {
           const int x = kk * kc;
           const int yt = acc * a.kirows + t.n0;
-          tma_3d(smem_u32(st), &mBh, x, yt, t.m, fb);
-          tma_3d(smem_u32(st + tab_bytes), &mBl, x, yt, t.m, fb);
-          tma_3d(smem_u32(st + raw_off), &mRaw, t.c0, x, t.m, fb);
-          tma_3d(smem_u32(st + raw_off + raw_bytes / 2), &mRaw, t.c0, a.nlat - x - kc, t.m, fb);
+          tma_3d(smem_u32(st), mBh, x, yt, t.m, fb);
+          tma_3d(smem_u32(st + tab_bytes), mBl, x, yt, t.m, fb);
+          tma_3d(smem_u32(st + raw_off), mRaw, t.c0, x, t.m, fb);
+          tma_3d(smem_u32(st + raw_off + raw_bytes / 2), mRaw, t.c0, a.nlat - x - kc, t.m, fb);
         }
         ++fills[s];
         rs.next(ns);
@@ -832,7 +844,7 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
           nv = q0 < t.K ? (t.K - q0 + 1) / 2 : 0;
         } else {
           nv = a.nh - kk * kc;
-          plus = (acc == 0) != (a.parityH != 0);
+          plus = (acc == 0) != ((t.job ? a.second.parityH : a.parityH) != 0);
         }
         // convert before waiting for the A slot: the loads and the split
         // overlap the MMAs still reading it
@@ -932,6 +944,9 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
         ++titem;
       }
       const int c = t.c0 + q4 * 32 + lane;
+      const int ncols = t.job ? a.second.ncols : a.ncols, parityH = t.job ? a.second.parityH : a.parityH;
+      const long ldout = t.job ? a.second.ldout : a.ldout;
+      float* const out = (t.job ? a.second.out : a.out) + (long)t.seg * a.seg_stride;
       for (int g = 0; g < N; g += 16) {
         float e[16], o[16];
         uint32_t re[16], ro[16];
@@ -960,7 +975,7 @@ __global__ void __launch_bounds__(TCF_THREADS, 1)
 #pragma unroll
           for (int q = 0; q < 16; ++q) e[q] = __uint_as_float(re[q]), o[q] = __uint_as_float(ro[q]);
         }
-        if (c < a.ncols) tc_store16(a, t, a.out + (long)t.seg * a.seg_stride, g, c, e, o);
+        if (c < ncols) tc_store16(a, t, out, ldout, parityH, g, c, e, o);
       }
       if (bt >= 0) {
         tc_fence_before();
@@ -1257,8 +1272,8 @@ static bool fused_ok(const TcPlan& p, const void* base, long ld) {
          ((uintptr_t)base % 16) == 0 && ld % 4 == 0;
 }
 
-static void launch_fused(const TcPlan& p, const CUtensorMap& raw, const CUtensorMap& bh, const CUtensorMap& bl,
-                         TcArgs& args, int nitems, uint32_t raw_bytes, cudaStream_t s) {
+static void launch_fused(const TcPlan& p, const TcfMaps& maps, TcArgs& args, int nitems, uint32_t raw_bytes,
+                         cudaStream_t s) {
   const uint32_t stage = (uint32_t)round_up(2 * args.N * 128 + (int)raw_bytes, 1024);
   const size_t avail = 227 * 1024 - 1024 - 256;
   // TMA ring depth: as many stages as shared memory holds (at most
@@ -1284,51 +1299,81 @@ static void launch_fused(const TcPlan& p, const CUtensorMap& raw, const CUtensor
     attr = true;
   }
   const int grid = std::min(nitems, p.nsm);
-  k_tc_gemm_f<<<grid, TCF_THREADS, sm, s>>>(raw, bh, bl, args, nitems, ns, raw_bytes);
+  k_tc_gemm_f<<<grid, TCF_THREADS, sm, s>>>(maps, args, nitems, ns, raw_bytes);
   count_launch();
   GD_LAUNCH_CHECK();
 }
 
-void tc_synth(TcPlan& p, const long* d_moff, bool useH, const float* B, long ldB, long nrowsB, int ncols, float* F,
-              long ldF, cudaStream_t s) {
-  if (ncols > p.ncap) throw std::runtime_error("tc_synth: too many columns");
-  const long nlm = (long)(p.T + 1) * (p.T + 2) / 2;
-  if (fused_ok(p, B, ldB) && 2 * (nrowsB / 2) >= nlm) {
-    const int ct = (ncols + TC_M - 1) / TC_M, nt = (p.nh + p.nsyn - 1) / p.nsyn;
-    std::vector<int4> it;
-    for (int m = 1; m <= p.T; ++m)  // order 0 (zonal means) runs on the IEEE SIMT path
-      for (int a = 0; a < ct; ++a)
-        for (int b2 = 0; b2 < nt; ++b2) it.push_back(make_int4(m, a, b2, 0));
-    if (it.empty()) return;
-    TcArgs args{};
-    args.items = cached_items(p, ((long)ncols << 2) | 0, it);
-    args.mode = 0;
-    args.T = p.T;
-    args.nh = p.nh;
-    args.nlat = p.nlat;
-    args.N = p.nsyn;
-    args.kc = p.kc;
-    args.kepad = p.kepad;
-    args.kirows = p.kirows;
-    args.xbase = p.d_xbase;
-    args.moff = d_moff;
-    args.parityH = useH ? 1 : 0;
-    args.ncols = ncols;
-    args.coff = 0;
-    args.out = F;
-    args.ldout = ldF;
-    args.err = p.d_err;
-    args.idesc = make_idesc(p.kind, p.nsyn);
-    // spectral rows viewed as (column, parity slot, row pair): a chunk is one
-    // parity slot of kc consecutive pairs
-    const uint64_t dims[3] = {(uint64_t)ncols, 2, (uint64_t)(nrowsB / 2)};
-    const uint64_t strides[2] = {(uint64_t)ldB * 4, (uint64_t)ldB * 8};
-    const uint32_t box[3] = {TC_M, 1, (uint32_t)p.kc};
-    const CUtensorMap& raw = cached_raw_map(p, B, dims, strides, box);
-    const int t = useH ? 1 : 0;
-    launch_fused(p, raw, p.m_tsyn[t][0], p.m_tsyn[t][1], args, (int)it.size(), (uint32_t)(p.kc * TC_M * 4), s);
-    return;
+// the legs' common arguments of the fused kernel
+static TcArgs fused_args(const TcPlan& p, const long* d_moff, int mode, const TcLeg* legs, int n) {
+  TcArgs args{};
+  args.mode = mode;
+  args.T = p.T;
+  args.nh = p.nh;
+  args.nlat = p.nlat;
+  args.N = mode ? p.nana : p.nsyn;
+  args.kc = p.kc;
+  args.kepad = p.kepad;
+  args.kirows = p.kirows;
+  args.xbase = p.d_xbase;
+  args.moff = d_moff;
+  args.parityH = legs[0].useH ? 1 : 0;
+  args.ncols = legs[0].ncols;
+  args.out = legs[0].out;
+  args.ldout = legs[0].ldout;
+  const TcLeg& l = legs[n - 1];
+  args.second = {l.useH ? 1 : 0, l.ncols, l.out, l.ldout};
+  args.err = p.d_err;
+  args.idesc = make_idesc(p.kind, args.N);
+  return args;
+}
+static TcfMaps fused_maps(TcPlan& p, const TcLeg* legs, int n, int mode, long nrowsB) {
+  TcfMaps m;
+  for (int i = 0; i < 2; ++i) {
+    const TcLeg& l = legs[std::min(i, n - 1)];
+    const int t = l.useH ? 1 : 0;
+    if (mode == 0) {
+      // spectral rows viewed as (column, parity slot, row pair): a chunk is one
+      // parity slot of kc consecutive pairs
+      const uint64_t dims[3] = {(uint64_t)l.ncols, 2, (uint64_t)(nrowsB / 2)};
+      const uint64_t strides[2] = {(uint64_t)l.ldin * 4, (uint64_t)l.ldin * 8};
+      const uint32_t box[3] = {TC_M, 1, (uint32_t)p.kc};
+      m.raw[i] = cached_raw_map(p, l.in, dims, strides, box);
+    } else {
+      // Fourier rows [m][lat][column]: a chunk is kc northern latitudes plus
+      // the kc mirrored southern ones
+      const uint64_t dims[3] = {(uint64_t)l.ncols, (uint64_t)p.nlat, (uint64_t)p.T + 1};
+      const uint64_t strides[2] = {(uint64_t)l.ldin * 4, (uint64_t)l.ldin * 4 * p.nlat};
+      const uint32_t box[3] = {TC_M, (uint32_t)p.kc, 1};
+      m.raw[i] = cached_raw_map(p, l.in, dims, strides, box);
+    }
+    m.bh[i] = mode ? p.m_tana[t][0] : p.m_tsyn[t][0];
+    m.bl[i] = mode ? p.m_tana[t][1] : p.m_tsyn[t][1];
   }
+  return m;
+}
+// orders m >= 1 (order 0, the zonal means, runs in IEEE arithmetic), both legs' tiles of an order side by side
+static const int4* fused_items(TcPlan& p, const TcLeg* legs, int n, int mode, int nseg, int* nitems) {
+  const long key = 1L << 62 | (long)(n > 1 ? legs[1].ncols : 0) << 36 | (long)legs[0].ncols << 12 | nseg << 2 | mode;
+  std::vector<int4> it;
+  const int N = mode ? p.nana : p.nsyn;
+  for (int m = 1; m <= p.T; ++m) {
+    const int rows = mode ? (p.T - m + 2) / 2 : p.nh;
+    for (int i = 0; i < n; ++i)
+      for (int a = 0; a < (legs[i].ncols + TC_M - 1) / TC_M; ++a)
+        for (int b = 0; b < (rows + N - 1) / N; ++b)
+          for (int q = 0; q < nseg; ++q) it.push_back(make_int4(m, a, b, i << 16 | q));
+  }
+  *nitems = (int)it.size();
+  return it.empty() ? nullptr : cached_items(p, key, it);
+}
+
+static void synth_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaStream_t s) {
+  const bool useH = leg.useH;
+  const float* B = leg.in;
+  float* F = leg.out;
+  const long ldB = leg.ldin, ldF = leg.ldout;
+  const int ncols = leg.ncols;
   // 1) split the spectral columns into the padded K-major staging
   if (!p.d_xmap) {
     std::vector<long> hm(p.T + 2);
@@ -1391,55 +1436,36 @@ void tc_synth(TcPlan& p, const long* d_moff, bool useH, const float* B, long ldB
                          (int)it.size(), s);
 }
 
+void tc_synth(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, long nrowsB, cudaStream_t s) {
+  if (n > 1 && legs[1].ncols <= 0) n = 1;
+  if (legs[0].ncols <= 0) return;
+  const long nlm = (long)(p.T + 1) * (p.T + 2) / 2;
+  bool fused = 2 * (nrowsB / 2) >= nlm;
+  for (int i = 0; i < n; ++i) {
+    if (legs[i].ncols > p.ncap) throw std::runtime_error("tc_synth: too many columns");
+    fused = fused && fused_ok(p, legs[i].in, legs[i].ldin);
+  }
+  if (!fused) {
+    for (int i = 0; i < n; ++i) synth_unfused(p, d_moff, legs[i], s);
+    return;
+  }
+  TcArgs args = fused_args(p, d_moff, 0, legs, n);
+  int nitems = 0;
+  args.items = fused_items(p, legs, n, 0, 1, &nitems);
+  if (nitems == 0) return;
+  launch_fused(p, fused_maps(p, legs, n, 0, nrowsB), args, nitems, (uint32_t)(p.kc * TC_M * 4), s);
+}
+
 int tc_anal_segments(const TcPlan& p) {  // K segments of the latitude sum: at most one per chunk
   return std::max(1, std::min(p.aseg, (p.nh + p.kc - 1) / p.kc));
 }
 
-void tc_anal(TcPlan& p, const long* d_moff, bool useH, const float* G, long ldG, int ncols, float* A, long ldA,
-             cudaStream_t s) {
-  if (ncols > p.ncap) throw std::runtime_error("tc_anal: too many columns");
-  if (fused_ok(p, G, ldG)) {
-    const int ct = (ncols + TC_M - 1) / TC_M;
-    std::vector<int4> it;
-    const int nseg = tc_anal_segments(p);
-    for (int m = 1; m <= p.T; ++m) {  // order 0 runs on the IEEE SIMT path
-      const int ke = (p.T - m + 2) / 2;
-      for (int a = 0; a < ct; ++a)
-        for (int b2 = 0; b2 < (ke + p.nana - 1) / p.nana; ++b2)
-          for (int q = 0; q < nseg; ++q) it.push_back(make_int4(m, a, b2, q));
-    }
-    if (it.empty()) return;
-    TcArgs args{};
-    args.items = cached_items(p, ((long)ncols << 8) | ((long)nseg << 2) | 1, it);
-    args.nseg = nseg;
-    args.seg_stride = (long)(p.T + 1) * (p.T + 2) / 2 * ldA;
-    args.mode = 1;
-    args.T = p.T;
-    args.nh = p.nh;
-    args.nlat = p.nlat;
-    args.N = p.nana;
-    args.kc = p.kc;
-    args.kepad = p.kepad;
-    args.kirows = p.kirows;
-    args.xbase = p.d_xbase;
-    args.moff = d_moff;
-    args.parityH = useH ? 1 : 0;
-    args.ncols = ncols;
-    args.coff = 0;
-    args.out = A;
-    args.ldout = ldA;
-    args.err = p.d_err;
-    args.idesc = make_idesc(p.kind, p.nana);
-    // Fourier rows [m][lat][column]: a chunk is kc northern latitudes plus
-    // the kc mirrored southern ones
-    const uint64_t dims[3] = {(uint64_t)ncols, (uint64_t)p.nlat, (uint64_t)p.T + 1};
-    const uint64_t strides[2] = {(uint64_t)ldG * 4, (uint64_t)ldG * 4 * p.nlat};
-    const uint32_t box[3] = {TC_M, (uint32_t)p.kc, 1};
-    const CUtensorMap& raw = cached_raw_map(p, G, dims, strides, box);
-    const int t = useH ? 1 : 0;
-    launch_fused(p, raw, p.m_tana[t][0], p.m_tana[t][1], args, (int)it.size(), (uint32_t)(2 * p.kc * TC_M * 4), s);
-    return;
-  }
+static void anal_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaStream_t s) {
+  const bool useH = leg.useH;
+  const float* G = leg.in;
+  float* A = leg.out;
+  const long ldG = leg.ldin, ldA = leg.ldout;
+  const int ncols = leg.ncols;
   dim3 g((unsigned)((p.nhpad + 31) / 32), (unsigned)((ncols + 31) / 32), (unsigned)(p.T + 1)), b(32, 8);
   if (p.kind == TC_TF32)
     k_tc_split_g<TC_TF32><<<g, b, 0, s>>>(G, ldG, ncols, p.nh, p.nlat, p.nhpad, p.ncap, (uint32_t*)p.gp[0],
@@ -1487,6 +1513,32 @@ void tc_anal(TcPlan& p, const long* d_moff, bool useH, const float* G, long ldG,
     launch_gemm<TC_TF32>(p, e0[0], e0[1], e1[0], e1[1], p.m_tana[t][0], p.m_tana[t][1], args, (int)it.size(), s);
   else
     launch_gemm<TC_BF16>(p, e0[0], e0[1], e1[0], e1[1], p.m_tana[t][0], p.m_tana[t][1], args, (int)it.size(), s);
+}
+
+void tc_anal(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, cudaStream_t s) {
+  if (n > 1 && legs[1].ncols <= 0) n = 1;
+  if (legs[0].ncols <= 0) return;
+  bool fused = true;
+  for (int i = 0; i < n; ++i) {
+    if (legs[i].ncols > p.ncap) throw std::runtime_error("tc_anal: too many columns");
+    fused = fused && fused_ok(p, legs[i].in, legs[i].ldin);
+  }
+  const int nseg = tc_anal_segments(p);
+  if (!fused || (n > 1 && nseg > 1)) {  // the segments' partial sums have one stride
+    for (int i = 0; i < n; ++i)
+      if (fused)
+        tc_anal(p, d_moff, legs + i, 1, s);
+      else
+        anal_unfused(p, d_moff, legs[i], s);
+    return;
+  }
+  TcArgs args = fused_args(p, d_moff, 1, legs, n);
+  int nitems = 0;
+  args.items = fused_items(p, legs, n, 1, nseg, &nitems);
+  if (nitems == 0) return;
+  args.nseg = nseg;
+  args.seg_stride = (long)(p.T + 1) * (p.T + 2) / 2 * legs[0].ldout;
+  launch_fused(p, fused_maps(p, legs, n, 1, 0), args, nitems, (uint32_t)(2 * p.kc * TC_M * 4), s);
 }
 
 int tc_check(TcPlan& p, cudaStream_t s) {
