@@ -778,27 +778,35 @@ int gd_mlp_init(int nin, int nhidden, int nlayers, int nout, unsigned long long 
     GD_CUDA(cudaStreamCreateWithFlags(&p->own, cudaStreamNonBlocking));
     p->stream = p->own;
     GD_CUDA(cudaMallocHost(&p->hres, sizeof(float) * 2));
-    p->p32 = (float*)p->alloc(sizeof(float) * off);
-    p->w16 = (__nv_bfloat16*)p->alloc(sizeof(__nv_bfloat16) * off);
-    p->grad = (float*)p->alloc(sizeof(float) * off);
-    p->am = (float*)p->alloc(sizeof(float) * off);
-    p->av = (float*)p->alloc(sizeof(float) * off);
-    p->partial = (float*)p->alloc(sizeof(float) * KPART);
     long wmax = 0;
     for (int l = 0; l < p->nlayer; ++l) wmax = std::max(wmax, (long)p->fin[l] * p->fout[l]);
-    p->kpart = (float*)p->alloc(sizeof(float) * KSPLIT * wmax);
-    p->lossd = (float*)p->alloc(sizeof(float));
-    p->in_mu = (float*)p->alloc(sizeof(float) * nin);
-    p->in_sd = (float*)p->alloc(sizeof(float) * nin);
-    p->out_mu = (float*)p->alloc(sizeof(float) * nout);
-    p->out_sd = (float*)p->alloc(sizeof(float) * nout);
+    // one allocation: the sizes first, then the addresses
+    char* base = nullptr;
+    size_t used = 0;
+    auto take = [&](auto** q, size_t n) {
+      *q = reinterpret_cast<std::remove_reference_t<decltype(*q)>>(base ? base + used : nullptr);
+      used += (n * sizeof(**q) + 255) / 256 * 256;
+    };
+    auto carve = [&]() {
+      for (float** q : {&p->p32, &p->grad, &p->am, &p->av}) take(q, off);
+      take(&p->w16, off);
+      take(&p->partial, KPART);
+      take(&p->kpart, KSPLIT * wmax);
+      take(&p->lossd, 1);
+      for (float** q : {&p->in_mu, &p->in_sd}) take(q, nin);
+      for (float** q : {&p->out_mu, &p->out_sd}) take(q, nout);
+      if (!p->tc) return;
+      take(&p->wpf, (size_t)p->rowsf * p->kpf);
+      if (p->rowsb > 0) take(&p->wpb, (size_t)p->rowsb * p->kpb);
+      take(&p->terr, 1);
+    };
+    carve();
+    base = (char*)p->alloc(used);
+    used = 0;
+    carve();
     if (p->tc) {
-      p->wpf = (__nv_bfloat16*)p->alloc(sizeof(__nv_bfloat16) * (size_t)p->rowsf * p->kpf);
       tc_chain_map(&p->mapf, p->wpf, p->kpf, p->rowsf);
-      if (p->rowsb > 0) {
-        p->wpb = (__nv_bfloat16*)p->alloc(sizeof(__nv_bfloat16) * (size_t)p->rowsb * p->kpb);
-        tc_chain_map(&p->mapb, p->wpb, p->kpb, p->rowsb);
-      }
+      if (p->rowsb > 0) tc_chain_map(&p->mapb, p->wpb, p->kpb, p->rowsb);
       p->pack = to_device(p.get(), pack);
       std::vector<TcChainLayer> inf;
       for (int l = 0; l < p->nlayer; ++l) {
@@ -808,7 +816,6 @@ int gd_mlp_init(int nin, int nhidden, int nlayers, int nout, unsigned long long 
         inf.push_back(L);
       }
       p->inf_layers = to_device(p.get(), inf);
-      p->terr = (int*)p->alloc(sizeof(int));
       GD_CUDA(cudaMemset(p->terr, 0, sizeof(int)));
       GD_CUDA(cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, p->device));
     }
