@@ -252,8 +252,8 @@ class Dycore : public DycoreBase {
     launch_r2c<R>(sd, plan, grid, GP, ldP, GH, ldH, stream);
   }
   // One Legendre transform of an array: its columns through a table.  The
-  // split modes run order 0 on the IEEE path ahead of the tensor-core GEMMs of
-  // orders m >= 1, both tables' order 0 in one launch.
+  // tensor-core paths run order 0 in IEEE arithmetic ahead of the GEMMs of orders
+  // m >= 1, both tables' order 0 in one launch.
   struct Leg {
     bool useH;
     const GemmPlan* plan;  // all-orders SIMT work list (null on the tensor-core paths)

@@ -1,6 +1,6 @@
 """The plain FP64 Legendre GEMMs on the tensor cores (operands split into exact
 8-bit digits) at the edges of their tiles: latitude and degree counts around
-the 16-column step and the 64-column tile, contractions around the 32-deep
+the 16-column step and the 32-column tile, contractions around the 32-deep
 chunk and the 128-deep segment, columns around the 128-column tile, orders
 with a single degree; columns of very different size side by side; infinities
 and NaN.  Against the FP64 oracle at the plain path's 1e-12 of each field's
