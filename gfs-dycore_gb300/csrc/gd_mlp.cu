@@ -119,10 +119,25 @@ struct gd_mlp {
   std::vector<void*> allocs;
   void* alloc(size_t bytes) {
     void* p = nullptr;
-    GD_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
+    const cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 16));
+    if (e != cudaSuccess) cudaGetLastError();  // the caller may try a smaller batch: no later launch check is to see it
+    GD_CUDA(e);
     allocs.push_back(p);
     return p;
   }
+  // Gives back what was allocated since it was made, unless kept: a growth of
+  // the net's buffers that fails leaves the net as it was.
+  struct Growth {
+    gd_mlp* p;
+    size_t n;
+    bool kept = false;
+    explicit Growth(gd_mlp* q) : p(q), n(q->allocs.size()) {}
+    ~Growth() {
+      if (kept) return;
+      cudaStreamSynchronize(p->stream);
+      for (; p->allocs.size() > n; p->allocs.pop_back()) cudaFree(p->allocs.back());
+    }
+  };
   ~gd_mlp() {
     int cur = 0;
     if (cudaGetDevice(&cur) == cudaSuccess && cur != device) cudaSetDevice(device);
@@ -472,15 +487,23 @@ void pack_weights(gd_mlp* p) {
 // (activations stay on chip), the activations on the SIMT path.  Old buffers
 // are kept until the net is destroyed: a context's captured step may still
 // address them.
-void act_reserve(gd_mlp* p, int ncols) {
-  if (ncols <= p->bcap) return;
+struct Acts {
+  int cap;
+  float *zb, *ab;
+};
+Acts act_buffers(gd_mlp* p, int ncols) {
+  if (ncols <= p->bcap) return Acts{p->bcap, p->zb, p->ab};
   GD_CUDA(cudaStreamSynchronize(p->stream));
-  p->zb = (float*)p->alloc(sizeof(float) * (size_t)p->nl * ncols * p->nh);
-  p->ab = (float*)p->alloc(sizeof(float) * (size_t)p->nl * ncols * p->nh);
-  p->bcap = ncols;
+  const size_t bytes = sizeof(float) * (size_t)p->nl * ncols * p->nh;
+  float* zb = (float*)p->alloc(bytes);
+  return Acts{ncols, zb, (float*)p->alloc(bytes)};
 }
+void act_set(gd_mlp* p, const Acts& a) { p->bcap = a.cap, p->zb = a.zb, p->ab = a.ab; }
 void mlp_reserve(gd_mlp* p, int ncols) {
-  if (!p->tc) act_reserve(p, ncols);
+  if (p->tc) return;
+  gd_mlp::Growth g(p);
+  act_set(p, act_buffers(p, ncols));
+  g.kept = true;
 }
 
 namespace {
@@ -494,42 +517,47 @@ X* to_device(gd_mlp* p, const std::vector<X>& h) {
 }  // namespace
 
 // Training buffers for batches of up to ncols columns, and on the tensor
-// cores the layer tables over them.
+// cores the layer tables over them: all of them first, then the net takes them
+// over together, since a batch within the capacity uses every one.
 void train_reserve(gd_mlp* p, int ncols) {
   if (ncols <= p->tcap) return;
   if (p->tcb && p->nin > 256)
     throw std::invalid_argument("gd_mlp: training on the tensor cores takes at most 256 inputs");
-  act_reserve(p, ncols);
+  gd_mlp::Growth grown(p);
+  const Acts a = act_buffers(p, ncols);
   GD_CUDA(cudaStreamSynchronize(p->stream));
-  const int cap = p->bcap;
-  p->yb = (float*)p->alloc(sizeof(float) * (size_t)cap * p->nout);
-  p->gy = (float*)p->alloc(sizeof(float) * (size_t)cap * p->nout);
-  p->tcap = cap;
+  const int cap = a.cap;
+  float* yb = (float*)p->alloc(sizeof(float) * (size_t)cap * p->nout);
+  float* gy = (float*)p->alloc(sizeof(float) * (size_t)cap * p->nout);
   if (!p->tcb) {
     const long w = std::max(p->nh, std::max(p->nin, p->nout));
-    p->g0 = (float*)p->alloc(sizeof(float) * (size_t)cap * w);
-    p->g1 = (float*)p->alloc(sizeof(float) * (size_t)cap * w);
+    float* g0 = (float*)p->alloc(sizeof(float) * (size_t)cap * w);
+    float* g1 = (float*)p->alloc(sizeof(float) * (size_t)cap * w);
+    act_set(p, a);
+    p->yb = yb, p->gy = gy, p->g0 = g0, p->g1 = g1;
+    p->tcap = cap;
+    grown.kept = true;
     return;
   }
   const size_t act = (size_t)cap * p->nh;
-  p->dzb = (float*)p->alloc(sizeof(float) * (size_t)p->nl * act);
+  float* dzb = (float*)p->alloc(sizeof(float) * (size_t)p->nl * act);
   std::vector<TcChainLayer> f, b;
   for (int l = 0; l < p->nlayer; ++l) {
     TcChainLayer L{};
     L.N = p->fout[l], L.K = p->fin[l], L.wrow = p->wrowf[l], L.bias = p->p32 + p->offb[l];
-    if (l < p->nl) L.act = 1, L.z = p->zb + l * act, L.out = p->ab + l * act, L.ldz = p->nh;
+    if (l < p->nl) L.act = 1, L.z = a.zb + l * act, L.out = a.ab + l * act, L.ldz = p->nh;
     f.push_back(L);
   }
   for (int l = p->nlayer - 1; l >= 1; --l) {  // dZ_{l-1} = (dZ_l W_l) GELU'(Z_{l-1})
     TcChainLayer L{};
     L.N = p->fin[l], L.K = p->fout[l], L.wrow = p->wrowb[l], L.act = 2;
-    L.zin = p->zb + (l - 1) * act, L.out = p->dzb + (l - 1) * act, L.ldz = p->nh;
+    L.zin = a.zb + (l - 1) * act, L.out = dzb + (l - 1) * act, L.ldz = p->nh;
     b.push_back(L);
   }
-  p->trn_layers = to_device(p, f);
-  p->bwd_layers = to_device(p, b);
+  TcChainLayer* trn_layers = to_device(p, f);
+  TcChainLayer* bwd_layers = to_device(p, b);
   // weight gradients: stacked transposed operands over a slab of the batch
-  const int cols = std::min((cap + 31) / 32 * 32, kSlab);
+  const int cols = std::max(p->opcols, std::min((cap + 31) / 32 * 32, kSlab));
   long ar = 0, br = 0, po = 0;
   int bo = 0;
   std::vector<TcWgradItem> items;
@@ -542,35 +570,42 @@ void train_reserve(gd_mlp* p, int ncols) {
     lay.push_back({p->offw[l], p->offb[l], po, p->fout[l], p->fin[l], Np, bo});
     ar += Mp, br += (p->fin[l] + 63) / 64 * 64, po += (long)Mp * Np, bo += p->fout[l];
   }
+  uint32_t *zth = p->zth, *ztl = p->ztl, *ath = p->ath, *atl = p->atl;
   if (cols > p->opcols) {  // rows past a layer's outputs or inputs stay zero
     auto z = [&](size_t words) {
       uint32_t* q = (uint32_t*)p->alloc(sizeof(uint32_t) * words);
       GD_CUDA(cudaMemsetAsync(q, 0, sizeof(uint32_t) * words, p->stream));
       return q;
     };
-    p->zth = z((size_t)ar * cols), p->ztl = z((size_t)ar * cols);
-    p->ath = z((size_t)br * cols), p->atl = z((size_t)br * cols);
-    p->opcols = cols;
+    zth = z((size_t)ar * cols), ztl = z((size_t)ar * cols);
+    ath = z((size_t)br * cols), atl = z((size_t)br * cols);
     GD_CUDA(cudaStreamSynchronize(p->stream));
   }
   std::vector<TsplitJob> jobs;
   for (int l = 0; l < p->nlayer; ++l) {
-    const size_t za = (size_t)arow[l] * p->opcols, ba = (size_t)brow[l] * p->opcols;
-    jobs.push_back({l == p->nlayer - 1 ? p->gy : p->dzb + l * act, p->fout[l], lay[l].boff, p->zth + za, p->ztl + za});
-    jobs.push_back({l == 0 ? nullptr : p->ab + (l - 1) * act, p->fin[l], -1, p->ath + ba, p->atl + ba});
+    const size_t za = (size_t)arow[l] * cols, ba = (size_t)brow[l] * cols;
+    jobs.push_back({l == p->nlayer - 1 ? gy : dzb + l * act, p->fout[l], lay[l].boff, zth + za, ztl + za});
+    jobs.push_back({l == 0 ? nullptr : a.ab + (l - 1) * act, p->fin[l], -1, ath + ba, atl + ba});
   }
-  p->jobs = to_device(p, jobs);
-  p->wlay = to_device(p, lay);
-  p->nbias = bo;
-  p->wg.items = to_device(p, items);
-  p->wg.nitems = (int)items.size();
-  p->wg.pstride = po;
-  p->wg.err = p->terr;
+  TsplitJob* djobs = to_device(p, jobs);
+  WgradLayer* wlay = to_device(p, lay);
+  TcWgrad wg;
+  wg.items = to_device(p, items);
+  wg.nitems = (int)items.size();
+  wg.pstride = po;
+  wg.err = p->terr;
   const int nslab = ceil_div(cap, kSlab);
-  p->wpart = (float*)p->alloc(sizeof(float) * (size_t)nslab * std::max(1, p->nsm / p->wg.nitems) * po);
-  p->wg.part = p->wpart;
-  p->bpart = (float*)p->alloc(sizeof(float) * (size_t)ceil_div(cap, kTrows) * bo);
-  tc_wgrad_maps(p->wg, p->zth, p->ztl, p->ath, p->atl, ar, br, p->opcols);
+  wg.part = (float*)p->alloc(sizeof(float) * (size_t)nslab * std::max(1, p->nsm / wg.nitems) * po);
+  float* bpart = (float*)p->alloc(sizeof(float) * (size_t)ceil_div(cap, kTrows) * bo);
+  tc_wgrad_maps(wg, zth, ztl, ath, atl, ar, br, cols);
+  act_set(p, a);
+  p->yb = yb, p->gy = gy, p->dzb = dzb;
+  p->trn_layers = trn_layers, p->bwd_layers = bwd_layers;
+  p->zth = zth, p->ztl = ztl, p->ath = ath, p->atl = atl, p->opcols = cols;
+  p->jobs = djobs, p->wlay = wlay, p->nbias = bo;
+  p->wg = wg, p->wpart = wg.part, p->bpart = bpart;
+  p->tcap = cap;
+  grown.kept = true;
 }
 
 // y [n][nout] = net(x [n][nin]) on stream s, on the tensor cores when the

@@ -1,0 +1,55 @@
+"""What the host code does when a call of the CUDA runtime fails and the order
+in which it hands work to the device, on a runtime without a GPU
+(fake_runtime.py)."""
+import pytest
+
+import fake_runtime
+
+
+@pytest.mark.parametrize("hidden", [16, 300])  # the tensor-core and the SIMT training path
+def test_training_after_a_failed_allocation(hidden):
+    """A training batch whose buffers do not fit is refused and leaves the net as
+    it was: the next smaller batch runs on the buffers it had (or gets its own),
+    the same batch runs once there is memory."""
+    fake_runtime.run(r"""
+H, SMALL, BIG, NOUT = %d, 128, 40000, 3
+rt.fake_watch(b"k_mse", 3)  # the output gradient's buffer
+x, t = device(4 * BIG * 5), device(4 * BIG * NOUT)
+
+def net():
+    h = vp()
+    assert lib.gd_mlp_init(5, H, 2, NOUT, 1, 0, ctypes.byref(h)) == 0
+    return h
+
+def grad(h, n):
+    # status, device memory it took, where the output gradient went, kernels
+    before = rt.fake_used()
+    log()
+    rc = lib.gd_mlp_loss_grad(h, x, t, n, None, None)
+    l = log()
+    gy = [p for w, p, _, _ in l if w.startswith("launch:") and "5k_mse" in w and "final" not in w]
+    return rc, rt.fake_used() - before, gy, sum(w.startswith("launch:") for w, _, _, _ in l)
+
+h = net()
+_, small, _, n_small = grad(h, SMALL)
+lib.gd_mlp_destroy(h)
+for trained in (False, True):
+    k = 0
+    while True:
+        h = net()
+        gy0 = grad(h, SMALL)[2] if trained else None
+        rt.fake_fail(k)
+        rc, kept, gy, n = grad(h, BIG)
+        rt.fake_fail(-1)
+        if rc == 0:
+            break
+        assert rc == core.GD_ERR_CUDA and n == 0 and kept == 0, (k, rc, n, kept)
+        rc, took, gy, n = grad(h, SMALL)
+        assert rc == 0 and n == n_small, (k, rc, n)
+        assert gy == gy0 if trained else took == small, (k, took)
+        rc, took, gy, n = grad(h, BIG)
+        assert rc == 0 and took > 0 and gy != gy0, (k, rc, took)
+        lib.gd_mlp_destroy(h)
+        k += 1
+    assert k >= (6 if H > 256 else 14), k  # every buffer's allocation was made to fail
+""" % hidden)
