@@ -109,6 +109,16 @@ __device__ __forceinline__ double float_to_double(float x) {
   return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + 0x38000000u)), (int)(u << 29));
 }
 
+// Copies a host array that may go away to the device, in the order of the
+// stream whose kernels read it.  Not cudaMemcpy or cudaMemset: they run on the
+// legacy default stream and may return before the device has the bytes, and
+// the non-blocking streams used here do not wait for that stream.
+inline void upload_on(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  if (bytes == 0) return;
+  GD_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+  GD_CUDA(cudaStreamSynchronize(s));
+}
+
 // Launch accounting (reported by gd_launch_count).
 extern long long g_launches;
 inline void count_launch(int n = 1) { g_launches += n; }

@@ -511,7 +511,7 @@ void forward_simt(gd_mlp* p, const float* x, int n, float* y, cudaStream_t s);
 template <typename X>
 X* to_device(gd_mlp* p, const std::vector<X>& h) {
   X* d = (X*)p->alloc(sizeof(X) * h.size());
-  GD_CUDA(cudaMemcpy(d, h.data(), sizeof(X) * h.size(), cudaMemcpyHostToDevice));
+  upload_on(d, h.data(), sizeof(X) * h.size(), p->stream);
   return d;
 }
 }  // namespace
@@ -851,13 +851,11 @@ int gd_mlp_init(int nin, int nhidden, int nlayers, int nout, unsigned long long 
         inf.push_back(L);
       }
       p->inf_layers = to_device(p.get(), inf);
-      GD_CUDA(cudaMemset(p->terr, 0, sizeof(int)));
+      GD_CUDA(cudaMemsetAsync(p->terr, 0, sizeof(int), p->stream));
       GD_CUDA(cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, p->device));
     }
-    GD_CUDA(cudaMemcpy(p->p32, h.data(), sizeof(float) * off, cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemset(p->am, 0, sizeof(float) * off));
-    GD_CUDA(cudaMemset(p->av, 0, sizeof(float) * off));
-    GD_CUDA(cudaMemset(p->grad, 0, sizeof(float) * off));
+    upload_on(p->p32, h.data(), sizeof(float) * off, p->stream);
+    for (float* q : {p->am, p->av, p->grad}) GD_CUDA(cudaMemsetAsync(q, 0, sizeof(float) * off, p->stream));
     to_bf16(p.get());
     pack_weights(p.get());
     GD_CUDA(cudaStreamSynchronize(p->stream));
@@ -894,7 +892,7 @@ int gd_mlp_set_params(gd_mlp* p, const float* params) {
   if (!params) return GD_ERR_ARG;
   return mguard(p, [&] {
     GD_CUDA(cudaStreamSynchronize(p->stream));
-    GD_CUDA(cudaMemcpy(p->p32, params, sizeof(float) * p->np, cudaMemcpyHostToDevice));
+    upload_on(p->p32, params, sizeof(float) * p->np, p->stream);
     to_bf16(p);
     pack_weights(p);
     GD_CUDA(cudaStreamSynchronize(p->stream));
@@ -907,10 +905,10 @@ int gd_mlp_set_norm(gd_mlp* p, const float* in_mu, const float* in_sd, const flo
     for (int i = 0; i < p->nin; ++i)
       if (!(in_sd[i] > 0)) throw std::invalid_argument("gd_mlp_set_norm: input scales must be > 0");
     GD_CUDA(cudaStreamSynchronize(p->stream));
-    GD_CUDA(cudaMemcpy(p->in_mu, in_mu, sizeof(float) * p->nin, cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemcpy(p->in_sd, in_sd, sizeof(float) * p->nin, cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemcpy(p->out_mu, out_mu, sizeof(float) * p->nout, cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemcpy(p->out_sd, out_sd, sizeof(float) * p->nout, cudaMemcpyHostToDevice));
+    upload_on(p->in_mu, in_mu, sizeof(float) * p->nin, p->stream);
+    upload_on(p->in_sd, in_sd, sizeof(float) * p->nin, p->stream);
+    upload_on(p->out_mu, out_mu, sizeof(float) * p->nout, p->stream);
+    upload_on(p->out_sd, out_sd, sizeof(float) * p->nout, p->stream);
     p->has_norm = true;
   });
 }

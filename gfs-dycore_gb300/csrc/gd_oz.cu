@@ -580,7 +580,7 @@ void oz_map(CUtensorMap* m, void* base, long k, long rows, int boxrows) {
                                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) throw CudaError("cuTensorMapEncodeTiled (digits) failed: " + std::to_string((int)r));
 }
-const int4* oz_items(OzPlan& p, const OzLeg* legs, int nlegs, int mode, int* n) {
+const int4* oz_items(OzPlan& p, const OzLeg* legs, int nlegs, int mode, int* n, cudaStream_t s) {
   int ct[2] = {0, 0};
   for (int i = 0; i < nlegs; ++i) ct[i] = (legs[i].ncols + OZ_M - 1) / OZ_M;
   for (const auto& l : p.items)
@@ -598,7 +598,7 @@ const int4* oz_items(OzPlan& p, const OzLeg* legs, int nlegs, int mode, int* n) 
   OzPlan::Items l{{ct[0], ct[1]}, mode, (int)it.size(), nullptr};
   GD_CUDA(cudaMalloc(&l.d, sizeof(int4) * it.size()));
   p.items.push_back(l);
-  GD_CUDA(cudaMemcpy(l.d, it.data(), sizeof(int4) * it.size(), cudaMemcpyHostToDevice));
+  upload_on(l.d, it.data(), sizeof(int4) * it.size(), s);
   *n = l.n;
   return l.d;
 }
@@ -631,7 +631,7 @@ void oz_gemm(OzPlan& p, const long* d_moff, int mode, const OzLeg* legs, const i
     a.job[i] = {t, l.ncols, at, mode ? p.eana[t] : p.esyn[t], l.out, l.ldout};
     mb[i] = mode ? &p.m_tana[t] : &p.m_tsyn[t];
   }
-  a.items = oz_items(p, legs, nlegs, mode, &a.nitems);
+  a.items = oz_items(p, legs, nlegs, mode, &a.nitems, s);
   const size_t sm = (size_t)OZ_NS * (OZ_ABYTES + (size_t)OZ_S * a.N * OZ_KC * 2) + 1024 + 128;
   k_oz_gemm<<<std::min(a.nitems, p.nsm), OZ_THREADS, sm, s>>>(mode ? p.m_g[0] : p.m_x, mode ? p.m_g[1] : p.m_x, *mb[0],
                                                              *mb[1], a);

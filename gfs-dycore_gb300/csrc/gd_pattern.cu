@@ -357,11 +357,11 @@ int gd_pattern_init(double lscale, double delt, double tscale, double stdev, int
     mt[0] = (uint32_t)p->seed;
     for (int i = 1; i < gd::MT_N; ++i) mt[i] = 69069u * mt[i - 1];
     const int mti = gd::MT_N;
-    GD_CUDA(cudaMemcpy(p->d_mt, mt, sizeof(mt), cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemcpy(p->d_st, &mti, sizeof(int), cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemcpy(p->d_vs, p->vs.data(), sizeof(float) * nlm, cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemcpy(p->d_dego, p->dego.data(), sizeof(int2) * nlm, cudaMemcpyHostToDevice));
-    GD_CUDA(cudaMemset(p->d_spec, 0, sizeof(float2) * nlm * nfields));
+    GD_CUDA(cudaMemsetAsync(p->d_spec, 0, sizeof(float2) * nlm * nfields, p->stream));
+    gd::upload_on(p->d_mt, mt, sizeof(mt), p->stream);
+    gd::upload_on(p->d_st, &mti, sizeof(int), p->stream);
+    gd::upload_on(p->d_vs, p->vs.data(), sizeof(float) * nlm, p->stream);
+    gd::upload_on(p->d_dego, p->dego.data(), sizeof(int2) * nlm, p->stream);
   });
   if (rc != GD_OK) {
     g_pattern_init_error = p->err;

@@ -1256,12 +1256,12 @@ static void launch_gemm(const TcPlan& p, const CUtensorMap& a0h, const CUtensorM
   GD_LAUNCH_CHECK();
 }
 
-static int4* cached_items(TcPlan& p, long key, const std::vector<int4>& it) {
+static int4* cached_items(TcPlan& p, long key, const std::vector<int4>& it, cudaStream_t s) {
   for (auto& kv : p.item_cache)
     if (kv.first == key) return kv.second;
   int4* d = nullptr;
   GD_CUDA(cudaMalloc(&d, sizeof(int4) * std::max<size_t>(it.size(), 1)));
-  GD_CUDA(cudaMemcpy(d, it.data(), sizeof(int4) * it.size(), cudaMemcpyHostToDevice));
+  upload_on(d, it.data(), sizeof(int4) * it.size(), s);
   p.item_cache.push_back({key, d});
   p.allocs.push_back(d);
   return d;
@@ -1353,7 +1353,7 @@ static TcfMaps fused_maps(TcPlan& p, const TcLeg* legs, int n, int mode, long nr
   return m;
 }
 // orders m >= 1 (order 0, the zonal means, runs in IEEE arithmetic), both legs' tiles of an order side by side
-static const int4* fused_items(TcPlan& p, const TcLeg* legs, int n, int mode, int nseg, int* nitems) {
+static const int4* fused_items(TcPlan& p, const TcLeg* legs, int n, int mode, int nseg, int* nitems, cudaStream_t s) {
   const long key = 1L << 62 | (long)(n > 1 ? legs[1].ncols : 0) << 36 | (long)legs[0].ncols << 12 | nseg << 2 | mode;
   std::vector<int4> it;
   const int N = mode ? p.nana : p.nsyn;
@@ -1365,7 +1365,7 @@ static const int4* fused_items(TcPlan& p, const TcLeg* legs, int n, int mode, in
           for (int q = 0; q < nseg; ++q) it.push_back(make_int4(m, a, b, i << 16 | q));
   }
   *nitems = (int)it.size();
-  return it.empty() ? nullptr : cached_items(p, key, it);
+  return it.empty() ? nullptr : cached_items(p, key, it, s);
 }
 
 static void synth_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaStream_t s) {
@@ -1389,7 +1389,7 @@ static void synth_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaS
         }
     }
     p.d_xmap = (int*)tc_alloc(p, sizeof(int) * p.xlen);
-    GD_CUDA(cudaMemcpy(p.d_xmap, xm.data(), sizeof(int) * p.xlen, cudaMemcpyHostToDevice));
+    upload_on(p.d_xmap, xm.data(), sizeof(int) * p.xlen, s);
   }
   dim3 g((unsigned)((p.xlen + 31) / 32), (unsigned)((ncols + 31) / 32)), b(32, 8);
   if (p.kind == TC_TF32)
@@ -1406,7 +1406,7 @@ static void synth_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaS
     for (int a = 0; a < ct; ++a)
       for (int b2 = 0; b2 < nt; ++b2) it.push_back(make_int4(m, a, b2, 0));
   if (it.empty()) return;
-  int4* dit = cached_items(p, ((long)ncols << 2) | 0, it);
+  int4* dit = cached_items(p, ((long)ncols << 2) | 0, it, s);
   TcArgs args{};
   args.items = dit;
   args.mode = 0;
@@ -1451,7 +1451,7 @@ void tc_synth(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, long nrow
   }
   TcArgs args = fused_args(p, d_moff, 0, legs, n);
   int nitems = 0;
-  args.items = fused_items(p, legs, n, 0, 1, &nitems);
+  args.items = fused_items(p, legs, n, 0, 1, &nitems, s);
   if (nitems == 0) return;
   launch_fused(p, fused_maps(p, legs, n, 0, nrowsB), args, nitems, (uint32_t)(p.kc * TC_M * 4), s);
 }
@@ -1484,7 +1484,7 @@ static void anal_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaSt
       for (int b2 = 0; b2 < (ke + p.nana - 1) / p.nana; ++b2) it.push_back(make_int4(m, a, b2, 0));
   }
   if (it.empty()) return;
-  int4* dit = cached_items(p, ((long)ncols << 2) | 1, it);
+  int4* dit = cached_items(p, ((long)ncols << 2) | 1, it, s);
   TcArgs args{};
   args.items = dit;
   args.mode = 1;
@@ -1534,7 +1534,7 @@ void tc_anal(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, cudaStream
   }
   TcArgs args = fused_args(p, d_moff, 1, legs, n);
   int nitems = 0;
-  args.items = fused_items(p, legs, n, 1, nseg, &nitems);
+  args.items = fused_items(p, legs, n, 1, nseg, &nitems, s);
   if (nitems == 0) return;
   args.nseg = nseg;
   args.seg_stride = (long)(p.T + 1) * (p.T + 2) / 2 * legs[0].ldout;

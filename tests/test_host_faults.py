@@ -53,3 +53,45 @@ for trained in (False, True):
         k += 1
     assert k >= (6 if H > 256 else 14), k  # every buffer's allocation was made to fail
 """ % hidden)
+
+
+@pytest.mark.parametrize("fused", ["1", "0"])
+def test_uploads_are_ordered_with_the_kernels_that_read_them(fused):
+    """Tables and parameters are copied in the order of the stream that reads
+    them: whatever goes through the legacy default stream has completed before
+    a kernel starts on another stream, which would not wait for it."""
+    fake_runtime.run(r"""
+T, nlon, nlat, L = 21, 64, 32, 8
+ak, bk = inputs.hybrid_coords(L)
+st = inputs.hs_rest_state(T, L, seed=0)
+for mode in core.PREC:
+    p = vp()
+    assert lib.gd_pattern_init(500e3, 1200.0, 21600.0, 0.5, 1, nlon, nlat, T, 1.0, 1, 0, ctypes.byref(p)) == 0
+    assert lib.gd_pattern_start(p) == 0
+    g = core.Dycore(T, nlon, nlat, L, ak, bk, dt=1200.0, precision=mode)
+    g.set_state(st["vrt"], st["div"], st["tv"], st["lnps"])
+    assert lib.gd_set_sppt(g.h, p, 0.05, 0.1) == 0
+    g.advance(3)
+    s = np.zeros((3, g.nlm), complex)
+    g.getvrtdivspec(*g.getuv(s, s))
+    g.getgrad(g.grdtospec(g.spectogrd(s)))
+    g.close()
+for shape in ((5, 16, 2, 3), (5, 300, 2, 3)):
+    h, n = vp(), ctypes.c_longlong()
+    assert lib.gd_mlp_init(*shape, 1, 0, ctypes.byref(h)) == 0
+    lib.gd_mlp_nparams(h, ctypes.byref(n))
+    q = [ptr(np.ones(k, np.float32)) for k in (n.value, 5, 5, 3, 3)]
+    assert lib.gd_mlp_set_params(h, q[0]) == 0 and lib.gd_mlp_set_norm(h, *q[1:]) == 0
+    x, t = device(4 * 5 * 1000), device(4 * 3 * 1000)
+    assert lib.gd_mlp_train_step(h, x, t, 1000, 1e-3, None) == 0
+l = log()
+assert sum(w == "h2d" for w, _, _, _ in l) > 50
+pending = None
+for w, p, n, s in l:
+    if w in ("h2d", "memset") and s == 0:
+        pending = (w, n)
+    elif w == "sync" and s == 0:
+        pending = None
+    elif w.startswith("launch:") and s != 0:
+        assert pending is None, (pending, w)
+""", {"GD_TC_FUSED": fused})
