@@ -385,12 +385,22 @@ class Dycore : public DycoreBase {
   Leg leg_anaP(const GemmPlan& plan, int ncol) { return Leg{false, &plan, FPb, ldGP, 2 * ncol, AP, ldAP}; }
   Leg leg_anaH() { return Leg{true, &anaH, FHb, ldGH, 2 * ah.ncol, AH, ldAH}; }
   void check() override {
-    tc_status();
+    finish();
     if (closure) mlp_check(closure, stream);
   }
-  void tc_status() {
-    if ((tcp && tc_check(*tcp, stream)) || (ozp && oz_check(*ozp, stream)))
-      throw CudaError("tensor-core Legendre pipeline: a bounded wait gave up (results invalid)");
+  // The end of every entry point that hands out results: waits for the stream
+  // and raises a bounded wait of the tensor-core Legendre kernels that gave up
+  // (what the call has copied out is then invalid).  The flag comes through a
+  // page-locked word, in the stream's order, so the call's one wait covers it.
+  int* herr_ = nullptr;
+  void finish() {
+    int* const d = tcp ? tcp->d_err : ozp ? ozp->d_err : nullptr;
+    if (d) GD_CUDA(cudaMemcpyAsync(herr_, d, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    GD_CUDA(cudaStreamSynchronize(stream));
+    if (!d || *herr_ == 0) return;
+    GD_CUDA(cudaMemsetAsync(d, 0, sizeof(int), stream));
+    GD_CUDA(cudaStreamSynchronize(stream));
+    throw CudaError("tensor-core Legendre pipeline: a bounded wait gave up (results invalid)");
   }
 
   template <typename X>
@@ -476,6 +486,7 @@ class Dycore : public DycoreBase {
       release(H64keep);
       P64keep = H64keep = nullptr;
     }
+    if (tcp || ozp) GD_CUDA(cudaMallocHost(&herr_, sizeof(int)));
     GD_CUDA(cudaStreamSynchronize(stream));
   }
   ~Dycore() override {
@@ -501,6 +512,7 @@ class Dycore : public DycoreBase {
     for (auto& kv : api_plans_) free_fft_plan(kv.second);
     if (stream) cudaStreamSynchronize(stream);
     for (void* p : allocs) cudaFree(p);
+    if (herr_) cudaFreeHost(herr_);
     if (stream && own_stream) cudaStreamDestroy(stream);
   }
 
@@ -1142,7 +1154,7 @@ class Dycore : public DycoreBase {
       }
       tcp->aslots = bs;
       tc_set_nsyn(*tcp, bn);
-      tc_status();
+      finish();
     }
     GD_CUDA(cudaEventDestroy(e0));
     GD_CUDA(cudaEventDestroy(e1));
@@ -1210,7 +1222,7 @@ class Dycore : public DycoreBase {
     inverse_pass(false);
     launch_closure_in<R>(gS, sr, L, ng, nullptr, nullptr, clos_x, stream);
     GD_CUDA(cudaMemcpyAsync(x, clos_x, sizeof(float) * (size_t)ng * (3 * L + 1), cudaMemcpyDeviceToHost, stream));
-    GD_CUDA(cudaStreamSynchronize(stream));
+    finish();
   }
   // Stochastically perturbed physics: an attached pattern (gd_pattern) is
   // advanced one step at the start of every step and put on the grid with the
@@ -1498,8 +1510,7 @@ class Dycore : public DycoreBase {
     get(tv, L, sc.tv);
     if (nt > 0) get(trc, nt * L, sc.trc);
     get(lnps, 1, sc.lnps);
-    GD_CUDA(cudaStreamSynchronize(stream));
-    tc_status();
+    finish();
   }
   void spec_out(const R* src, long ld, int col, int nb, double* h, double* tmp) {
     if (!h) return;
@@ -1512,7 +1523,7 @@ class Dycore : public DycoreBase {
     if (!state_set) throw std::runtime_error("state not set (gd_set_state)");
     if (inverse_only) {
       inverse_pass(true);
-      GD_CUDA(cudaStreamSynchronize(stream));
+      finish();
       return;
     }
     dyn_pass(rkstage == 1 ? 0 : 1, true);
@@ -1525,6 +1536,7 @@ class Dycore : public DycoreBase {
     if (nt > 0) spec_out(TD[0], ldTD, tc.dtrc, nt * L, dtrc, tmp);
     spec_out(TD[0], ldTD, tc.dlnps, 1, dlnps, tmp);
     release(tmp);
+    finish();
   }
   void getphytend(double* dvrt, double* ddiv, double* dtv, double* dtrc, double* dlnps) override {
     if (!state_set) throw std::runtime_error("state not set (gd_set_state)");
@@ -1552,6 +1564,7 @@ class Dycore : public DycoreBase {
       }
       release(tmp);
       if (dlnps) memset(dlnps, 0, sizeof(double) * 2 * (size_t)nlm);
+      finish();
       return;
     }
     if (c.dcmip >= 0 || !c.heldsuarez) {  // dry DCMIP or no physics: zero tendencies
@@ -1571,6 +1584,7 @@ class Dycore : public DycoreBase {
     release(tmp);
     if (dtrc) memset(dtrc, 0, sizeof(double) * 2 * (size_t)nt * L * nlm);
     if (dlnps) memset(dlnps, 0, sizeof(double) * 2 * (size_t)nlm);
+    finish();
   }
 
   // ------------------------------------------------------ transform API --
@@ -1617,12 +1631,13 @@ class Dycore : public DycoreBase {
   }
   // the end of a transform call: every copy has completed
   void api_done() {
-    GD_CUDA(cudaStreamSynchronize(stream));
     if (xfer_cap_ > kXferKeep) {
+      GD_CUDA(cudaStreamSynchronize(stream));
       release(xfer_);
       xfer_ = nullptr;
       xfer_cap_ = 0;
     }
+    finish();
   }
   // synthesis of ncs complex columns X[nlm][ldS] to grid rows in gS
   void api_synth(const R* X, int ncs, bool needH, const FftPlan& p) {
@@ -1820,7 +1835,7 @@ class Dycore : public DycoreBase {
   double get_pdryini() override {
     double h = 0.0;
     GD_CUDA(cudaMemcpyAsync(&h, pdryini, sizeof(double), cudaMemcpyDeviceToHost, stream));
-    GD_CUDA(cudaStreamSynchronize(stream));
+    finish();
     return h;
   }
   void diag(double* out) override {
@@ -1829,7 +1844,7 @@ class Dycore : public DycoreBase {
     double h[5];
     GD_CUDA(cudaMemcpyAsync(h, diagout, 4 * sizeof(double), cudaMemcpyDeviceToHost, stream));
     GD_CUDA(cudaMemcpyAsync(h + 4, pdryini, sizeof(double), cudaMemcpyDeviceToHost, stream));
-    GD_CUDA(cudaStreamSynchronize(stream));
+    finish();
     memcpy(out, h, sizeof(h));
   }
 };

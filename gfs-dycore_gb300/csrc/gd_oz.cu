@@ -770,12 +770,4 @@ void oz_anal(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cuda
   oz_gemm(p, d_moff, 1, legs, coff, nl, s);
 }
 
-int oz_check(OzPlan& p, cudaStream_t s) {
-  int h = 0;
-  GD_CUDA(cudaMemcpyAsync(&h, p.d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  GD_CUDA(cudaStreamSynchronize(s));
-  if (h) GD_CUDA(cudaMemsetAsync(p.d_err, 0, sizeof(int), s));
-  return h;
-}
-
 }  // namespace gd

@@ -39,7 +39,7 @@ struct OzPlan {
     int4* d;
   };
   std::vector<Items> items;
-  int* d_err = nullptr;
+  int* d_err = nullptr;   // device error flag: nonzero, a bounded wait gave up
   void* mem = nullptr;  // all of the above but the work lists
 };
 
@@ -61,7 +61,5 @@ struct OzLeg {
 // syntheses F[m][j][c] of B[nlm][c], analyses A[nlm][c] of G[m][j][c]: one or two legs in a launch
 void oz_synth(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s);
 void oz_anal(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s);
-// returns and clears the device error flag (nonzero: a bounded wait gave up)
-int oz_check(OzPlan& p, cudaStream_t s);
 
 }  // namespace gd

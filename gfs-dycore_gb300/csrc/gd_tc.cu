@@ -1541,14 +1541,6 @@ void tc_anal(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, cudaStream
   launch_fused(p, fused_maps(p, legs, n, 1, 0), args, nitems, (uint32_t)(2 * p.kc * TC_M * 4), s);
 }
 
-int tc_check(TcPlan& p, cudaStream_t s) {
-  int h = 0;
-  GD_CUDA(cudaMemcpyAsync(&h, p.d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  GD_CUDA(cudaStreamSynchronize(s));
-  if (h) GD_CUDA(cudaMemsetAsync(p.d_err, 0, sizeof(int), s));
-  return h;
-}
-
 
 // ------------------------------------------------- closure network --
 // A chain of dense layers over 128 rows (grid columns of the closure) per

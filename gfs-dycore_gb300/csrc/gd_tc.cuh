@@ -66,7 +66,7 @@ struct TcPlan {
   std::vector<std::pair<long, int4*>> item_cache;  // work lists by (ncols, direction)
   std::vector<std::pair<std::array<uint64_t, 9>, CUtensorMap>> raw_maps;  // fused-path maps by geometry
   int* d_xmap = nullptr;  // padded synthesis position -> spectral index (or -1)
-  int* d_err = nullptr;   // device error flag (bounded waits)
+  int* d_err = nullptr;   // device error flag: nonzero, a bounded wait gave up
   std::vector<void*> allocs;
 };
 
@@ -102,8 +102,6 @@ void tc_synth(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, long nrow
 void tc_anal(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, cudaStream_t s);
 // the K segments tc_anal uses (the plan's aseg, at most one per latitude chunk)
 int tc_anal_segments(const TcPlan& p);
-// returns and clears the device error flag (nonzero: a bounded wait gave up)
-int tc_check(TcPlan& p, cudaStream_t s);
 
 // A chain of dense layers of the closure network on the tensor cores, one
 // launch: layer l takes the rows of the layer before it (the first x [M][ldx])

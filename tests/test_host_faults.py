@@ -95,3 +95,39 @@ for w, p, n, s in l:
     elif w.startswith("launch:") and s != 0:
         assert pending is None, (pending, w)
 """, {"GD_TC_FUSED": fused})
+
+
+@pytest.mark.parametrize("mode", ["fp64", "tf32x3", "f64_eddy"])
+def test_a_wait_that_gave_up_is_raised_by_the_call_that_ran_it(mode):
+    """A bounded wait of the tensor-core Legendre kernels that gives up leaves a
+    code in the context's error flag: every entry point that hands out results
+    raises it, once."""
+    fake_runtime.run(r"""
+T, nlon, nlat, L = 42, 128, 64, 8
+ak, bk = inputs.hybrid_coords(L)
+st = inputs.hs_rest_state(T, L, seed=0)
+log()
+g = core.Dycore(T, nlon, nlat, L, ak, bk, dt=1200.0, precision="%s")
+flag, = [p for w, p, n, _ in log() if w == "memset" and n == 4]
+g.set_state(st["vrt"], st["div"], st["tv"], st["lnps"])
+s, s1 = np.zeros((3, g.nlm), complex), np.zeros((3, g.nlm), np.complex64)
+x, x1 = np.zeros((3, nlat, nlon)), np.zeros((3, nlat, nlon), np.float32)
+feat = np.zeros((nlat * nlon, 3 * L + 1), np.float32)
+calls = dict(spectogrd=lambda: g.spectogrd(s), spectogrd_f=lambda: g.spectogrd(s1), grdtospec=lambda: g.grdtospec(x),
+             grdtospec_f=lambda: g.grdtospec(x1), getuv=lambda: g.getuv(s, s), getuv_f=lambda: g.getuv(s1, s1),
+             getvrtdivspec=lambda: g.getvrtdivspec(x, x), getvrtdivspec_f=lambda: g.getvrtdivspec(x1, x1),
+             getgrad=lambda: g.getgrad(s), getgrad_f=lambda: g.getgrad(s1), getdyntend=lambda: g.getdyntend(1),
+             getphytend=lambda: g.getphytend(), inverse=lambda: g.getdyntend(1, inverse_only=True),
+             get_state=lambda: g.get_state(), get_grid=lambda: g.get_grid("ug"), diag=lambda: g.diag(),
+             features=lambda: g._chk(lib.gd_closure_features(g.h, ptr(feat))), sync=lambda: g.sync())
+for name, f in calls.items():
+    f()
+    ctypes.memset(flag, 54, 1)
+    try:
+        f()
+    except core.GdError as e:
+        assert e.code == core.GD_ERR_CUDA and "gave up" in str(e), (name, e)
+    else:
+        raise AssertionError(name + " returned")
+    f()
+""" % mode)
