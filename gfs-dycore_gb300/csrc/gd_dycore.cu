@@ -407,6 +407,11 @@ class Dycore : public DycoreBase {
   X* dalloc(size_t n) {
     X* p = nullptr;
     cudaError_t e = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(X));
+    if (e == cudaErrorMemoryAllocation && ozp) {  // what a context must have goes before its digits
+      cudaGetLastError();
+      drop_digits();
+      e = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(X));
+    }
     if (e != cudaSuccess) throw CudaError(std::string("cudaMalloc: ") + cudaGetErrorString(e));
     allocs.push_back(p);
     return p;
@@ -436,22 +441,26 @@ class Dycore : public DycoreBase {
     ng = (long)nlon * nlat;
     GD_CUDA(cudaSetDevice(c.device));
     GD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    GD_CUDA(cudaMallocHost(&herr_, sizeof(int)));
     eddy_ = sizeof(R) == 8 && c.precision == GD_PREC_F64_EDDY && fft_eddy_supported(M);
     init_grid();
     init_vertical(ak_, bk_);
     init_buffers();
     if constexpr (std::is_same<R, double>::value) {
       if (c.precision == GD_PREC_FP64) {
-        // the digits take 4 to 8 times the FP64 tables and operands: contexts
-        // where that is more than a quarter of the device's memory (T1148 with
-        // 64 levels; GD_FP64_TC_GB sets the line, 0: none) keep the FP64 pipe
+        // The digits take half as much again as everything else of a context
+        // (T574 with 64 levels and 4 tracers: 9.9 GB beside 24.7), and only
+        // speed comes of them: at most a quarter of the device's memory, and
+        // only while half of it stays free for the contexts and programs that
+        // come later.  GD_FP64_TC_GB sets a line of its own (0: none).  Contexts
+        // without digits run on the FP64 pipe.
         size_t free_b = 0, total_b = 0;
         GD_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const int gb = env_int("GD_FP64_TC_GB", -1);
+        const size_t half = total_b / 2, room = free_b > half ? free_b - half : 0;
+        const size_t line = gb < 0 ? std::min(total_b / 4, room) : (size_t)gb << 30;
         ozp.reset(new OzPlan());
-        if (!oz_init(*ozp, T, nh, nlat, 2 * std::max(sc.ncol, ap.ncol + ah.ncol), gb < 0 ? total_b / 4 : (size_t)gb << 30, moff,
-                     toff, P, H, stream))
-          ozp.reset();
+        if (!oz_init(*ozp, T, nh, nlat, 2 * std::max(sc.ncol, ap.ncol + ah.ncol), line, moff, toff, P, H, stream)) ozp.reset();
       }
     }
     init_plans();
@@ -486,7 +495,6 @@ class Dycore : public DycoreBase {
       release(H64keep);
       P64keep = H64keep = nullptr;
     }
-    if (tcp || ozp) GD_CUDA(cudaMallocHost(&herr_, sizeof(int)));
     GD_CUDA(cudaStreamSynchronize(stream));
   }
   ~Dycore() override {
@@ -830,14 +838,27 @@ class Dycore : public DycoreBase {
     stage_items = upload(items);
   }
 
+  // the step's all-orders work lists of the SIMT Legendre kernels
+  void simt_plans() {
+    synP = make_synth_plan(T, nh, 2 * sc.ncol, stream);
+    synH = make_synth_plan(T, nh, 2 * (sc.ncol - 2 * L), stream);
+    anaP = make_anal_plan(T, 2 * ap.ncol, stream);
+    anaH = make_anal_plan(T, 2 * ah.ncol, stream);
+    anaPhys = make_anal_plan(T, 2 * (3 * L + 1), stream);
+    if (simple() || closure) anaSimple = make_anal_plan(T, 2 * (4 * L + 1), stream);
+  }
+  // gives the FP64 mode's digits back: the context goes on on the FP64 pipe.
+  // Between passes only (a pass looks at simt() as it goes).
+  void drop_digits() {
+    finish();
+    oz_free(*ozp);
+    ozp.reset();
+    drop_graph();
+    steps_done = 0;  // the captured step changes
+    simt_plans();
+  }
   void init_plans() {
-    if (simt()) {
-      synP = make_synth_plan(T, nh, 2 * sc.ncol, stream);
-      synH = make_synth_plan(T, nh, 2 * (sc.ncol - 2 * L), stream);
-      anaP = make_anal_plan(T, 2 * ap.ncol, stream);
-      anaH = make_anal_plan(T, 2 * ah.ncol, stream);
-      anaPhys = make_anal_plan(T, 2 * (3 * L + 1), stream);
-    }
+    if (simt()) simt_plans();
     const double ai = 1.0 / Phys::rerth;
     const int h0 = 2 * L;  // FH column = S column - 2L
     std::vector<SynthDesc> full = {
@@ -886,7 +907,6 @@ class Dycore : public DycoreBase {
       };
       if (c.massfix) sd_.push_back({1, 4 * L, 2 * L, 0, -1, 1.0, 0.0});
       r2cSimple = mk_r2c(sd_.data(), (int)sd_.size());
-      if (simt()) anaSimple = make_anal_plan(T, 2 * (4 * L + 1), stream);
     }
   }
 

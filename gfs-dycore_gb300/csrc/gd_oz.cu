@@ -670,13 +670,15 @@ bool oz_init(OzPlan& p, int T, int nh, int nlat, int ncap, size_t limit, const l
   };
   const long rsyn = (long)(T + 1) * nh, rg = (long)(T + 1) * p.ncap;
   const size_t dig = 2 * OZ_S;  // bytes of an operand's digits
-  const size_t ox = part(dig * p.ncap * p.xlen), oex = part(sizeof(int) * rg), oxb = part(sizeof(long) * (T + 1)),
+  // a synthesis and an analysis of a context never overlap (one stream), and
+  // each writes its operand's digits before it reads them: one place for both
+  const size_t gbytes = (dig * rg * p.nhpad + 255) / 256 * 256;
+  const size_t ox = part(std::max(dig * p.ncap * p.xlen, 2 * gbytes)), oex = part(sizeof(int) * rg), oxb = part(sizeof(long) * (T + 1)),
                oerr = part(sizeof(int));
-  size_t ots[2], ota[2], og[2], oes[2], oea[2], oeg[2];
+  size_t ots[2], ota[2], oes[2], oea[2], oeg[2];
   for (int t = 0; t < 2; ++t) {
     ots[t] = part(dig * nh * p.xlen);
     ota[t] = part(dig * p.nlm * p.nhpad);
-    og[t] = part(dig * rg * p.nhpad);
     oes[t] = part(sizeof(int) * rsyn);
     oea[t] = part(sizeof(int) * p.nlm);
     oeg[t] = part(sizeof(int) * rg);
@@ -703,7 +705,7 @@ bool oz_init(OzPlan& p, int T, int nh, int nlat, int ncap, size_t limit, const l
     const double* tab = t ? H : P;
     p.tsyn[t] = at(ots[t]);
     p.tana[t] = at(ota[t]);
-    p.g[t] = at(og[t]);
+    p.g[t] = at(ox + t * gbytes);
     p.esyn[t] = (int*)at(oes[t]);
     p.eana[t] = (int*)at(oea[t]);
     p.eg[t] = (int*)at(oeg[t]);

@@ -26,7 +26,7 @@ struct OzPlan {
   long* d_xbase = nullptr;
   // digits: synthesis tables [8][nh][xlen], analysis tables [8][nlm][nhpad] (an
   // order's even degrees, then its odd ones); operands X [8][ncap][xlen] and, per
-  // parity, G [8][(T+1) ncap][nhpad].  A tile that reaches past its own rows reads
+  // parity, G [8][(T+1) ncap][nhpad], in the same memory.  A tile that reaches past its own rows reads
   // other rows' digits into outputs that are not stored.
   void *tsyn[2] = {nullptr, nullptr}, *tana[2] = {nullptr, nullptr};
   void *x = nullptr, *g[2] = {nullptr, nullptr};

@@ -131,3 +131,67 @@ for name, f in calls.items():
         raise AssertionError(name + " returned")
     f()
 """ % mode)
+
+
+def test_digits_leave_room_for_other_contexts():
+    """The digits of the plain FP64 mode are there for speed: contexts take them
+    while half of the device stays free, and what fits without them in half of
+    the device fits with them."""
+    fake_runtime.run(r"""
+ak, bk = inputs.hybrid_coords(20)
+
+def fill(total):
+    # contexts until one does not fit: device memory each took, with digits or not
+    rt.fake_total(total)
+    out, keep = [], []
+    while True:
+        log()
+        before = rt.fake_used()
+        try:
+            keep.append(core.Dycore(42, 128, 64, 20, ak, bk, dt=1200.0))
+        except core.GdError as e:
+            assert e.code == core.GD_ERR_NOMEM
+            for g in keep:
+                g.close()
+            return out
+        out.append((rt.fake_used() - before, any("k_oz_table" in w for w, _, _, _ in log())))
+        assert not out[-1][1] or total - rt.fake_used() >= total // 2
+
+big = 1 << 30
+with_digits = fill(big)
+assert with_digits[0][1] and not with_digits[-1][1]
+plain = with_digits[-1][0]
+assert len(with_digits) >= big // 2 // plain, (len(with_digits), plain)
+""")
+
+
+def test_a_context_gives_its_digits_back_for_what_it_must_have():
+    """An allocation of a context that only fits without the context's digits
+    gets their memory; the context goes on on the FP64 pipe."""
+    fake_runtime.run(r"""
+ak, bk = inputs.hybrid_coords(20)
+st = inputs.hs_rest_state(42, 20, seed=0)
+rt.fake_total(1 << 30)
+
+def kernels(f):
+    log()
+    f()
+    l = [w for w, _, _, _ in log() if w.startswith("launch:")]
+    return any("k_oz_gemm" in w for w in l), any("k_synthI" in w or "k_analI" in w for w in l)
+
+for step in (0, 1, 3):
+    g = core.Dycore(42, 128, 64, 20, ak, bk, dt=1200.0)
+    g.set_state(st["vrt"], st["div"], st["tv"], st["lnps"])
+    g.advance(step)
+    assert kernels(g.getphytend) == (True, False)
+    used, rest = rt.fake_used(), device((1 << 30) - rt.fake_used() - 4096)
+    s = np.zeros((70, g.nlm), complex)
+    assert kernels(lambda: g.getuv(s, s)) == (False, True)
+    rt.cudaFree(rest)
+    assert rt.fake_used() < used
+    assert kernels(lambda: g.advance(1)) == (False, True)
+    assert kernels(g.getphytend) == (False, True)
+    assert kernels(lambda: g.grdtospec(np.zeros((3, 64, 128)))) == (False, True)
+    g.advance(3)
+    g.close()
+""")
