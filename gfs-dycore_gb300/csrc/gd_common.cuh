@@ -33,9 +33,11 @@ struct CudaError : std::runtime_error {
 #define GD_CUDA(call)                                                                         \
   do {                                                                                        \
     cudaError_t e_ = (call);                                                                  \
-    if (e_ != cudaSuccess)                                                                    \
+    if (e_ != cudaSuccess) {                                                                  \
+      cudaGetLastError(); /* reported here: no later launch check is to see it again */       \
       throw ::gd::CudaError(std::string(#call) + ": " + cudaGetErrorString(e_) + " @" +      \
                             __FILE__ + ":" + std::to_string(__LINE__));                      \
+    }                                                                                         \
   } while (0)
 
 #define GD_LAUNCH_CHECK() GD_CUDA(cudaGetLastError())

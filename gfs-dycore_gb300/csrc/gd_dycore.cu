@@ -412,7 +412,10 @@ class Dycore : public DycoreBase {
       drop_digits();
       e = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(X));
     }
-    if (e != cudaSuccess) throw CudaError(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      throw CudaError(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     allocs.push_back(p);
     return p;
   }

@@ -119,9 +119,7 @@ struct gd_mlp {
   std::vector<void*> allocs;
   void* alloc(size_t bytes) {
     void* p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 16));
-    if (e != cudaSuccess) cudaGetLastError();  // the caller may try a smaller batch: no later launch check is to see it
-    GD_CUDA(e);
+    GD_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
     allocs.push_back(p);
     return p;
   }

@@ -597,8 +597,8 @@ const int4* oz_items(OzPlan& p, const OzLeg* legs, int nlegs, int mode, int* n, 
   }
   OzPlan::Items l{{ct[0], ct[1]}, mode, (int)it.size(), nullptr};
   GD_CUDA(cudaMalloc(&l.d, sizeof(int4) * it.size()));
-  p.items.push_back(l);
   upload_on(l.d, it.data(), sizeof(int4) * it.size(), s);
+  p.items.push_back(l);
   *n = l.n;
   return l.d;
 }

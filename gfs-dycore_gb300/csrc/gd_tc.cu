@@ -1054,7 +1054,10 @@ static int tile_n(int n, int cap) {
 static void* tc_alloc(TcPlan& p, size_t bytes) {
   void* d = nullptr;
   cudaError_t e = cudaMalloc(&d, std::max<size_t>(bytes, 16));
-  if (e != cudaSuccess) throw CudaError(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    throw CudaError(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   p.allocs.push_back(d);
   return d;
 }

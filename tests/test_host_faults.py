@@ -195,3 +195,23 @@ for step in (0, 1, 3):
     g.advance(3)
     g.close()
 """)
+
+
+def test_a_failed_call_does_not_fail_the_next_one():
+    """An allocation that fails is reported by its own call: the same call
+    afterwards, with memory there, runs."""
+    fake_runtime.run(r"""
+ak, bk = inputs.hybrid_coords(8)
+for mode in ("fp64", "fp32", "tf32x3"):
+    for k in range(8):
+        g = core.Dycore(21, 64, 32, 8, ak, bk, dt=1200.0, precision=mode)
+        s = np.zeros((3, g.nlm), complex)
+        rt.fake_fail(k)
+        try:
+            g.getuv(s, s)
+        except core.GdError as e:
+            assert e.code == core.GD_ERR_CUDA
+        rt.fake_fail(-1)
+        g.getuv(s, s)
+        g.close()
+""")
