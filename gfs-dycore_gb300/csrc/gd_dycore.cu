@@ -433,6 +433,15 @@ class Dycore : public DycoreBase {
   static long pad2(long ncol) { return 2 * ((ncol + 1) / 2 * 2); }  // reals, even complex count
 
   Dycore(const gd_config& cfg, const double* ak_, const double* bk_) : c(cfg) {
+    try {
+      init(ak_, bk_);
+    } catch (...) {  // the destructor does not run
+      destroy();
+      throw;
+    }
+  }
+  ~Dycore() override { destroy(); }
+  void init(const double* ak_, const double* bk_) {
     T = c.ntrunc;
     nlon = c.nlon;
     nlat = c.nlat;
@@ -500,7 +509,7 @@ class Dycore : public DycoreBase {
     }
     GD_CUDA(cudaStreamSynchronize(stream));
   }
-  ~Dycore() override {
+  void destroy() {
     if (gexec) cudaGraphExecDestroy(gexec);
     if (gstep) cudaGraphDestroy(gstep);
     if (tcp) tc_free(*tcp);

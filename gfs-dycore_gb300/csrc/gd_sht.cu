@@ -1833,8 +1833,10 @@ static FftPlan make_plan(const D* descs, int ndesc, cudaStream_t s, int M) {
   FftPlan p;
   p.njobs = (int)jobs.size();
   if (p.njobs == 0) return p;
-  GD_CUDA(cudaMalloc(&p.jobs, sizeof(int2) * jobs.size()));
-  GD_CUDA(cudaMalloc(&p.descs, sizeof(D) * ndesc));
+  // one allocation: the jobs, then the descriptors
+  const size_t at = (sizeof(int2) * jobs.size() + 255) / 256 * 256;
+  GD_CUDA(cudaMalloc(&p.jobs, at + sizeof(D) * ndesc));
+  p.descs = (char*)p.jobs + at;
   GD_CUDA(cudaMemcpyAsync(p.jobs, jobs.data(), sizeof(int2) * jobs.size(), cudaMemcpyHostToDevice, s));
   GD_CUDA(cudaMemcpyAsync(p.descs, descs, sizeof(D) * ndesc, cudaMemcpyHostToDevice, s));
   GD_CUDA(cudaStreamSynchronize(s));
@@ -1855,7 +1857,6 @@ template FftPlan make_r2c_plan<float>(const AnalDesc*, int, cudaStream_t, int);
 
 void free_fft_plan(FftPlan& p) {
   if (p.jobs) cudaFree(p.jobs);
-  if (p.descs) cudaFree(p.descs);
   p.jobs = nullptr;
   p.descs = nullptr;
   p.njobs = 0;

@@ -215,3 +215,29 @@ for mode in ("fp64", "fp32", "tf32x3"):
         g.getuv(s, s)
         g.close()
 """)
+
+
+def test_a_context_that_cannot_be_made_leaves_nothing():
+    """Whichever allocation of gd_init fails, all memory taken before it is given back."""
+    fake_runtime.run(r"""
+ak, bk = inputs.hybrid_coords(8)
+for mode in core.PREC:
+    for T, nlon, nlat in ((21, 64, 32), (42, 128, 64)):
+        k = 0
+        while True:
+            rt.fake_fail(k)
+            try:
+                g = core.Dycore(T, nlon, nlat, 8, ak, bk, dt=1200.0, precision=mode)
+            except core.GdError:
+                assert rt.fake_used() == 0, (mode, k, rt.fake_used())
+            else:
+                failed = any(w == "nomem" for w, _, _, _ in log())  # the digits are the one optional allocation
+                g.close()
+                assert rt.fake_used() == 0
+                if not failed:
+                    break
+            rt.fake_fail(-1)
+            k += 1
+        rt.fake_fail(-1)
+        assert k > 50
+""")
