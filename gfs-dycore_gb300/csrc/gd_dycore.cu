@@ -1897,21 +1897,26 @@ static std::string g_init_error;
 template <typename F>
 static int guarded(gd_ctx* ctx, F f) {
   if (!ctx || !ctx->d) return GD_ERR_ARG;
+  // A call that fails half way waits for what it has started: copies from or to
+  // the caller's page-locked arrays may be in flight, and the caller may free
+  // the arrays or use them again.
+  auto failed = [&](const std::exception& e, int code) {
+    ctx->err = e.what();
+    cudaStreamSynchronize(ctx->d->stream);
+    cudaGetLastError();
+    return code;
+  };
   try {
     f();
     return GD_OK;
   } catch (const gd::CudaError& e) {
-    ctx->err = e.what();
-    return GD_ERR_CUDA;
+    return failed(e, GD_ERR_CUDA);
   } catch (const std::invalid_argument& e) {
-    ctx->err = e.what();
-    return GD_ERR_ARG;
+    return failed(e, GD_ERR_ARG);
   } catch (const std::runtime_error& e) {
-    ctx->err = e.what();
-    return GD_ERR_STATE;
+    return failed(e, GD_ERR_STATE);
   } catch (const std::exception& e) {
-    ctx->err = e.what();
-    return GD_ERR_CUDA;
+    return failed(e, GD_ERR_CUDA);
   }
 }
 

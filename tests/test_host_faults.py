@@ -241,3 +241,28 @@ for mode in core.PREC:
         rt.fake_fail(-1)
         assert k > 50
 """)
+
+
+def test_a_call_that_fails_leaves_no_copy_in_flight():
+    """A transform in several chunks that fails in one of them has waited for the
+    copies of the chunks before it when it returns."""
+    fake_runtime.run(r"""
+ak, bk = inputs.hybrid_coords(8)
+for mode in ("fp64", "fp32", "tf32x3"):
+    for k in range(12):
+        g = core.Dycore(21, 64, 32, 8, ak, bk, dt=1200.0, precision=mode)
+        s, x = np.zeros((50, g.nlm), complex), np.zeros((50, 32, 64))
+        for f in (lambda: g.getuv(s, s), lambda: g.getvrtdivspec(x, x)):
+            log()
+            rt.fake_fail(k)
+            try:
+                f()
+            except core.GdError:
+                pass
+            rt.fake_fail(-1)
+            l = log()
+            copies = [i for i, (w, _, n, _) in enumerate(l) if w in ("h2d", "d2h")]
+            stream = l[copies[-1]][3] if copies else 0
+            assert not copies or ("sync", 0, 0, stream) in l[copies[-1]:], (mode, k, l[copies[-1]:])
+        g.close()
+""")
