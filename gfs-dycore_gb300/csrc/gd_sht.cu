@@ -1926,7 +1926,8 @@ template void launch_r2c<float>(const ShtDev<float>&, const FftPlan&, const floa
 // FP64 zonal mean of every (grid row, latitude) a r2c plan reads, in a fixed
 // summation order: one warp per row takes lane-strided partial sums, then the
 // first warp adds every row's 32, four lanes a row, and divides by nlon with
-// one corrected multiplication by its reciprocal.  The job list is the FP32
+// its reciprocal: the product corrected by its remainder, which is the correctly
+// rounded quotient (Markstein 1990).  The job list is the FP32
 // four-step plan's: NR = 8 rows per job.  Bound by the FP64 adds: a butterfly
 // and a division per row cost more than the row's own sum (analysis FFT phase of an
 // eddy step T254L64 3.21 -> 2.75 ms, T126L64 1.02 -> 0.78 ms).
@@ -1956,8 +1957,9 @@ __global__ void __launch_bounds__(32 * NR) k_rowmean(const int2* __restrict__ jo
   const unsigned live = nr == 8 ? 0xffffffffu : (1u << (4 * nr)) - 1u;
   s += __shfl_xor_sync(live, s, 1);
   s += __shfl_xor_sync(live, s, 2);
-  const double q = s * inv;
-  if ((lane & 3) == 0) rmean[(row0 + r) * nlat + j] = fma(fma(-(double)nlon, q, s), inv, q);
+  double q = s * inv;
+  if (isfinite(q)) q = fma(fma(-(double)nlon, q, s), inv, q);  // the remainder of an infinite sum is not a number
+  if ((lane & 3) == 0) rmean[(row0 + r) * nlat + j] = q;
 }
 
 bool fft_eddy_supported(int M) { return four_step_len(M) && !getenv("GD_FFT_STOCKHAM"); }
