@@ -390,16 +390,14 @@ class Dycore : public DycoreBase {
   }
   // The end of every entry point that hands out results: waits for the stream
   // and raises a bounded wait of the tensor-core Legendre kernels that gave up
-  // (what the call has copied out is then invalid).  The flag comes through a
-  // page-locked word, in the stream's order, so the call's one wait covers it.
+  // (what the call has copied out is then invalid).  The flag is page-locked host
+  // memory, which only a kernel that gives up writes: a copy of a device flag
+  // would cost each call 8 us (a T42 transform of one field 80 -> 87 us).
   int* herr_ = nullptr;
   void finish() {
-    int* const d = tcp ? tcp->d_err : ozp ? ozp->d_err : nullptr;
-    if (d) GD_CUDA(cudaMemcpyAsync(herr_, d, sizeof(int), cudaMemcpyDeviceToHost, stream));
     GD_CUDA(cudaStreamSynchronize(stream));
-    if (!d || *herr_ == 0) return;
-    GD_CUDA(cudaMemsetAsync(d, 0, sizeof(int), stream));
-    GD_CUDA(cudaStreamSynchronize(stream));
+    if (*(volatile int*)herr_ == 0) return;
+    *herr_ = 0;
     throw CudaError("tensor-core Legendre pipeline: a bounded wait gave up (results invalid)");
   }
 
@@ -454,6 +452,7 @@ class Dycore : public DycoreBase {
     GD_CUDA(cudaSetDevice(c.device));
     GD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     GD_CUDA(cudaMallocHost(&herr_, sizeof(int)));
+    *herr_ = 0;
     eddy_ = sizeof(R) == 8 && c.precision == GD_PREC_F64_EDDY && fft_eddy_supported(M);
     init_grid();
     init_vertical(ak_, bk_);
@@ -472,12 +471,14 @@ class Dycore : public DycoreBase {
         const size_t half = total_b / 2, room = free_b > half ? free_b - half : 0;
         const size_t line = gb < 0 ? std::min(total_b / 4, room) : (size_t)gb << 30;
         ozp.reset(new OzPlan());
+        ozp->err = herr_;
         if (!oz_init(*ozp, T, nh, nlat, 2 * std::max(sc.ncol, ap.ncol + ah.ncol), line, moff, toff, P, H, stream)) ozp.reset();
       }
     }
     init_plans();
     if (split_mode()) {
       tcp.reset(new TcPlan());
+      tcp->err = herr_;
       // widest N tile at init (GD_TC_TILE_CAP: a tuning and measurement knob)
       tcp->tile_cap = std::max(16, env_int("GD_TC_TILE_CAP", tcp->tile_cap) / 16 * 16);
       const int ncap = 2 * std::max(sc.ncol, ap.ncol);

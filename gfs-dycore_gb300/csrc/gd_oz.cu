@@ -621,7 +621,7 @@ OzSplit oz_split_args(const OzPlan& p, const long* d_moff, const OzLeg* legs, in
 void oz_gemm(OzPlan& p, const long* d_moff, int mode, const OzLeg* legs, const int* coff, int nlegs, cudaStream_t s) {
   OzArgs a{};
   a.mode = mode, a.T = p.T, a.nh = p.nh, a.nlat = p.nlat, a.ncap = p.ncap, a.N = mode ? p.nana : p.nsyn;
-  a.xbase = p.d_xbase, a.moff = d_moff, a.err = p.d_err;
+  a.xbase = p.d_xbase, a.moff = d_moff, a.err = p.err;
   for (int t = 0; t < 2; ++t) a.ea[t] = mode ? p.eg[t] : p.ex;
   const CUtensorMap* mb[2];
   for (int i = 0; i < 2; ++i) {
@@ -673,8 +673,7 @@ bool oz_init(OzPlan& p, int T, int nh, int nlat, int ncap, size_t limit, const l
   // a synthesis and an analysis of a context never overlap (one stream), and
   // each writes its operand's digits before it reads them: one place for both
   const size_t gbytes = (dig * rg * p.nhpad + 255) / 256 * 256;
-  const size_t ox = part(std::max(dig * p.ncap * p.xlen, 2 * gbytes)), oex = part(sizeof(int) * rg), oxb = part(sizeof(long) * (T + 1)),
-               oerr = part(sizeof(int));
+  const size_t ox = part(std::max(dig * p.ncap * p.xlen, 2 * gbytes)), oex = part(sizeof(int) * rg), oxb = part(sizeof(long) * (T + 1));
   size_t ots[2], ota[2], oes[2], oea[2], oeg[2];
   for (int t = 0; t < 2; ++t) {
     ots[t] = part(dig * nh * p.xlen);
@@ -696,10 +695,8 @@ bool oz_init(OzPlan& p, int T, int nh, int nlat, int ncap, size_t limit, const l
   p.x = at(ox);
   p.ex = (int*)at(oex);
   p.d_xbase = (long*)at(oxb);
-  p.d_err = (int*)at(oerr);
   GD_CUDA(cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   GD_CUDA(cudaMemcpyAsync(p.d_xbase, xb.data(), sizeof(long) * (T + 1), cudaMemcpyHostToDevice, s));
-  GD_CUDA(cudaMemsetAsync(p.d_err, 0, sizeof(int), s));
   oz_map(&p.m_x, p.x, p.xlen, p.ncap, OZ_M);
   for (int t = 0; t < 2; ++t) {
     const double* tab = t ? H : P;

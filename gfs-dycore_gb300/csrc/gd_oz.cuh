@@ -39,7 +39,9 @@ struct OzPlan {
     int4* d;
   };
   std::vector<Items> items;
-  int* d_err = nullptr;   // device error flag: nonzero, a bounded wait gave up
+  // error flag, nonzero: a bounded wait gave up.  Page-locked host memory of the
+  // caller's, set before init; kernels write it in that case alone
+  int* err = nullptr;
   void* mem = nullptr;  // all of the above but the work lists
 };
 

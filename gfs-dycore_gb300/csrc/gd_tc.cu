@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const bool ok = mbar_wait(smem_u32(done), 0, a.err, 4);
   tc_fence_after();
   // warp-uniform decision: tcgen05.ld is a .sync.aligned warp instruction
-  const bool go = __all_sync(0xffffffffu, ok && *(volatile int*)a.err == 0);
+  const bool go = __all_sync(0xffffffffu, ok);
   if (go) {
     const int c = c0 + warp * 32 + lane;
     const uint32_t tw = tbase + ((uint32_t)(warp * 32) << 16);
@@ -1173,8 +1173,6 @@ void tc_init(TcPlan& p, int kind, int T, int nh, int nlat, int ncap, const long*
   }
   p.d_xbase = (long*)tc_alloc(p, sizeof(long) * (T + 1));
   GD_CUDA(cudaMemcpyAsync(p.d_xbase, p.xbase.data(), sizeof(long) * (T + 1), cudaMemcpyHostToDevice, s));
-  p.d_err = (int*)tc_alloc(p, sizeof(int));
-  GD_CUDA(cudaMemsetAsync(p.d_err, 0, sizeof(int), s));
   // tensor maps
   for (int t = 0; t < 2; ++t)
     for (int h = 0; h < 2; ++h) {
@@ -1326,7 +1324,7 @@ static TcArgs fused_args(const TcPlan& p, const long* d_moff, int mode, const Tc
   args.ldout = legs[0].ldout;
   const TcLeg& l = legs[n - 1];
   args.second = {l.useH ? 1 : 0, l.ncols, l.out, l.ldout};
-  args.err = p.d_err;
+  args.err = p.err;
   args.idesc = make_idesc(p.kind, args.N);
   return args;
 }
@@ -1427,7 +1425,7 @@ static void synth_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaS
   args.coff = 0;
   args.out = F;
   args.ldout = ldF;
-  args.err = p.d_err;
+  args.err = p.err;
   args.idesc = make_idesc(p.kind, p.nsyn);
   args.tmem_cols = tmem_cols_for(p.nsyn);
   const int t = useH ? 1 : 0;
@@ -1505,7 +1503,7 @@ static void anal_unfused(TcPlan& p, const long* d_moff, const TcLeg& leg, cudaSt
   args.coff = 0;
   args.out = A;
   args.ldout = ldA;
-  args.err = p.d_err;
+  args.err = p.err;
   args.idesc = make_idesc(p.kind, p.nana);
   args.tmem_cols = tmem_cols_for(p.nana);
   const int t = useH ? 1 : 0;

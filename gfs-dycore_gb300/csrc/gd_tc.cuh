@@ -66,7 +66,9 @@ struct TcPlan {
   std::vector<std::pair<long, int4*>> item_cache;  // work lists by (ncols, direction)
   std::vector<std::pair<std::array<uint64_t, 9>, CUtensorMap>> raw_maps;  // fused-path maps by geometry
   int* d_xmap = nullptr;  // padded synthesis position -> spectral index (or -1)
-  int* d_err = nullptr;   // device error flag: nonzero, a bounded wait gave up
+  // error flag, nonzero: a bounded wait gave up.  Page-locked host memory of the
+  // caller's, set before init; kernels write it in that case alone
+  int* err = nullptr;
   std::vector<void*> allocs;
 };
 

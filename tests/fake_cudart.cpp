@@ -84,6 +84,7 @@ cudaError_t cudaFree(void* p) {
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
   *p = calloc(1, n);
+  put("hostalloc", *p, n, nullptr);
   return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaHostAlloc(p, n, 0); }
