@@ -57,21 +57,7 @@ struct SimpleConst {
   static constexpr double pbltop = 85000., pblconst = 10000., T00 = 288.0, u0 = 35.0;
   static constexpr double pi = 3.14159265358979323846, a = 6371220.0, omega = 7.29212e-5;
 };
-
-// quotients; by the short reciprocal in the FP64 state
-__device__ __forceinline__ float quot(float a, float b) { return a / b; }
-__device__ __forceinline__ double quot(double a, double b) { return a * crcp(b); }
-// (1 / x)^(2/7), the Exner factor of x = p / p0, FP64: one step of the
-// third-order iteration y (1 + e/7 + (4/49) e^2), e = 1 - x^2 y^7, on the FP32
-// power (e below 4e-5; the next term, 0.06 e^3, is below 4e-15 e).  A dozen
-// multiply-adds in place of a quotient and a power.
-__device__ __forceinline__ double exner(double x) {
-  static_assert(SimpleConst<double>::rair * 7 == SimpleConst<double>::cpair * 2, "kappa is 2/7");
-  const double y = (double)exp2f(-2.f / 7.f * log2f((float)x));
-  const double y2 = y * y, y4 = y2 * y2, y7 = y4 * y2 * y;
-  const double e = fma(-(x * x), y7, 1.0);
-  return fma(y * e, fma(e, 4.0 / 49.0, 1.0 / 7.0), y);
-}
+static_assert(SimpleConst<double>::rair * 7 == SimpleConst<double>::cpair * 2, "exner: kappa is 2/7");
 
 }  // namespace
 
