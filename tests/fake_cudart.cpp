@@ -1,15 +1,19 @@
 // A CUDA runtime without a GPU, preloaded ahead of libcudart by the host-side
 // tests: device memory is host memory, kernels do nothing, and every call is
-// written to a log.  The n-th allocation can be made to fail, and the device's
-// free memory to be what a test wants.
+// written to a log ("absent": a copy to host pages that nothing has touched).
+// The n-th allocation can be made to fail, and the device's free memory to be
+// what a test wants.
 #include <cuda_runtime_api.h>
 #include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <map>
 #include <string>
+#include <vector>
 
 namespace {
 std::string g_log;
@@ -33,6 +37,15 @@ struct Config {
   size_t sm;
   cudaStream_t s;
 } g_conf;
+// whether some page of host memory has not been touched yet
+bool absent(const void* p, size_t n) {
+  const uintptr_t page = sysconf(_SC_PAGESIZE), lo = (uintptr_t)p / page * page;
+  std::vector<unsigned char> v(((uintptr_t)p + n - lo + page - 1) / page);
+  if (n == 0 || mincore((void*)lo, (uintptr_t)p + n - lo, v.data())) return false;
+  for (unsigned char c : v)
+    if (!(c & 1)) return true;
+  return false;
+}
 int encode_tiled(...) { return 0; }
 int ctx_current(void** c) {
   *c = (void*)0x10;
@@ -100,6 +113,7 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t st) {
   put(k == cudaMemcpyHostToDevice ? "h2d" : k == cudaMemcpyDeviceToHost ? "d2h" : "d2d",
       k == cudaMemcpyDeviceToHost ? s : d, n, st);
+  if (k == cudaMemcpyDeviceToHost && absent(d, n)) put("absent", d, n, st);
   if (k != cudaMemcpyDeviceToDevice) memcpy(d, s, n);
   return cudaSuccess;
 }

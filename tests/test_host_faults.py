@@ -266,3 +266,20 @@ for mode in ("fp64", "fp32", "tf32x3"):
             assert not copies or ("sync", 0, 0, stream) in l[copies[-1]:], (mode, k, l[copies[-1]:])
         g.close()
 """)
+
+
+def test_results_are_copied_to_pages_that_are_there():
+    """The transforms' results go to the caller's arrays in pages that the host has
+    brought into being: the device faults new pages one by one."""
+    fake_runtime.run(r"""
+ak, bk = inputs.hybrid_coords(20)
+for mode in ("fp64", "tf32x3"):
+    g = core.Dycore(42, 128, 64, 20, ak, bk, dt=1200.0, precision=mode)
+    keep = []
+    for nb in (3, 20, 65):
+        s = np.zeros((nb, g.nlm), complex)
+        log()
+        keep += [g.getgrad(s), g.getuv(s, s), g.spectogrd(s)]
+        l = log()
+        assert any(w == "d2h" for w, _, _, _ in l) and not any(w == "absent" for w, _, _, _ in l), nb
+""")
