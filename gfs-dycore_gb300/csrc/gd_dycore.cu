@@ -399,7 +399,7 @@ class Dycore : public DycoreBase {
   int* herr_ = nullptr;
   void finish() {
     GD_CUDA(cudaStreamSynchronize(stream));
-    if (*(volatile int*)herr_ == 0) return;
+    if (!herr_ || *(volatile int*)herr_ == 0) return;
     *herr_ = 0;
     throw CudaError("tensor-core Legendre pipeline: a bounded wait gave up (results invalid)");
   }
@@ -454,8 +454,10 @@ class Dycore : public DycoreBase {
     ng = (long)nlon * nlat;
     GD_CUDA(cudaSetDevice(c.device));
     GD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    GD_CUDA(cudaMallocHost(&herr_, sizeof(int)));
-    *herr_ = 0;
+    if (c.precision != GD_PREC_FP32) {  // the others use the tensor cores
+      GD_CUDA(cudaMallocHost(&herr_, sizeof(int)));
+      *herr_ = 0;
+    }
     eddy_ = sizeof(R) == 8 && c.precision == GD_PREC_F64_EDDY && fft_eddy_supported(M);
     init_grid();
     init_vertical(ak_, bk_);

@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
     const R bkt = __ldg(bk + t), bkt1 = __ldg(bk + t + 1);
     const R bp1 = bpb3;  // bk(t+1) / p(t+1)
     R rl, al, bpt;
-    if (kKeep) {
+    if constexpr (kKeep) {
       rl = rls[t * 32 + lane];
       al = als[t * 32 + lane];
       bpt = bps[t * 32 + lane];
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(32 * NWM, (sizeof(R) == 4 ? 32 : 16) / NWM)
       rl = a.rlnp_top;
       al = a.log2sp;
       if (t > 0) {
-        rl = clog(cdiv((float)pkt1, (float)pkt));
+        rl = clog(cdiv(pkt1, pkt));
         al = R(1) - (pkt * idp) * rl;
       }
     }

@@ -824,7 +824,7 @@ int gd_mlp_init(int nin, int nhidden, int nlayers, int nout, unsigned long long 
       for (float** q : {&p->p32, &p->grad, &p->am, &p->av}) take(q, off);
       take(&p->w16, off);
       take(&p->partial, KPART);
-      take(&p->kpart, KSPLIT * wmax);
+      if (!p->tcb) take(&p->kpart, KSPLIT * wmax);  // SIMT training
       take(&p->lossd, 1);
       for (float** q : {&p->in_mu, &p->in_sd}) take(q, nin);
       for (float** q : {&p->out_mu, &p->out_sd}) take(q, nout);

@@ -732,11 +732,8 @@ void oz_synth(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cud
   if (a.ncols <= 0) return;
   // both tables read the same columns: one split serves them
   const long off = b ? b->in - a.in : 0;
-  if (b && (b->ldin != a.ldin || off < 0 || off + b->ncols > a.ncols)) {
-    oz_synth(p, d_moff, a, nullptr, s);
-    oz_synth(p, d_moff, *b, nullptr, s);
-    return;
-  }
+  if (b && (b->ldin != a.ldin || off < 0 || off + b->ncols > a.ncols))
+    throw std::runtime_error("FP64 tensor-core Legendre path: legs of different arrays");
   int n = 0;
   OzSplit sp = oz_split_args(p, d_moff, &a, 1, &n);
   sp.out[0] = (uint16_t*)p.x;
@@ -752,11 +749,6 @@ void oz_synth(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cud
 void oz_anal(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s) {
   if (b && b->ncols <= 0) b = nullptr;
   if (a.ncols <= 0) return;
-  if (b && a.ncols + b->ncols > p.ncap) {
-    oz_anal(p, d_moff, a, nullptr, s);
-    oz_anal(p, d_moff, *b, nullptr, s);
-    return;
-  }
   const OzLeg legs[2] = {a, b ? *b : a};
   const int nl = b ? 2 : 1;
   int n = 0;

@@ -60,7 +60,8 @@ struct OzLeg {
   double* out;
   long ldout;
 };
-// syntheses F[m][j][c] of B[nlm][c], analyses A[nlm][c] of G[m][j][c]: one or two legs in a launch
+// syntheses F[m][j][c] of B[nlm][c], analyses A[nlm][c] of G[m][j][c]: one or two
+// legs in a launch, within the capacity; a synthesis' second leg reads columns of the first
 void oz_synth(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s);
 void oz_anal(OzPlan& p, const long* d_moff, const OzLeg& a, const OzLeg* b, cudaStream_t s);
 
