@@ -395,8 +395,10 @@ class Dycore : public DycoreBase {
   // and raises a bounded wait of the tensor-core Legendre kernels that gave up
   // (what the call has copied out is then invalid).  The flag is page-locked host
   // memory, which only a kernel that gives up writes: a copy of a device flag
-  // would cost each call 8 us (a T42 transform of one field 80 -> 87 us).
-  int* herr_ = nullptr;
+  // would cost each call 8 us (a T42 transform of one field 80 -> 87 us).  A page
+  // registered by the context costs its creation and end 20 us; cudaMallocHost
+  // took 0.3 ms of them.
+  int *herr_ = nullptr, *derr_ = nullptr;  // as the host and as the kernels see it
   void finish() {
     GD_CUDA(cudaStreamSynchronize(stream));
     if (!herr_ || *(volatile int*)herr_ == 0) return;
@@ -455,8 +457,15 @@ class Dycore : public DycoreBase {
     GD_CUDA(cudaSetDevice(c.device));
     GD_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     if (c.precision != GD_PREC_FP32) {  // the others use the tensor cores
-      GD_CUDA(cudaMallocHost(&herr_, sizeof(int)));
-      *herr_ = 0;
+      const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+      int* w = (int*)aligned_alloc(page, page);
+      if (!w) throw std::bad_alloc();
+      *w = 0;
+      const cudaError_t e = cudaHostRegister(w, page, cudaHostRegisterMapped);
+      if (e != cudaSuccess) free(w);
+      GD_CUDA(e);
+      herr_ = w;
+      GD_CUDA(cudaHostGetDevicePointer(&derr_, w, 0));
     }
     eddy_ = sizeof(R) == 8 && c.precision == GD_PREC_F64_EDDY && fft_eddy_supported(M);
     init_grid();
@@ -476,14 +485,14 @@ class Dycore : public DycoreBase {
         const size_t half = total_b / 2, room = free_b > half ? free_b - half : 0;
         const size_t line = gb < 0 ? std::min(total_b / 4, room) : (size_t)gb << 30;
         ozp.reset(new OzPlan());
-        ozp->err = herr_;
+        ozp->err = derr_;
         if (!oz_init(*ozp, T, nh, nlat, 2 * std::max(sc.ncol, ap.ncol + ah.ncol), line, moff, toff, P, H, stream)) ozp.reset();
       }
     }
     init_plans();
     if (split_mode()) {
       tcp.reset(new TcPlan());
-      tcp->err = herr_;
+      tcp->err = derr_;
       // widest N tile at init (GD_TC_TILE_CAP: a tuning and measurement knob)
       tcp->tile_cap = std::max(16, env_int("GD_TC_TILE_CAP", tcp->tile_cap) / 16 * 16);
       const int ncap = 2 * std::max(sc.ncol, ap.ncol);
@@ -538,7 +547,10 @@ class Dycore : public DycoreBase {
     for (auto& kv : api_plans_) free_fft_plan(kv.second);
     if (stream) cudaStreamSynchronize(stream);
     for (void* p : allocs) cudaFree(p);
-    if (herr_) cudaFreeHost(herr_);
+    if (herr_) {
+      cudaHostUnregister(herr_);
+      free(herr_);
+    }
     if (stream && own_stream) cudaStreamDestroy(stream);
   }
 

@@ -97,12 +97,20 @@ cudaError_t cudaFree(void* p) {
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
   *p = calloc(1, n);
-  put("hostalloc", *p, n, nullptr);
   return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaHostAlloc(p, n, 0); }
 cudaError_t cudaFreeHost(void* p) {
   free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaHostRegister(void* p, size_t n, unsigned) {
+  put("register", p, n, nullptr);
+  return cudaSuccess;
+}
+cudaError_t cudaHostUnregister(void*) { return cudaSuccess; }
+cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) {
+  *d = h;
   return cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {

@@ -10,6 +10,8 @@ from gdpy import build
 pytestmark = pytest.mark.gpu
 
 SOURCE = r"""
+#include <stdlib.h>
+#include <unistd.h>
 #include "gd_common.cuh"
 #include "gd_ptx.cuh"
 __global__ void k(int arrive, int* err) {
@@ -19,14 +21,18 @@ __global__ void k(int arrive, int* err) {
   gd::mbar_wait(gd::smem_u32(&bar), 0, err, 77);
 }
 extern "C" int run(int arrive) {
-  int* err = nullptr;
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  int *err = (int*)aligned_alloc(page, page), *derr = nullptr;
   cudaStream_t s;
-  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess || cudaMallocHost(&err, sizeof(int)) != cudaSuccess)
+  if (!err || cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaHostRegister(err, page, cudaHostRegisterMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer(&derr, err, 0) != cudaSuccess)
     return -1;
   *err = 0;
-  k<<<1, 1, 0, s>>>(arrive, err);
-  const int got = cudaStreamSynchronize(s) == cudaSuccess ? *err : -1;
-  cudaFreeHost(err);
+  k<<<1, 1, 0, s>>>(arrive, derr);
+  const int got = cudaStreamSynchronize(s) == cudaSuccess ? *(volatile int*)err : -1;
+  cudaHostUnregister(err);
+  free(err);
   cudaStreamDestroy(s);
   return got;
 }

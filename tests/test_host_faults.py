@@ -108,7 +108,7 @@ ak, bk = inputs.hybrid_coords(L)
 st = inputs.hs_rest_state(T, L, seed=0)
 log()
 g = core.Dycore(T, nlon, nlat, L, ak, bk, dt=1200.0, precision="%s")
-flag, = [p for w, p, n, _ in log() if w == "hostalloc"]
+flag, = [p for w, p, n, _ in log() if w == "register"]
 g.set_state(st["vrt"], st["div"], st["tv"], st["lnps"])
 s, s1 = np.zeros((3, g.nlm), complex), np.zeros((3, g.nlm), np.complex64)
 x, x1 = np.zeros((3, nlat, nlon)), np.zeros((3, nlat, nlon), np.float32)
