@@ -6,8 +6,10 @@
 // product).  Each operand row is scaled by a power of two to 62-bit integers
 // q = sum_b d_b 256^b, b = 0..7, with balanced digits |d_b| <= 128, exact in
 // BF16.  The products of digit pairs with b1 + b2 = g + 7 share accumulator g
-// (0..7, 36 pairs; what is dropped is below 2^-61 of the largest operands'
-// product per term, an FP64 rounding is 2^-53).  An accumulator sums at most 8
+// (0..7, 36 pairs).  What is dropped is at most 2^-57 of the product of the two
+// rows' largest entries per term (every dropped digit -128 against row maxima of
+// a power of two: 2^-57.2; digits of both signs, as operands have, 2^-60 and
+// less), an FP64 rounding of it is 2^-53.  An accumulator sums at most 8
 // x 128 products of at most 2^14 between drains, so every FP32 accumulation
 // in tensor memory is an exact integer below 2^24, and the epilogue adds the
 // eight of them as 64-bit integers and rounds once to FP64.
@@ -24,9 +26,9 @@
 //
 // One step of T126 with 64 levels and 3 tracers (1026 columns; 152 SMs): all its
 // Legendre transforms 18.8 ms on the FP64 pipe (70% of its rate), 3.92 ms here.
-// The syntheses read 0.9 GB of operands from L2 per table and need 0.13 ms for
-// it, 0.11 ms of tensor-core issue and 0.13 ms of FP64 additions; the three
-// overlap in part (0.29 ms).  T42 with 20 levels: 0.57 -> 0.35 ms; with a launch
+// With 4 tracers (1154 columns) a synthesis through P reads 0.9 GB of operands from L2 and
+// needs 0.13 ms for it, 0.11 ms of tensor-core issue and 0.13 ms of FP64
+// additions; the three overlap in part (0.29 ms).  T42 with 20 levels: 0.57 -> 0.35 ms; with a launch
 // per table 0.47 ms (and 4.35 ms at T126).
 #include <algorithm>
 #include <stdexcept>

@@ -1044,8 +1044,7 @@ static const CUtensorMap& cached_raw_map(TcPlan& p, const void* base, const uint
 }
 
 static int round_up(int x, int a) { return (x + a - 1) / a * a; }
-// N tile: multiple of 16, at most 160 so that three stages of
-// (2 x 128 + 2 x N) rows of 128 bytes fit in 227 KB of shared memory
+// the balanced tile at most cap wide over n rows: a multiple of 16
 static int tile_n(int n, int cap) {
   int nt = (n + cap - 1) / cap;
   return round_up((n + nt - 1) / nt, 16);

@@ -85,9 +85,6 @@ int tc_slots(const TcPlan& p, int n);
 // switches the synthesis GEMM to latitude tile nsyn (autotuning)
 void tc_set_nsyn(TcPlan& p, int nsyn);
 
-// F[m][j][c] (real columns c0.. of the GEMM) = Legendre synthesis of the
-// real columns [0, ncols) of B[idx][.] (row pitch ldB, nrowsB rows
-// allocated), tensor-core path.  The fused path reads B in pairs of rows,
 // One transform's columns through a table (useH: dP/dphi); the fused kernel
 // takes one or two (both tables, any arrays) in a launch.
 struct TcLeg {
@@ -98,9 +95,11 @@ struct TcLeg {
   float* out;
   long ldout;
 };
-// so it needs 2 floor(nrowsB / 2) >= nlm; otherwise the split path runs.
+// Legendre synthesis out[m][j][c] of each leg's real columns [0, ncols) of
+// in[idx][.] (nrowsB rows allocated).  The fused path reads the input in pairs of
+// rows, so it needs 2 floor(nrowsB / 2) >= nlm; otherwise the split path runs.
 void tc_synth(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, long nrowsB, cudaStream_t s);
-// A[idx][c] = Legendre analysis of G[m][j][c] (real columns [0, ncols)).
+// Legendre analysis out[idx][c] of each leg's in[m][j][c], real columns [0, ncols)
 void tc_anal(TcPlan& p, const long* d_moff, const TcLeg* legs, int n, cudaStream_t s);
 // the K segments tc_anal uses (the plan's aseg, at most one per latitude chunk)
 int tc_anal_segments(const TcPlan& p);
